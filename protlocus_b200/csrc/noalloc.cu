@@ -77,7 +77,7 @@ static int na_run(const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n_jo
 	plk_params_t P;
 	int dev = 0, max_sub = 0, i, m;
 	int64_t prep_total = 0, tmp_total = 0, trace_total = 0, off = 0, total_words = 0;
-	int32_t max_al = 1, pos = 0;
+	int32_t max_al = 1, max_len = 1, pos = 0;
 	unsigned char *base;
 	cudaError_t e;
 
@@ -131,6 +131,8 @@ static int na_run(const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n_jo
 		J->tmp_off = tmp_total, tmp_total += (int64_t)x->nl + x->al + 8;
 		J->trace_off = trace_total / 2, trace_total += (plk_trace_words(x->nl, x->al, 1, PLK_DP_ROWS) * 2 + 15) / 16 * 16;
 		if (x->al > max_al) max_al = x->al;
+		if (x->nl > max_len) max_len = x->nl;
+		if (x->al > max_len) max_len = x->al;
 	}
 	/* carve the array: jobs | order | counters | total | prep | tmp | ring | trace */
 	{
@@ -167,7 +169,7 @@ static int na_run(const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n_jo
 		if ((e = cudaMemcpyAsync(d_jobs, g_na_jobs, sizeof(plk_job_t) * (size_t)n_jobs, cudaMemcpyHostToDevice, st)) != cudaSuccess ||
 				(e = cudaMemcpyAsync(d_order, g_na_order, 4 * (size_t)n_jobs, cudaMemcpyHostToDevice, st)) != cudaSuccess)
 			goto cuda_fail;
-		if ((e = (cudaError_t)plk_prep(d_jobs, n_jobs, nt, aa, ss, d_prep, &P, st)) != cudaSuccess) goto cuda_fail;
+		if ((e = (cudaError_t)plk_prep(d_jobs, n_jobs, max_len, nt, aa, ss, d_prep, &P, st)) != cudaSuccess) goto cuda_fail;
 		for (m = 0, pos = 0; m < 3; ++m) {
 			int32_t n_m = 0;
 			while (pos + n_m < n_jobs && g_na_jobs[g_na_order[pos + n_m]].mode == m) ++n_m;

@@ -459,14 +459,14 @@ static uint64_t pl_fnv(uint64_t h, const void *p, size_t n)
 static int pl_group_of(const plk_job_t *J);
 
 static uint64_t pl_plan_key(const pl_engine_t *e, int32_t n, int32_t n_waves, int32_t two, int64_t arena_words,
-		int64_t ring_ints, int32_t max_al, const void *nt, const void *aa, const void *ss, const void *res,
+		int64_t ring_ints, int32_t max_al, int32_t max_len, const void *nt, const void *aa, const void *ss, const void *res,
 		const void *cig, int64_t cig_cap, cudaStream_t st, const plk_params_t *P)
 {
 	uint64_t h = 1469598103934665603ull;
 	const void *ptr[14];
-	int64_t v[7];
+	int64_t v[8];
 	int32_t i;
-	v[0] = n, v[1] = n_waves, v[2] = two, v[3] = arena_words, v[4] = ring_ints, v[5] = max_al, v[6] = cig_cap;
+	v[0] = n, v[1] = n_waves, v[2] = two, v[3] = arena_words, v[4] = ring_ints, v[5] = max_al, v[6] = cig_cap, v[7] = max_len;
 	ptr[0] = nt, ptr[1] = aa, ptr[2] = ss, ptr[3] = res, ptr[4] = cig, ptr[5] = (const void*)st, ptr[6] = e->jobs.p;
 	ptr[7] = e->order.p, ptr[8] = e->counters.p, ptr[9] = e->prep.p, ptr[10] = e->trace.p, ptr[11] = e->ring.p;
 	ptr[12] = e->tmp.p, ptr[13] = e->total.p;
@@ -485,7 +485,7 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		uint32_t *cig_dev, int64_t cig_cap, int64_t *total_out, cudaStream_t st)
 {
 	plk_params_t P;
-	int32_t q, max_al = 1, n_waves = 1, w, max_sub, *sorted, wave_n_coop = 0, two = 0;
+	int32_t q, max_al = 1, max_len = 1, n_waves = 1, w, max_sub, *sorted, wave_n_coop = 0, two = 0;
 	int64_t prep_total = 0, tmp_total = 0, trace_total = 0, max_trace = 0, slots, arena_budget, arena_words = 0;
 	int64_t ring_ints = 0;
 	int64_t *wave_bytes = 0, *wave_cells = 0, total_words = 0;
@@ -519,6 +519,8 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		J->tmp_off = tmp_total, tmp_total += (int64_t)x->nl + x->al + 8;
 		J->score = INT32_MIN;
 		if (x->al > max_al) max_al = x->al;
+		if (x->nl > max_len) max_len = x->nl;
+		if (x->al > max_len) max_len = x->al;
 		trace_total += plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2;
 		if (plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2 > max_trace)
 			max_trace = plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2;
@@ -623,7 +625,7 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	   * contents, which the copies above refresh.  A shape seen on the previous call is
 	   * captured into a CUDA graph on this one and replayed while it recurs (timed runs
 	   * launch directly: their events sit between the launches). */
-		const uint64_t key = pl_plan_key(e, n, n_waves, two, arena_words, ring_ints, max_al, nt, aa, ss, res_dev,
+		const uint64_t key = pl_plan_key(e, n, n_waves, two, arena_words, ring_ints, max_al, max_len, nt, aa, ss, res_dev,
 				cig_dev, cig_cap, st, &P);
 		const int use = e->graphs && !e->timing;
 		if (use && e->g_exec && key == e->g_key) {
@@ -645,7 +647,7 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		}
 	}
 	PL_TIME(e, st, 0);
-	CKK(plk_prep((const plk_job_t*)e->jobs.p, n, nt, aa, ss, (uint8_t*)e->prep.p, &P, st));
+	CKK(plk_prep((const plk_job_t*)e->jobs.p, n, max_len, nt, aa, ss, (uint8_t*)e->prep.p, &P, st));
 	PL_TIME(e, st, 0);
 	if (two) { /* fork: the side stream starts after the preparation */
 		CK(cudaEventRecord(e->ev_fork, st));

@@ -113,7 +113,7 @@ static inline int64_t plk_trace_words(int32_t nl, int32_t al, int32_t nw, int32_
 }
 
 /* launchers; all return a cudaError_t value as int */
-int plk_prep(const plk_job_t *jobs, int32_t n_jobs, const uint8_t *nt, const uint8_t *aa, const uint8_t *ss,
+int plk_prep(const plk_job_t *jobs, int32_t n_jobs, int32_t max_len, const uint8_t *nt, const uint8_t *aa, const uint8_t *ss,
 		uint8_t *prep, const plk_params_t *p, void *stream);
 /* order_coop: jobs run by a whole CTA (nw = PLK_WARPS_PER_CTA); order_solo: one warp each.
  * counters: 2 ints of device scratch.  ring: PLK_WARPS_PER_CTA * n_ctas * ring_stride_ints ints. */

@@ -40,22 +40,34 @@ static unsigned long long g_launches = 0;
 
 /* ------------------------------------------------------------------ preparation */
 
+/* A CTA prepares PREP_CHUNK positions of one job.  One CTA per job left a single request's
+ * 20 kb window on one SM (104 us; 16 us over chunks, and 365 -> 172 us for 509 windows of up
+ * to 50 kb); the batch's grid only gains CTAs that leave at once. */
+#define PREP_CHUNK 2048
+
 __global__ void k_prep(const plk_job_t *__restrict__ jobs, int n_jobs, const uint8_t *__restrict__ nt,
 		const uint8_t *__restrict__ aa, const uint8_t *__restrict__ ss, uint8_t *__restrict__ prep, plk_params_t P)
 {
 	__shared__ uint8_t s_nt4[256], s_aa20[256], s_codon[64];
-	for (int x = threadIdx.x; x < 256; x += blockDim.x) s_nt4[x] = P.nt4[x], s_aa20[x] = P.aa20[x];
-	for (int x = threadIdx.x; x < 64; x += blockDim.x) s_codon[x] = P.codon[x];
-	__syncthreads();
-	for (int jb = blockIdx.x; jb < n_jobs; jb += gridDim.x) {
+	int staged = 0;
+	for (int jb = blockIdx.x; jb < n_jobs; jb += gridDim.x)
+	for (int64_t p0 = (int64_t)blockIdx.y * PREP_CHUNK; ; p0 += (int64_t)gridDim.y * PREP_CHUNK) {
 		const plk_job_t J = jobs[jb];
 		const int nl = J.nl, al = J.al;
+		if (p0 > nl && p0 >= al) break;
+		if (!staged) { /* the CTA's first job inside its chunk: the same for every thread */
+			for (int x = threadIdx.x; x < 256; x += blockDim.x) s_nt4[x] = P.nt4[x], s_aa20[x] = P.aa20[x];
+			for (int x = threadIdx.x; x < 64; x += blockDim.x) s_codon[x] = P.codon[x];
+			__syncthreads();
+			staged = 1;
+		}
 		const uint8_t *ns = nt + J.nt_off, *as = aa + J.aa_off, *sst = J.ss_off >= 0 ? ss + J.ss_off : 0;
 		uint8_t *nas = prep + J.prep_off, *aas = nas + nl;
 		int8_t *donor = (int8_t*)(aas + al), *acceptor = donor + nl + 1;
-		for (int j = threadIdx.x; j < al; j += blockDim.x) aas[j] = s_aa20[as[j]];
-		for (int p = threadIdx.x; p <= nl; p += blockDim.x)
-			prep_fwd_pos(p, ns, nl, sst, s_nt4, s_codon, P, nas, donor, acceptor);
+		const int je = (int)min((int64_t)al, p0 + PREP_CHUNK), pe = (int)min((int64_t)nl, p0 + PREP_CHUNK - 1);
+		for (int64_t j = p0 + threadIdx.x; j < je; j += blockDim.x) aas[j] = s_aa20[as[j]];
+		for (int64_t p = p0 + threadIdx.x; p <= pe; p += blockDim.x)
+			prep_fwd_pos((int)p, ns, nl, sst, s_nt4, s_codon, P, nas, donor, acceptor);
 	}
 }
 
@@ -845,10 +857,24 @@ k_splice_pair(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_co
 /* trace-word bit of the extension flag of state 1..5 (I, D, A, B, C) */
 __device__ __forceinline__ int tb_ext_bit(int state) { return (0x6DC540 >> (4 * state)) & 15; }
 
-__device__ __forceinline__ void tb_push(uint32_t *out, int &n, uint32_t op, int len)
-{ /* ns_push_cigar merge rule (nasw.h:219-229) */
-	if (n == 0 || op != (out[n - 1] & 0xf) || op == NS_CIGAR_F || op == NS_CIGAR_G) out[n++] = (uint32_t)len << 4 | op;
-	else out[n - 1] += (uint32_t)len << 4;
+/* the walk's last CIGAR word, kept in a register until the op changes (ns_push_cigar's merge
+ * rule, nasw.h:219-229): merging into the word in memory cost dependent L2 round trips a
+ * step (with the wider scan of long intron runs: 357 -> 279 us for one 500 aa x 20 kb walk,
+ * 1388 -> 1039 us for 509 loci) */
+struct TbOut {
+	uint32_t *out;
+	uint32_t cur;  /* len << 4 | op, 0: none yet */
+	int n;         /* words stored */
+};
+
+__device__ __forceinline__ void tb_push(TbOut &T, uint32_t op, int len)
+{
+	if (T.cur != 0 && op == (T.cur & 0xf) && op != NS_CIGAR_F && op != NS_CIGAR_G) {
+		T.cur += (uint32_t)len << 4;
+		return;
+	}
+	if (T.cur != 0) T.out[T.n++] = T.cur;
+	T.cur = (uint32_t)len << 4 | op;
 }
 
 /* Traceback: one warp per job.  The walk is inherently sequential, so the warp
@@ -892,6 +918,35 @@ __device__ __forceinline__ void tb_norm8(uint16_t (&w)[8], const bool pair)
 	for (int r = 0; r < 8; ++r) w[r] = tb_pair_norm(w[r]);
 }
 
+/* the highest row <= i of column j whose extension bit is clear, among the 32*C R-row chunks
+ * down from chunk ch_top (lane l reads chunks l, l + 32, ...); -1 when none is */
+template <int C>
+__device__ __forceinline__ int tb_scan(const uint16_t *__restrict__ tr, const int R, const int nlanes, const int al,
+		const int ch_top, const int lane, const int j, const int i, const int bit, const bool pair)
+{
+	int end_row = -1;
+	__align__(16) uint16_t w[C][8];
+#pragma unroll
+	for (int m = 0; m < C; ++m) {
+		const int ch = ch_top - lane - 32 * m;
+		if (ch >= 0) tb_load_chunk(tr, R, nlanes, al, ch, j, w[m]);
+	}
+#pragma unroll
+	for (int m = 0; m < C; ++m) {
+		const int ch = ch_top - lane - 32 * m;
+		if (ch < 0) continue;
+		tb_norm8(w[m], pair);
+#pragma unroll
+		for (int r = 0; r < 8; ++r) { /* ascending rows: the highest clear one stays (end_row falls with m) */
+			const int row = ch * R + 2 + r;
+			if (r < R && row <= i && !((w[m][r] >> bit) & 1u)) end_row = max(end_row, row);
+		}
+	}
+#pragma unroll
+	for (int o = 16; o >= 1; o >>= 1) end_row = max(end_row, __shfl_xor_sync(FULL, end_row, o));
+	return end_row;
+}
+
 __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restrict__ jobs,
 		const int32_t *__restrict__ order, int n_order, const uint16_t *__restrict__ trace, uint32_t *__restrict__ tmp)
 {
@@ -902,10 +957,11 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 	plk_job_t *J = jobs + order[q];
 	const int nl = J->nl, al = J->al, R = J->rows;
 	const uint16_t *tr = trace + J->trace_off;
-	uint32_t *out = tmp + J->tmp_off;
+	TbOut T;  /* lane 0's */
+	T.out = tmp + J->tmp_off, T.cur = 0, T.n = 0;
 	const int nlanes = 32 * J->nw;
 	const bool pair = J->mode == 3;
-	int i = nl - 1, j = al - 1, last = 0, n = 0;
+	int i = nl - 1, j = al - 1, last = 0;
 	while (i >= 2 && j >= 0) {
 		/* stage the tile whose top-right corner holds (i, j): 8-row groups, one or two chunks each */
 		const int qc = (i - 2) / 8, jc = j;
@@ -937,67 +993,59 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 				const int state = last != 0 ? last : (x >> 14 & 1) ? 1 : 15 - (x & 0xf);
 				const int ext = state >= 1 && state <= 5 ? (x >> tb_ext_bit(state)) & 1 : 0;
 				switch (state) {
-				case 0: tb_push(out, n, NS_CIGAR_M, 1), i -= 3, --j; break;
-				case 1: tb_push(out, n, NS_CIGAR_I, 1), --j; break;
-				case 2: tb_push(out, n, NS_CIGAR_D, 1), i -= 3; break;
-				case 3: tb_push(out, n, NS_CIGAR_N, 1), --i; break;
-				case 4: tb_push(out, n, NS_CIGAR_U, 1), --i; if (!ext) --j; break;
-				case 5: tb_push(out, n, NS_CIGAR_V, 1), --i; if (!ext) --j; break;
-				case 6: tb_push(out, n, NS_CIGAR_F, 1), --i; break;
-				case 7: tb_push(out, n, NS_CIGAR_F, 2), i -= 2; break;
-				case 8: tb_push(out, n, NS_CIGAR_G, 1), --i, --j; break;
-				default: tb_push(out, n, NS_CIGAR_G, 2), i -= 2, --j; break;
+				case 0: tb_push(T, NS_CIGAR_M, 1), i -= 3, --j; break;
+				case 1: tb_push(T, NS_CIGAR_I, 1), --j; break;
+				case 2: tb_push(T, NS_CIGAR_D, 1), i -= 3; break;
+				case 3: tb_push(T, NS_CIGAR_N, 1), --i; break;
+				case 4: tb_push(T, NS_CIGAR_U, 1), --i; if (!ext) --j; break;
+				case 5: tb_push(T, NS_CIGAR_V, 1), --i; if (!ext) --j; break;
+				case 6: tb_push(T, NS_CIGAR_F, 1), --i; break;
+				case 7: tb_push(T, NS_CIGAR_F, 2), i -= 2; break;
+				case 8: tb_push(T, NS_CIGAR_G, 1), --i, --j; break;
+				default: tb_push(T, NS_CIGAR_G, 2), i -= 2, --j; break;
 				}
 				last = state >= 1 && state <= 5 && ext ? state : 0;
 			}
 		}
 		i = __shfl_sync(FULL, i, 0), j = __shfl_sync(FULL, j, 0);
-		last = __shfl_sync(FULL, last, 0), n = __shfl_sync(FULL, n, 0);
+		last = __shfl_sync(FULL, last, 0);
 		__syncwarp();
 		/* Inside an intron run (A/B/C extended: the path climbs column j one row per
-		 * step while the state's extension bit stays set) the warp scans 32*R rows of
-		 * the column at once: each lane reads one R-row chunk, and the run ends at the
-		 * highest row <= i whose bit is clear.  The rows of the run become one merged
-		 * N/U/V op, exactly what the row-by-row walk pushes. */
+		 * step while the state's extension bit stays set) the warp scans the column: each
+		 * lane reads R-row chunks, and the run ends at the highest row <= i whose bit is
+		 * clear.  The rows of the run become one merged N/U/V op, exactly what the
+		 * row-by-row walk pushes.  A run's first round takes 32*R rows (most introns end
+		 * there), later ones four times as many in flight: the flanks of a wide window are
+		 * one long run, and a round costs a memory latency whatever it reads. */
+		int wide = 0;
 		while (last >= 3 && last <= 5 && i >= 2 && j >= 0) {
-			const int ch_top = (i - 2) / R, ch = ch_top - lane;
-			const int bit = tb_ext_bit(last);
-			int end_row = -1;
-			if (ch >= 0) {
-				__align__(16) uint16_t w[8];
-				tb_load_chunk(tr, R, nlanes, al, ch, j, w);
-				tb_norm8(w, pair);
-				const int ra = ch * R;
-#pragma unroll
-				for (int r = 7; r >= 0; --r) {
-					const int row = ra + 2 + r;
-					if (r < R && end_row < 0 && row <= i && !((w[r] >> bit) & 1u)) end_row = row;
-				}
-			}
-#pragma unroll
-			for (int o = 16; o >= 1; o >>= 1) end_row = max(end_row, __shfl_xor_sync(FULL, end_row, o));
-			const int low = max(2, (ch_top - 31) * R + 2);
+			const int ch_top = (i - 2) / R, bit = tb_ext_bit(last);
 			const int op = last == 3 ? NS_CIGAR_N : (last == 4 ? NS_CIGAR_U : NS_CIGAR_V);
+			int end_row = -1;
+			if (wide) end_row = tb_scan<4>(tr, R, nlanes, al, ch_top, lane, j, i, bit, pair);
+			else end_row = tb_scan<1>(tr, R, nlanes, al, ch_top, lane, j, i, bit, pair);
+			const int low = max(2, (ch_top - (wide ? 127 : 31)) * R + 2);
+			wide = 1;
 			if (end_row >= low) { /* the run ends at end_row: its step clears the state (and moves j for U/V) */
-				if (lane == 0) tb_push(out, n, op, i - end_row + 1);
+				if (lane == 0) tb_push(T, op, i - end_row + 1);
 				i = end_row - 1;
 				if (last != 3) --j;
 				last = 0;
 			} else {              /* every row down to `low` extends the run */
-				if (lane == 0) tb_push(out, n, op, i - low + 1);
+				if (lane == 0) tb_push(T, op, i - low + 1);
 				i = low - 1;
 			}
-			n = __shfl_sync(FULL, n, 0);
 		}
 	}
 	if (lane == 0) {
-		if (j > 0) tb_push(out, n, NS_CIGAR_I, j);
+		if (j > 0) tb_push(T, NS_CIGAR_I, j);
 		if (i >= 0) {
 			const int l = (i + 1) / 3, t = (i + 1) % 3;
-			if (l > 0) tb_push(out, n, NS_CIGAR_D, l);
-			if (t != 0) tb_push(out, n, NS_CIGAR_F, t);
+			if (l > 0) tb_push(T, NS_CIGAR_D, l);
+			if (t != 0) tb_push(T, NS_CIGAR_F, t);
 		}
-		J->n_tmp = n;
+		if (T.cur != 0) T.out[T.n++] = T.cur;
+		J->n_tmp = T.n;
 	}
 }
 
@@ -1046,11 +1094,12 @@ __global__ void k_compact(const plk_job_t *__restrict__ jobs, int n_jobs, const 
 
 /* ------------------------------------------------------------------ launchers */
 
-extern "C" int plk_prep(const plk_job_t *jobs, int32_t n_jobs, const uint8_t *nt, const uint8_t *aa,
+extern "C" int plk_prep(const plk_job_t *jobs, int32_t n_jobs, int32_t max_len, const uint8_t *nt, const uint8_t *aa,
 		const uint8_t *ss, uint8_t *prep, const plk_params_t *p, void *stream)
 {
 	if (n_jobs <= 0) return 0;
-	const int grid = n_jobs < 65535 ? n_jobs : 65535;
+	const int chunks = max_len / PREP_CHUNK + 1;  /* max_len: the longest window or protein */
+	const dim3 grid(n_jobs < 65535 ? n_jobs : 65535, chunks < 65535 ? chunks : 65535);
 	k_prep<<<grid, 256, 0, (cudaStream_t)stream>>>(jobs, n_jobs, nt, aa, ss, prep, *p);
 	__sync_fetch_and_add(&g_launches, 1ull);
 	return (int)cudaGetLastError();
