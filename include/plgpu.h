@@ -202,8 +202,9 @@ void *pl_engine_stream(const pl_engine_t *e);
  * occupancy.  The DP kernels are bound by this pipe.  Returns 1 on success. */
 int pl_measure_int_peak(int32_t device, double *int32_lane_ops, double *int16x2_lane_ops);
 /* Tuning of the batched global DP: jobs with at most r4_rows DP rows (nl - 2) run 4
- * rows per lane, the rest 8; a job takes a whole CTA when it holds more than
- * coop_ratio times a warp's share of its wave's cells.  set: negative / non-positive
+ * rows per lane, the rest 8; the strips of a job (32 lanes of rows each) are shared among
+ * the GPU's warps when it holds more than coop_ratio times a third of a warp's share of its
+ * wave's cells, else one warp runs them all.  set: negative / non-positive
  * arguments keep the current value.  autotune: times the given batch (results
  * discarded) under a grid of both, keeps the fastest on the engine and reports it. */
 void pl_engine_set_tuning(pl_engine_t *e, int32_t r4_rows, double coop_ratio);
@@ -219,15 +220,16 @@ int pl_engine_autotune(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_
  * the failure is the error path the real failure takes.  Returns 1 when armed. */
 int pl_debug_fault(int32_t site, int32_t after);
 
-/* Number of trace waves, cooperative jobs and DP launches of the last batch. */
+/* Number of trace waves, jobs with shared strips and DP launches of the last batch. */
 void pl_engine_last_plan(const pl_engine_t *e, int32_t *n_waves, int32_t *n_coop, int32_t *n_dp_launches);
 /* Two 16-bit jobs that share one protein (the same aa_off in the job table) and one
  * window length -- the two strands of a locus -- run as a pair in the two halves of
  * the int16x2 DP kernel when their score range fits its 15-bit domain (on by
  * default; PLGPU_PAIR=0 or pl_engine_set_pairing(e, 0) turns it off).  With
  * enable = 1 the eligible jobs pair when they make at least PLGPU_PAIR_MIN (default 1)
- * times as many pairs as the DP launch has warps (a batch too small to fill the GPU
- * keeps its jobs single: a pair's unit of work is longer than a job's); enable = 2
+ * times as many pairs as the DP launch has warps, or when the strips of the single jobs
+ * would keep the warps busy for longer than the longest job's chain of strips takes as a
+ * pair (a batch too small to fill the GPU keeps its jobs single); enable = 2
  * pairs every eligible job.  Results are the same either way.
  * pl_engine_last_pairs: pairs formed in the last batch. */
 void pl_engine_set_pairing(pl_engine_t *e, int32_t enable);

@@ -266,10 +266,12 @@ int pl_max_sub(const ns_opt_t *opt)
 	return m;
 }
 
-/* A job runs on a whole CTA (a 2048-row cooperative wavefront) when it holds more
- * than this multiple of a warp's share of its wave's cells: fewer, longer jobs then
- * finish with the rest instead of trailing them.  PLGPU_COOP_RATIO overrides it
- * (the tuning sweep of the batched workload). */
+/* A job's strips are shared among the GPU's warps when it (a pair: both jobs) holds more than
+ * this multiple of a third of a warp's share of its wave's cells; the others run whole on one warp each,
+ * after the strips, and fill the end of the launch.  A strip of its own costs 31 steps of
+ * filling and draining the warp (al + 31 steps for al columns), which a whole job pays once,
+ * but a whole job of more than a small part of a warp's share would trail the launch.
+ * PLGPU_COOP_RATIO overrides it (the tuning sweep of the batched workload). */
 static double g_coop_ratio = 0.7;
 static pthread_once_t g_coop_once = PTHREAD_ONCE_INIT;
 static void pl_coop_ratio_init(void)
@@ -389,13 +391,13 @@ static int pl_cmp_pair(const void *a, const void *b)
 	return x->idx - y->idx;
 }
 
-/* A pair runs as one unit of work: one step of a pair costs about 1.7 steps of a single
- * job and does two jobs' cells.  While a batch's units fill the GPU that is a gain;
- * a batch with fewer units than the DP launch has warps would only make its units
- * longer.  So pairs are formed only when there are at least PLGPU_PAIR_MIN (default 1)
- * times as many of them as warps of a launch -- for every eligible job or none, since a
- * single job and a pair run in different launches, one after the other.  pairing = 2
- * pairs every eligible job. */
+/* One step of a pair costs about 1.7 steps of a single job and does two jobs' cells: a gain
+ * while there is work for every warp, a loss where a launch only waits for its longest chain
+ * of strips, each some 40 columns behind the one above.  So the jobs pair (every eligible one
+ * or none: single jobs and pairs run in different launches, one after the other) when there
+ * are at least PLGPU_PAIR_MIN (default 1) times as many pairs as the DP launch has warps, or
+ * when the warps' mean share of the single jobs' strips exceeds 1.7 of the longest chain.
+ * pairing = 2 pairs every eligible job. */
 static double g_pair_min = 1.0;
 static pthread_once_t g_pair_min_once = PTHREAD_ONCE_INIT;
 static void pl_pair_min_init(void)
@@ -412,7 +414,7 @@ static void pl_pair_min_init(void)
 static int32_t pl_form_pairs(pl_engine_t *e, const ns_opt_t *opt, int32_t n, int max_sub, plk_params_t *P)
 {
 	pl_pkey_t *key;
-	int32_t q, m = 0, n_pairs = 0, al_cap = 0, bias = 0;
+	int32_t q, m = 0, n_pairs = 0, al_cap = 0, bias = 0, pays = 1;
 	if (!e->pairing || n < 2 || !pl_pair_limits(opt, max_sub, &al_cap, &bias)) return 0;
 	key = (pl_pkey_t*)malloc(sizeof(*key) * (size_t)n);
 	if (!key) return 0;
@@ -425,7 +427,7 @@ static int32_t pl_form_pairs(pl_engine_t *e, const ns_opt_t *opt, int32_t n, int
 	for (q = 0; q + 1 < m; ++q) {
 		if (key[q].aa_off != key[q + 1].aa_off || key[q].al != key[q + 1].al || key[q].nl != key[q + 1].nl) continue;
 		/* a pair shares one wave: both traces must fit the budget together */
-		if (2 * plk_trace_words(key[q].nl, key[q].al, PLK_WARPS_PER_CTA, e->hj[key[q].idx].rows) * 2 > e->trace_budget)
+		if (2 * plk_trace_words(key[q].nl, key[q].al, e->hj[key[q].idx].rows) * 2 > e->trace_budget)
 			continue;
 		{
 			plk_job_t *A = &e->hj[key[q].idx], *B = &e->hj[key[q + 1].idx];
@@ -436,8 +438,18 @@ static int32_t pl_form_pairs(pl_engine_t *e, const ns_opt_t *opt, int32_t n, int
 	}
 	free(key);
 	pthread_once(&g_pair_min_once, pl_pair_min_init);
-	if (e->pairing == 1 && n_pairs > 0 &&
-			(double)n_pairs < g_pair_min * e->n_sm * e->ctas_per_sm[3][0] * PLK_WARPS_PER_CTA) {
+	if (e->pairing == 1 && n_pairs > 0) {
+		const double slots = (double)e->n_sm * e->ctas_per_sm[3][0] * PLK_WARPS_PER_CTA;
+		double steps = 0, chain = 0;
+		for (q = 0; q < n; ++q) {
+			const plk_job_t *J = &e->hj[q];
+			const double S = (double)plk_strips(J->nl, J->rows), c = S * 40 + J->al;
+			steps += S * (J->al + 31);
+			if (c > chain) chain = c;
+		}
+		pays = (double)n_pairs >= g_pair_min * slots || steps / slots > 1.7 * g_pair_min * chain;
+	}
+	if (!pays) {
 		for (q = 0; q < n; ++q)  /* too few to fill the GPU: every job single */
 			if (e->hj[q].mode == 3) e->hj[q].mode = 0, e->hj[q].pair = 0;
 		return 0;
@@ -459,21 +471,23 @@ static uint64_t pl_fnv(uint64_t h, const void *p, size_t n)
 static int pl_group_of(const plk_job_t *J);
 
 static uint64_t pl_plan_key(const pl_engine_t *e, int32_t n, int32_t n_waves, int32_t two, int64_t arena_words,
-		int64_t ring_ints, int32_t max_al, int32_t max_len, const void *nt, const void *aa, const void *ss, const void *res,
+		int64_t ring_stride, int64_t sring_ints, const plk_dp_group_t *grp, int32_t n_grp, int32_t max_len,
+		const void *nt, const void *aa, const void *ss, const void *res,
 		const void *cig, int64_t cig_cap, cudaStream_t st, const plk_params_t *P)
 {
 	uint64_t h = 1469598103934665603ull;
 	const void *ptr[14];
 	int64_t v[8];
 	int32_t i;
-	v[0] = n, v[1] = n_waves, v[2] = two, v[3] = arena_words, v[4] = ring_ints, v[5] = max_al, v[6] = cig_cap, v[7] = max_len;
+	v[0] = n, v[1] = n_waves, v[2] = two, v[3] = arena_words, v[4] = ring_stride, v[5] = max_len, v[6] = cig_cap, v[7] = sring_ints;
 	ptr[0] = nt, ptr[1] = aa, ptr[2] = ss, ptr[3] = res, ptr[4] = cig, ptr[5] = (const void*)st, ptr[6] = e->jobs.p;
 	ptr[7] = e->order.p, ptr[8] = e->counters.p, ptr[9] = e->prep.p, ptr[10] = e->trace.p, ptr[11] = e->ring.p;
 	ptr[12] = e->tmp.p, ptr[13] = e->total.p;
 	h = pl_fnv(h, v, sizeof(v)), h = pl_fnv(h, ptr, sizeof(ptr)), h = pl_fnv(h, P, sizeof(*P));
+	h = pl_fnv(h, grp, sizeof(*grp) * (size_t)n_grp);
 	for (i = 0; i < n; ++i) {
 		const plk_job_t *J = &e->hj[e->horder[i]];
-		const int32_t t = e->hwave[e->horder[i]] << 8 | pl_group_of(J) << 4 | J->rows << 1 | (J->nw > 1);
+		const int32_t t = e->hwave[e->horder[i]] << 8 | pl_group_of(J) << 4 | J->rows << 1 | J->shared;
 		h = pl_fnv(h, &t, sizeof(t));
 	}
 	return h ? h : 1;
@@ -485,9 +499,12 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		uint32_t *cig_dev, int64_t cig_cap, int64_t *total_out, cudaStream_t st)
 {
 	plk_params_t P;
-	int32_t q, max_al = 1, max_len = 1, n_waves = 1, w, max_sub, *sorted, wave_n_coop = 0, two = 0;
+	int32_t q, max_len = 1, n_waves = 1, w, max_sub, *sorted, wave_n_coop = 0, two = 0;
 	int64_t prep_total = 0, tmp_total = 0, trace_total = 0, max_trace = 0, slots, arena_budget, arena_words = 0;
-	int64_t ring_ints = 0;
+	int64_t ring_ints = 0, sring_ints = 0, ring_stride = 0, max_units = 0;
+	const int64_t units_off = ((int64_t)n * 4 + 15) / 16 * 16;  /* the strip queues sit behind the order array */
+	plk_dp_group_t *grp = 0;
+	int32_t *wave_grp = 0, *bucket = 0;
 	int64_t *wave_bytes = 0, *wave_cells = 0, total_words = 0;
 	int ok = 0, capturing = 0;
 	uint64_t g_launch0 = 0, g_key = 0;
@@ -499,7 +516,7 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	max_sub = pl_max_sub(opt);
 	slots = (int64_t)e->n_sm * e->ctas_per_sm[0][0] * PLK_WARPS_PER_CTA;
 
-	/* 1. per-job metadata with nw = 1 sizes */
+	/* 1. per-job metadata */
 	for (q = 0; q < n; ++q) {
 		plk_job_t *J = &e->hj[q];
 		const pl_splice_job_t *x = &jobs[q];
@@ -513,17 +530,15 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		J->nl = x->nl, J->al = x->al;
 		J->mode = bound + opt->end_bonus > 30000 ? 1 : (bound + 256 >= 32767 ? 2 : 0);
 		J->slen = J->mode == 1 ? (x->al + 3) / 4 : (x->al + 7) / 8;
-		J->nw = 1;
 		J->rows = x->nl - 2 <= e->r4_rows ? 4 : PLK_DP_ROWS;
 		J->prep_off = prep_total, prep_total += plk_prep_bytes(x->nl, x->al);
 		J->tmp_off = tmp_total, tmp_total += (int64_t)x->nl + x->al + 8;
 		J->score = INT32_MIN;
-		if (x->al > max_al) max_al = x->al;
 		if (x->nl > max_len) max_len = x->nl;
 		if (x->al > max_len) max_len = x->al;
-		trace_total += plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2;
-		if (plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2 > max_trace)
-			max_trace = plk_trace_words(x->nl, x->al, PLK_WARPS_PER_CTA, J->rows) * 2;
+		trace_total += plk_trace_words(x->nl, x->al, J->rows) * 2;
+		if (plk_trace_words(x->nl, x->al, J->rows) * 2 > max_trace)
+			max_trace = plk_trace_words(x->nl, x->al, J->rows) * 2;
 	}
 	if (max_trace > e->trace_budget) {
 		pl_set_error("one job needs %lld trace bytes, over the budget of %lld", (long long)max_trace, (long long)e->trace_budget);
@@ -533,8 +548,8 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	if (e->last_pairs > 0) /* the unit the waves are packed by is a pair: twice a job's trace */
 		for (q = 0; q < n; ++q)
 			if (e->hj[q].mode == 3 && e->hj[q].pair >= 0 &&
-					2 * plk_trace_words(e->hj[q].nl, e->hj[q].al, PLK_WARPS_PER_CTA, e->hj[q].rows) * 2 > max_trace)
-				max_trace = 2 * plk_trace_words(e->hj[q].nl, e->hj[q].al, PLK_WARPS_PER_CTA, e->hj[q].rows) * 2;
+					2 * plk_trace_words(e->hj[q].nl, e->hj[q].al, e->hj[q].rows) * 2 > max_trace)
+				max_trace = 2 * plk_trace_words(e->hj[q].nl, e->hj[q].al, e->hj[q].rows) * 2;
 	/* 2. waves by LPT bin packing on trace bytes.  A batch over the budget runs its
 	 * waves alternately on two streams, each with its own arena of half the budget:
 	 * a wave's DP then starts while the one before drains instead of after it. */
@@ -565,21 +580,20 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		for (t = 0; t < (J->mode == 3 ? 2 : 1); ++t) {
 			const int32_t jj = t == 0 ? j : J->pair;
 			e->hwave[jj] = best;
-			wave_bytes[best] += plk_trace_words(e->hj[jj].nl, e->hj[jj].al, PLK_WARPS_PER_CTA, e->hj[jj].rows) * 2;
+			wave_bytes[best] += plk_trace_words(e->hj[jj].nl, e->hj[jj].al, e->hj[jj].rows) * 2;
 			wave_cells[best] += (int64_t)(e->hj[jj].nl - 2) * e->hj[jj].al;
 		}
 	}
-	/* 3. cooperative or solo, trace offsets inside each wave's arena */
+	/* 3. shared or solo, trace offsets inside each wave's arena */
 	memset(wave_bytes, 0, sizeof(int64_t) * (size_t)n_waves);
 	for (q = 0; q < n; ++q) {
 		const int32_t j = sorted[q];
 		plk_job_t *J = &e->hj[j];
-		const int64_t cells = (int64_t)(J->nl - 2) * J->al, share = wave_cells[e->hwave[j]] / slots;
-		if (J->al >= 200 && J->nl - 2 >= 32 * PLK_WARPS_PER_CTA * J->rows && (double)cells > share * e->coop_ratio)
-			J->nw = PLK_WARPS_PER_CTA;
-		if (J->mode == 3 && J->pair >= 0) e->hj[J->pair].nw = J->nw;  /* a pair shares one wavefront */
+		const int64_t cells = (int64_t)(J->nl - 2) * J->al * (J->mode == 3 ? 2 : 1), strips = plk_strips(J->nl, J->rows);
+		J->shared = strips <= PLK_MAX_STRIPS &&
+				(double)cells > (double)(wave_cells[e->hwave[j]] / slots) * e->coop_ratio / 3.0;
 		J->trace_off = wave_bytes[e->hwave[j]] / 2;
-		wave_bytes[e->hwave[j]] += (plk_trace_words(J->nl, J->al, J->nw, J->rows) * 2 + 15) / 16 * 16;
+		wave_bytes[e->hwave[j]] += (plk_trace_words(J->nl, J->al, J->rows) * 2 + 15) / 16 * 16;
 	}
 	{
 		int64_t need_trace = 0;
@@ -588,35 +602,67 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		arena_words = need_trace / 2;
 		if (!dbuf_ensure(&e->trace, (size_t)need_trace * (two ? 2 : 1))) goto fail;
 	}
-	if (!dbuf_ensure(&e->jobs, sizeof(plk_job_t) * (size_t)n) || !dbuf_ensure(&e->order, sizeof(int32_t) * (size_t)n) ||
+	/* order array: per wave and launch group (mode, rows per lane) the shared jobs, then the
+	 * solo ones, each by decreasing size; the second jobs of pairs are a group without a launch
+	 * at the wave's end (its traceback takes them) */
+	{
+		const int32_t n_b = n_waves * 10 * 2;
+		int32_t pos = 0, b;
+		bucket = (int32_t*)calloc((size_t)n_b + 1, sizeof(int32_t));
+		grp = (plk_dp_group_t*)calloc((size_t)n_waves * 10, sizeof(*grp));
+		wave_grp = (int32_t*)calloc((size_t)n_waves + 1, sizeof(int32_t));
+		if (!bucket || !grp || !wave_grp) { pl_set_error("out of host memory"); goto fail; }
+#define PL_BUCKET(j) (((e->hwave[(j)] * 5 + pl_group_of(&e->hj[(j)])) * 2 + (e->hj[(j)].rows != 8)) * 2 + !e->hj[(j)].shared)
+		for (q = 0; q < n; ++q) ++bucket[PL_BUCKET(q)];
+		for (w = 0; w < n_waves; ++w) {
+			int g;
+			wave_grp[w] = pos;
+			for (g = 0; g < 10; ++g) {
+				plk_dp_group_t *G = &grp[w * 10 + g];
+				G->mode = g / 2, G->rows = g % 2 ? 4 : 8;
+				b = (w * 10 + g) * 2;
+				G->n_shared = bucket[b], G->n_solo = bucket[b + 1];
+				bucket[b] = pos, pos += G->n_shared, bucket[b + 1] = pos, pos += G->n_solo;
+			}
+		}
+		wave_grp[n_waves] = pos;
+		for (q = 0; q < n; ++q) e->horder[bucket[PL_BUCKET(sorted[q])]++] = sorted[q];
+#undef PL_BUCKET
+		for (w = 0, pos = 0; w < n_waves; ++w) {
+			int64_t ring = 0;
+			int g;
+			for (g = 0; g < 10; ++g) {
+				plk_dp_group_t *G = &grp[w * 10 + g];
+				int64_t units = 0;
+				G->ring_off = ring;
+				if (G->mode < 4) {
+					for (q = 0; q < G->n_solo; ++q) {
+						const int64_t al = e->hj[e->horder[pos + G->n_shared + q]].al;
+						if ((al + 1) * PLK_RING_INTS > ring_stride) ring_stride = (al + 1) * PLK_RING_INTS;
+					}
+					for (q = 0; q < G->n_shared; ++q) {
+						plk_job_t *J = &e->hj[e->horder[pos + q]];
+						const int64_t strips = plk_strips(J->nl, J->rows);
+						J->ring_off = ring, ring += 2 * (int64_t)J->al * PLK_RING_INTS;
+						units += strips;
+						if (strips > G->max_strips) G->max_strips = (int32_t)strips;
+					}
+				}
+				if (units > INT32_MAX / 2) { pl_set_error("%lld strips in one launch", (long long)units); goto fail; }
+				G->ring_ints = ring - G->ring_off, G->n_units = (int32_t)units;
+				if (units > max_units) max_units = units;
+				pos += G->n_shared + G->n_solo;
+			}
+			if (ring > sring_ints) sring_ints = ring;
+		}
+	}
+	if (!dbuf_ensure(&e->jobs, sizeof(plk_job_t) * (size_t)n) || !dbuf_ensure(&e->order, (size_t)units_off + 8 * (size_t)(max_units * (two ? 2 : 1))) ||
 			!dbuf_ensure(&e->counters, 64) || !dbuf_ensure(&e->prep, (size_t)prep_total + PLK_PREP_SLACK) ||
 			!dbuf_ensure(&e->tmp, sizeof(uint32_t) * (size_t)tmp_total) || !dbuf_ensure(&e->total, 64))
 		goto fail;
-	{
-		const int64_t stride = ((int64_t)max_al + 1) * PLK_RING_INTS;
-		const int64_t n_ctas = (int64_t)e->n_sm * pl_max_ctas(e);
-		ring_ints = stride * n_ctas * PLK_WARPS_PER_CTA;
-		if (!dbuf_ensure(&e->ring, sizeof(int32_t) * (size_t)(ring_ints * (two ? 2 : 1)))) goto fail;
-	}
-	/* order array: per wave, per mode: cooperative jobs then solo jobs, each by decreasing size */
-	{
-		int32_t pos = 0;
-		for (w = 0; w < n_waves; ++w) {
-			int m, r;
-			for (m = 0; m < 5; ++m)
-				for (r = 0; r < 2; ++r) {
-					const int rows = r == 0 ? 8 : 4;
-					int pass;
-					for (pass = 0; pass < 2; ++pass)
-						for (q = 0; q < n; ++q) {
-							const int32_t j = sorted[q];
-							const plk_job_t *J = &e->hj[j];
-							if (e->hwave[j] == w && pl_group_of(J) == m && J->rows == rows && (J->nw > 1) == (pass == 0))
-								e->horder[pos++] = j;
-						}
-				}
-		}
-	}
+	/* rings: a warp's own for solo jobs, and the shared jobs' (per arena) */
+	ring_ints = ring_stride * e->n_sm * pl_max_ctas(e) * PLK_WARPS_PER_CTA;
+	if (!dbuf_ensure(&e->ring, sizeof(int32_t) * (size_t)((ring_ints + sring_ints) * (two ? 2 : 1)))) goto fail;
 	CK(cudaMemcpyAsync(e->jobs.p, e->hj, sizeof(plk_job_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->order.p, e->horder, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	e->n_ev = 0;
@@ -625,7 +671,8 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	   * contents, which the copies above refresh.  A shape seen on the previous call is
 	   * captured into a CUDA graph on this one and replayed while it recurs (timed runs
 	   * launch directly: their events sit between the launches). */
-		const uint64_t key = pl_plan_key(e, n, n_waves, two, arena_words, ring_ints, max_al, max_len, nt, aa, ss, res_dev,
+		const uint64_t key = pl_plan_key(e, n, n_waves, two, arena_words, ring_stride, sring_ints, grp, n_waves * 10, max_len,
+				nt, aa, ss, res_dev,
 				cig_dev, cig_cap, st, &P);
 		const int use = e->graphs && !e->timing;
 		if (use && e->g_exec && key == e->g_key) {
@@ -654,36 +701,27 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		CK(cudaStreamWaitEvent(e->side, e->ev_fork, 0));
 	}
 	{
-		int32_t pos = 0;
 		for (w = 0; w < n_waves; ++w) {
-			const int32_t wave_start = pos, a = two ? (w & 1) : 0;
+			const int32_t a = two ? (w & 1) : 0;
+			int32_t *ring_w = (int32_t*)e->ring.p + a * (ring_ints + sring_ints);
 			cudaStream_t sw = a ? e->side : st;
 			uint16_t *trace_w = (uint16_t*)e->trace.p + a * arena_words;
-			int m, r;
-			for (m = 0; m < 5; ++m)
-				for (r = 0; r < 2; ++r) {
-					const int rows = r == 0 ? 8 : 4;
-					int32_t n_coop = 0, n_solo = 0;
-#define PL_IN_GROUP(x) (e->hwave[e->horder[(x)]] == w && pl_group_of(&e->hj[e->horder[(x)]]) == m && e->hj[e->horder[(x)]].rows == rows)
-					while (pos + n_coop < n && PL_IN_GROUP(pos + n_coop) && e->hj[e->horder[pos + n_coop]].nw > 1) ++n_coop;
-					while (pos + n_coop + n_solo < n && PL_IN_GROUP(pos + n_coop + n_solo)) ++n_solo;
-#undef PL_IN_GROUP
-					if (n_coop + n_solo > 0 && m < 4) {  /* group 4: second jobs of pairs, run with their first */
-						const int32_t *ord = (const int32_t*)e->order.p + pos;
-						const int64_t stride = ((int64_t)max_al + 1) * PLK_RING_INTS;
-						const int32_t ctas = e->n_sm * e->ctas_per_sm[m][r];
-						PL_TIME(e, sw, 1);
-						CKK(plk_splice_dp((plk_job_t*)e->jobs.p, ord, n_coop, ord + n_coop, n_solo,
-								(int32_t*)e->counters.p + 8 * a, (const uint8_t*)e->prep.p, trace_w,
-								(int32_t*)e->ring.p + a * ring_ints, stride, ctas, m, rows, &P, sw));
-						PL_TIME(e, sw, 1);
-						++e->last_dp_launches;
-						wave_n_coop += n_coop;
-					}
-					pos += n_coop + n_solo;
+			int32_t pos = wave_grp[w], g;
+			for (g = 0; g < 10; ++g) {
+				const plk_dp_group_t *G = &grp[w * 10 + g];
+				if (G->n_shared + G->n_solo > 0 && G->mode < 4) {
+					PL_TIME(e, sw, 1);
+					CKK(plk_splice_dp((plk_job_t*)e->jobs.p, G, (const int32_t*)e->order.p + pos,
+							(char*)e->order.p + units_off + 8 * a * max_units, (int32_t*)e->counters.p + 8 * a,
+							(const uint8_t*)e->prep.p, trace_w, ring_w, ring_stride, ring_w + ring_ints, e->n_sm * e->ctas_per_sm[G->mode][G->rows == 4], &P, sw));
+					PL_TIME(e, sw, 1);
+					++e->last_dp_launches;
+					wave_n_coop += G->n_shared;
 				}
+				pos += G->n_shared + G->n_solo;
+			}
 			PL_TIME(e, sw, 2);
-			CKK(plk_traceback((plk_job_t*)e->jobs.p, (const int32_t*)e->order.p + wave_start, pos - wave_start,
+			CKK(plk_traceback((plk_job_t*)e->jobs.p, (const int32_t*)e->order.p + wave_grp[w], pos - wave_grp[w],
 					trace_w, (uint32_t*)e->tmp.p, sw));
 			PL_TIME(e, sw, 2);
 		}
@@ -749,7 +787,7 @@ fail:
 		cudaGetLastError();
 		e->g_prev_key = 0;
 	}
-	free(wave_bytes), free(wave_cells);
+	free(wave_bytes), free(wave_cells), free(grp), free(wave_grp), free(bucket);
 	return ok;
 }
 

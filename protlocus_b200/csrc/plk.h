@@ -12,12 +12,13 @@
 extern "C" {
 #endif
 
-#define PLK_WARPS_PER_CTA 8     /* a CTA is one 256-lane wavefront (large jobs) or 8 independent warps */
+#define PLK_WARPS_PER_CTA 8     /* warps of a DP CTA, each on a strip or a job of its own */
+#define PLK_MAX_STRIPS 32768    /* strips of a job that other warps may share (k_strip_order's buckets) */
 #define PLK_ROWS 8              /* DP rows owned by one lane of a strip (extension DP) */
 /* the global DP gives every lane of a strip PLK_DP_ROWS (8) or 4 rows, chosen per job
  * (plk_job_t.rows): the trace layout, the kernel instance and the traceback follow */
 #define PLK_DP_ROWS 8
-#define PLK_RING_INTS 12        /* column state handed from one strip to the next (9 used, 48-byte entries) */
+#define PLK_RING_INTS 12        /* column state handed from one strip to the next (9 values, and 3 tags in a shared job) */
 
 /* scoring parameters and lookup tables, passed to kernels by value */
 typedef struct {
@@ -59,12 +60,13 @@ typedef struct {
 	int64_t prep_off;                /* nas[nl] | aas[al] | donor[nl+1] | acceptor[nl+1], 8-aligned */
 	int64_t trace_off;               /* first trace word (uint16) of this job in the wave arena */
 	int64_t tmp_off;                 /* reversed CIGAR scratch (uint32 words), capacity nl+al+8 */
+	int64_t ring_off;                /* shared: first int of its two-strip ring in the wave's shared rings */
 	int64_t out_off;                 /* final CIGAR offset in the output buffer (filled by the scan) */
 	int32_t nl, al;
 	int32_t mode;                    /* 0: int16 (lower clamp suffices), 1: int32 (gs32b), 2: int16 both clamps,
 	                                  * 3: int16 paired with a job of the same protein and window length */
 	int32_t slen;                    /* segment length of the striping being reproduced */
-	int32_t nw;                      /* warps cooperating on the job: 1 or PLK_WARPS_PER_CTA */
+	int32_t shared;                  /* its strips run on any warps, one each (else one warp runs them all) */
 	int32_t rows;                    /* DP rows per lane of a strip: 8 or 4 */
 	int32_t score, n_tmp;            /* outputs of the DP / traceback */
 	int32_t status;
@@ -105,21 +107,35 @@ static inline int64_t plk_prep_bytes(int32_t nl, int32_t al)
 	return ((int64_t)nl + al + 2 * ((int64_t)nl + 1) + 7) / 8 * 8;
 }
 
-/* trace words of a job in the strip layout (strips of 32*nw*rows rows) */
-static inline int64_t plk_trace_words(int32_t nl, int32_t al, int32_t nw, int32_t rows)
+/* strips of a job (32*rows rows each) and its trace words in their layout */
+static inline int64_t plk_strips(int32_t nl, int32_t rows)
 {
-	int64_t h = 32LL * nw * rows, nr = (int64_t)nl - 2, strips = (nr + h - 1) / h;
-	return strips * h * (int64_t)al;
+	const int64_t h = 32LL * rows;
+	return ((int64_t)nl - 2 + h - 1) / h;
 }
+static inline int64_t plk_trace_words(int32_t nl, int32_t al, int32_t rows)
+{
+	return plk_strips(nl, rows) * 32 * rows * (int64_t)al;
+}
+
+/* one DP launch of a wave: the jobs of one mode and row count, in the order array the shared
+ * ones first, then the solo ones */
+typedef struct {
+	int32_t mode, rows, n_shared, n_solo;
+	int32_t n_units;             /* strips of the shared jobs */
+	int32_t max_strips;          /* of one of them */
+	int64_t ring_off, ring_ints; /* their part of the wave's shared rings */
+} plk_dp_group_t;
 
 /* launchers; all return a cudaError_t value as int */
 int plk_prep(const plk_job_t *jobs, int32_t n_jobs, int32_t max_len, const uint8_t *nt, const uint8_t *aa, const uint8_t *ss,
 		uint8_t *prep, const plk_params_t *p, void *stream);
-/* order_coop: jobs run by a whole CTA (nw = PLK_WARPS_PER_CTA); order_solo: one warp each.
- * counters: 2 ints of device scratch.  ring: PLK_WARPS_PER_CTA * n_ctas * ring_stride_ints ints. */
-int plk_splice_dp(plk_job_t *jobs, const int32_t *order_coop, int32_t n_coop, const int32_t *order_solo,
-		int32_t n_solo, int32_t *counters, const uint8_t *prep, uint16_t *trace, int32_t *ring,
-		int64_t ring_stride_ints, int32_t n_ctas, int32_t mode, int32_t rows, const plk_params_t *p, void *stream);
+/* one DP launch.  order: the group's jobs; units: n_units pairs of ints of scratch; counters: 4
+ * ints of scratch.  ring: PLK_WARPS_PER_CTA * n_ctas * ring_stride_ints ints (solo jobs);
+ * sring: the wave's shared rings. */
+int plk_splice_dp(plk_job_t *jobs, const plk_dp_group_t *G, const int32_t *order, void *units, int32_t *counters,
+		const uint8_t *prep, uint16_t *trace, int32_t *ring, int64_t ring_stride_ints, int32_t *sring, int32_t n_ctas,
+		const plk_params_t *p, void *stream);
 int plk_traceback(plk_job_t *jobs, const int32_t *order, int32_t n_order, const uint16_t *trace,
 		uint32_t *tmp, void *stream);
 int plk_scan_compact(plk_job_t *jobs, int32_t n_jobs, const uint32_t *tmp, uint32_t *out, int64_t out_cap,

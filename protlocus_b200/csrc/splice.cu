@@ -7,14 +7,16 @@
  *   k_prep       per-position input preparation (nasw-sse.c:95-159): codon
  *                translation, donor/acceptor penalties with the int8 wrap of the
  *                reference, optional splice-score track.
- *   k_splice_dp  the DP.  One warp per job (persistent, jobs pulled from a
- *                length-sorted queue).  A job's rows are cut into strips of
- *                32*R rows; lane t owns rows [tR, tR+R) of the strip and walks
+ *   k_splice_dp  the DP (persistent warps).  A job's rows are cut into strips of
+ *                32*R rows; a warp takes one strip of a shared job at a time, the
+ *                strips of a job pipelined over any warps of the GPU, or the whole
+ *                of a solo job (both pulled from ordered queues).  In a strip lane t owns rows [tR, tR+R) of the strip and walks
  *                the protein columns one per step, one step behind lane t-1
  *                (anti-diagonal wavefront).  The column state of the three rows
  *                above a lane (H and D of rows i-1..i-3, A/B/C of row i-1) comes
  *                from lane t-1 by __shfl_up_sync; lane 0 gets it from lane 31 of
- *                the previous strip through a per-warp ring in L2.  The
+ *                the previous strip through a ring in L2 (tagged when another
+ *                warp wrote it).  The
  *                reference's striped schedule (vsize lanes of slen columns, a
  *                first pass with the insertion chain restarted at every segment
  *                start, then the lazy-F correction) is reproduced exactly with
@@ -93,9 +95,7 @@ __device__ __forceinline__ void store_trace(uint16_t *p, const unsigned (&z)[R])
 
 struct DpShared {
 	int32_t sct[22 * 22];                               /* score table, transposed: sct[b*22 + a] */
-	int32_t slot[2][PLK_WARPS_PER_CTA][PLK_RING_INTS];  /* warp-to-warp hand-off of a cooperative wavefront */
-	int32_t job;
-	int32_t pre[PLK_WARPS_PER_CTA][PLK_RING_INTS] __attribute__((aligned(16)));
+	int32_t pre[PLK_WARPS_PER_CTA][2][PLK_RING_INTS] __attribute__((aligned(16)));  /* lane 0's prefetched ring entries */
 	/* per warp, double-buffered by strip parity: the codons, donor and acceptor
 	 * penalties of the warp's 32*R rows of a strip, staged ahead of the strip */
 	uint8_t rows[PLK_WARPS_PER_CTA][2][3][ROWBLK] __attribute__((aligned(16)));
@@ -155,7 +155,7 @@ __device__ __forceinline__ unsigned sign_bytes(int a, int b)
 	return d;
 }
 
-template <int NW, int R>
+template <int R>
 __device__ __forceinline__ void cells_scaled(const int (&in)[9], int (&hm)[R], const int ah1, const int ah2,
 		const int ah3, const bool row2, const int *__restrict__ sct_b, const int (&code)[R],
 		const int (&gi)[R], const int (&dn)[R + 2], const int (&ac)[R + 2],
@@ -320,17 +320,17 @@ __device__ __forceinline__ void cells_plain(const int (&in)[9], int (&hm)[R], co
 	o[0] = h1, o[1] = h2, o[2] = h3, o[3] = d1, o[4] = d2, o[5] = d3, o[6] = va, o[7] = vb, o[8] = vc;
 }
 
-/* One DP job on a wavefront of NW warps (32*NW lanes).  All threads of the
- * group call this with the same job; `L` is the lane index in the wavefront. */
-template <int MODE, int NW, int R>
+/* One DP job on one warp, strip after strip: lane 0 starts the next strip while the last
+ * lanes finish the one before. */
+template <int MODE, int R>
 __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t *__restrict__ prep,
 		uint16_t *__restrict__ trace, int32_t *__restrict__ myring, DpShared &sh, const plk_params_t &P,
 		const int L, const int wib)
 {
-	constexpr int NL = 32 * NW, HS = NL * R;
+	constexpr int NL = 32, HS = NL * R;
 	constexpr int SC = MODE == 0 ? 16 : 1;                  /* value scale of the mode */
 	const int NEG = Ar<MODE>::NEG * SC;
-	const int lane = L & 31, w = L >> 5;
+	const int lane = L;
 	const int nl = J->nl, al = J->al, slen = J->slen;
 	const uint8_t *nas = prep + J->prep_off, *aas = nas + nl;
 	const int8_t *donor = (const int8_t*)(aas + al), *acceptor = donor + nl + 1;
@@ -338,7 +338,7 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 	const int nr = nl - 2, nstrip = (nr + HS - 1) / HS;
 	const int Pc = al > NL ? al : NL + 1;  /* period >= NL+1 keeps lane 0's one-step ring prefetch behind the writer */
 	const int total = nstrip * Pc + NL - 1;
-	int32_t *pre = sh.pre[wib];          /* lane 0's prefetched ring entry (cp.async target) */
+	int32_t *pre = sh.pre[wib][0];       /* lane 0's prefetched ring entry (cp.async target) */
 	uint8_t (*rowbuf)[3][ROWBLK] = sh.rows[wib];
 	const int *c16 = P.s16;             /* x16 penalties, read as kernel constants */
 	const int GOE = P.s16[8], GE16 = P.s16[1];
@@ -354,7 +354,7 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 #pragma unroll
 	for (int r = 0; r < R + 2; ++r) dn[r] = ac[r] = 0;
 	/* the first strip's row inputs, and the ring entry of the first strip (the -inf row) */
-	stage_rows<R>(rowbuf[0], nas, donor, acceptor, nl, 2 + w * 32 * R, lane);
+	stage_rows<R>(rowbuf[0], nas, donor, acceptor, nl, 2, lane);
 	if (L == 0) {
 #pragma unroll
 		for (int q = 0; q < 9; ++q) pre[q] = NEG;
@@ -368,8 +368,8 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 			 * period ago) are visible after the wait; stage those of the next strip */
 			cp_async_wait_all();
 			__syncwarp();
-			const int kn = (s - 32 * w) / Pc + 1;
-			if (kn < nstrip) stage_rows<R>(rowbuf[kn & 1], nas, donor, acceptor, nl, 2 + kn * HS + w * 32 * R, lane);
+			const int kn = s / Pc + 1;
+			if (kn < nstrip) stage_rows<R>(rowbuf[kn & 1], nas, donor, acceptor, nl, 2 + kn * HS, lane);
 		}
 		/* column state of the rows above: lane-1's output of the previous step */
 		int in[9];
@@ -377,9 +377,9 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
 		const bool started = c >= 0 && k < nstrip;
 		if (lane == 0 && started) {
-			/* the ring entry (prefetched, -inf before the second strip) or the slot of the warp above */
-			if (w == 0) cp_async_wait_all();
-			const int32_t *p = w == 0 ? pre : sh.slot[(s - 1) & 1][wib - 1];
+			/* the ring entry (prefetched, -inf before the second strip) */
+			cp_async_wait_all();
+			const int32_t *p = pre;
 			const int4 v0 = *(const int4*)p, v1 = *(const int4*)(p + 4);
 			in[0] = v0.x, in[1] = v0.y, in[2] = v0.z, in[3] = v0.w;
 			in[4] = v1.x, in[5] = v1.y, in[6] = v1.z, in[7] = v1.w, in[8] = p[8];
@@ -429,7 +429,7 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 #pragma unroll
 					for (int r = 0; r < R; ++r) ic[r] = max(ic[r] - GE16, NEG);
 				}
-				cells_scaled<NW, R>(in, hm, ah1, ah2, ah3, row2, sct_b, code, gi, dn, ac, ip, lh, ic, c16, go_e, seg_i,
+				cells_scaled<R>(in, hm, ah1, ah2, ah3, row2, sct_b, code, gi, dn, ac, ip, lh, ic, c16, go_e, seg_i,
 						o, z, hn);
 			} else {
 				cells_plain<MODE, R>(in, hm, ah1, ah2, ah3, row2, seg, first, sct_b, code, gi, dn, ac, ip, lh, ic, P,
@@ -446,14 +446,7 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
-		if (NW > 1) {
-			if (lane == 31) {
-				int32_t *sl = sh.slot[s & 1][wib];
-#pragma unroll
-				for (int q = 0; q < 9; ++q) sl[q] = o[q];
-			}
-			__syncthreads();
-		} else __syncwarp();
+		__syncwarp();
 		/* advance; lane 0 of the wavefront prefetches the ring entry of its next position */
 		++c;
 		if (c > 0) {
@@ -479,15 +472,228 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
 	}
 }
 
-/* Persistent DP kernel: first every CTA takes cooperative jobs (a whole CTA per
- * job) until that queue is empty, then every warp takes solo jobs.  Both queues
- * are sorted by decreasing size on the host (longest-processing-time first). */
+/* ------------------------------------------------------------------ one strip of a shared job
+ *
+ * A job whose strips run one after the other on a warp (or on the eight warps of a CTA, as
+ * large jobs did before) sets the end of a batch that has fewer jobs than the GPU has warps:
+ * a request's 79 strips took 4.4 ms on one SM, and the longest of 509 loci 50 ms while the
+ * rest of the GPU idled.  The only dependence between strips is the column state of the last
+ * row of strip k-1 at column c, which lane 0 of strip k needs 32 columns later at the
+ * earliest, so the strips of a job run side by side on any warps, each some 35 columns behind
+ * the one above: the unit of work is one (job, strip) pair.
+ *
+ * Hand-off.  Lane 31 writes each column's state as a 48-byte entry of three 16-byte words,
+ * each three values and the tag k + 1, into the job's ring (two strips deep, zeroed before
+ * the launch: strip k writes half k & 1).  Lane 0 of the strip below copies the entry with
+ * cp.async one column ahead (L2 is the point of coherence for both) and takes it when all
+ * three words carry its tag, else fetches again; a 16-byte aligned access is one transaction,
+ * so a word's values are those of its tag.  Strip k + 2 reaches column c only after strip
+ * k + 1 has taken the entry of column c from strip k, so no entry is overwritten before it
+ * is read and the halves need no other guard.
+ *
+ * Measured (DP launch before -> after): one 500 aa x 20 kb request 5.9 -> 2.3 ms, 96 short jobs
+ * 1.82 -> 0.44 ms, 509 loci of 1-50 kb 52.9 -> 18.7 ms; the batch of 8192 strands 291 -> 190 ms
+ * a call (its waves end without a tail of long jobs, and no block barrier holds eight warps
+ * in step).
+ *
+ * Progress.  Warps claim units by an atomic ticket in an order that has every strip after the
+ * one above it (k_strip_order), and a claimed unit runs to its end, so the strip a warp waits
+ * for is always held by a running warp: no co-residency of the grid is needed.  A wait is
+ * bounded all the same (STRIP_WAIT cycles, some ten seconds): on expiry the launch's abort
+ * word ctl[2] is set, every waiting strip goes on with what it has, and the jobs concerned
+ * get status -3.
+ */
+#define STRIP_WAIT 20000000000LL
+
+__device__ __forceinline__ void ring_fetch(int32_t *pre, const int32_t *e)
+{
+	cp_async16(pre, e), cp_async16(pre + 4, e + 4), cp_async16(pre + 8, e + 8);
+}
+
+/* the entry at e, already fetched into pre, once it carries tag; false when the wait ran out */
+__device__ __forceinline__ bool ring_take(int32_t *pre, const int32_t *e, const int tag, int32_t *ctl, int (&in)[9])
+{
+	bool ok = true;
+	cp_async_wait_all();
+	int4 v0 = *(const int4*)pre, v1 = *(const int4*)(pre + 4), v2 = *(const int4*)(pre + 8);
+	if (v0.w != tag || v1.w != tag || v2.w != tag) {
+		const long long t0 = clock64();
+		do {
+			if (*(volatile int32_t*)(ctl + 2) != 0) { ok = false; break; }
+			if (clock64() - t0 > STRIP_WAIT) { atomicExch(ctl + 2, 1); ok = false; break; }
+			ring_fetch(pre, e);
+			cp_async_wait_all();
+			v0 = *(const int4*)pre, v1 = *(const int4*)(pre + 4), v2 = *(const int4*)(pre + 8);
+		} while (v0.w != tag || v1.w != tag || v2.w != tag);
+	}
+	in[0] = v0.x, in[1] = v0.y, in[2] = v0.z, in[3] = v1.x, in[4] = v1.y, in[5] = v1.z;
+	in[6] = v2.x, in[7] = v2.y, in[8] = v2.z;
+	return ok;
+}
+
+__device__ __forceinline__ void ring_put(int32_t *e, const int tag, const int (&o)[9])
+{
+	__stcg((int4*)e, make_int4(o[0], o[1], o[2], tag));
+	__stcg((int4*)(e + 4), make_int4(o[3], o[4], o[5], tag));
+	__stcg((int4*)(e + 8), make_int4(o[6], o[7], o[8], tag));
+}
+
+/* lane 0's first entry: the -inf row above strip 0 (both buffers, tag 0), else column 0 of strip k-1 */
+__device__ __forceinline__ void strip_begin(int32_t (*pre)[PLK_RING_INTS], const int32_t *rin, const int k, const int neg,
+		const int lane)
+{
+	if (lane == 0 && k > 0) ring_fetch(pre[0], rin);
+	if (k == 0 && lane < 2 * PLK_RING_INTS) pre[0][lane] = (lane & 3) == 3 ? 0 : neg;
+	__syncwarp();
+}
+
+template <int MODE, int R>
+__device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k, const uint8_t *__restrict__ prep,
+		uint16_t *__restrict__ trace, int32_t *__restrict__ sring, int32_t *ctl, DpShared &sh, const plk_params_t &P,
+		const int lane, const int wib)
+{
+	constexpr int HS = 32 * R;
+	constexpr int SC = MODE == 0 ? 16 : 1;
+	const int NEG = Ar<MODE>::NEG * SC;
+	const int nl = J->nl, al = J->al, slen = J->slen;
+	const uint8_t *nas = prep + J->prep_off, *aas = nas + nl;
+	const int8_t *donor = (const int8_t*)(aas + al), *acceptor = donor + nl + 1;
+	uint16_t *tr = trace + J->trace_off + (int64_t)k * al * HS + lane * R;
+	const int32_t *rin = sring + J->ring_off + (int64_t)((k & 1) ^ 1) * al * PLK_RING_INTS;
+	int32_t *rout = sring + J->ring_off + (int64_t)(k & 1) * al * PLK_RING_INTS;
+	const bool more = k + 1 < (nl - 2 + HS - 1) / HS;  /* a strip below reads this one's last row */
+	int32_t (*pre)[PLK_RING_INTS] = sh.pre[wib];
+	const int *c16 = P.s16;
+	const int GOE = P.s16[8], GE16 = P.s16[1];
+	const int i0 = 2 + k * HS + lane * R;
+
+	strip_begin(pre, rin, k, NEG, lane);
+	int ip[R], lh[R], ic[R], hm[R], code[R], gi[R], dn[R + 2], ac[R + 2], o[9];
+	int ah1 = NEG, ah2 = NEG, ah3 = NEG;
+#pragma unroll
+	for (int q = 0; q < 9; ++q) o[q] = NEG;
+#pragma unroll
+	for (int r = 0; r < R; ++r) {
+		code[r] = i0 + r < nl ? nas[i0 + r] : 0;
+		gi[r] = MODE == 0 ? -16 * (code[r] == 20 ? P.fs : P.ge) : (code[r] == 20 ? P.fs : P.ge);
+		ip[r] = lh[r] = ic[r] = hm[r] = NEG;
+	}
+#pragma unroll
+	for (int r = 0; r < R + 2; ++r) {
+		const int pd = i0 - 1 + r, pa = i0 - 2 + r;
+		const int dv = pd <= nl ? donor[pd] : 0, av = pa <= nl ? acceptor[pa] : 0;
+		dn[r] = MODE == 0 ? -16 * dv : dv;
+		ac[r] = MODE == 0 ? -16 * av : av;
+	}
+	const bool rows_in = i0 < nl;
+	int cs = 0, dcol = 0;  /* dcol: s modulo al, the trace diagonal of every lane in step s */
+	for (int s = 0; s < al + 31; ++s) {
+		const int c = s - lane;
+		int in[9];
+#pragma unroll
+		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
+		if (lane == 0 && s < al) {
+			if (!ring_take(pre[s & 1], rin + (int64_t)s * PLK_RING_INTS, k, ctl, in)) J->status = -3;
+			if (k > 0 && s + 1 < al) ring_fetch(pre[(s + 1) & 1], rin + (int64_t)(s + 1) * PLK_RING_INTS);
+		}
+		const bool live = (unsigned)c < (unsigned)al && rows_in;
+		const bool any_seg = __any_sync(FULL, live && cs == 0);
+		if (live) {
+			const bool seg = cs == 0, first = c == 0, row2 = first && i0 == 2;
+			const int *sct_b = sh.sct + 22 * aas[c];
+			int hn[R];
+			unsigned z[R];
+			if (MODE == 0) { /* the segment hand-over as in dp_job */
+				const int go_e = seg ? -(1 << 28) : -c16[0], seg_i = seg ? -(1 << 28) : 0;
+				if (any_seg) {
+					const int goe_e = seg ? -GOE : -(1 << 28), ge_e = seg ? -GE16 : -(1 << 28);
+#pragma unroll
+					for (int r = 0; r < R; ++r)
+						ic[r] = __viaddmax_s32(ic[r], -GE16, __viaddmax_s32(ip[r], ge_e, __viaddmax_s32(lh[r], goe_e, NEG)));
+				} else {
+#pragma unroll
+					for (int r = 0; r < R; ++r) ic[r] = max(ic[r] - GE16, NEG);
+				}
+				cells_scaled<R>(in, hm, ah1, ah2, ah3, row2, sct_b, code, gi, dn, ac, ip, lh, ic, c16, go_e, seg_i,
+						o, z, hn);
+			} else {
+				cells_plain<MODE, R>(in, hm, ah1, ah2, ah3, row2, seg, first, sct_b, code, gi, dn, ac, ip, lh, ic, P,
+						o, z, hn);
+			}
+			store_trace<R>(tr + (int64_t)dcol * HS, z);
+			if (lane == 31 && more) ring_put(rout + (int64_t)c * PLK_RING_INTS, k + 1, o);
+#pragma unroll
+			for (int r = 0; r < R; ++r) hm[r] = hn[r];
+			ah1 = in[0], ah2 = in[1], ah3 = in[2];
+		}
+		__syncwarp();
+		if (c >= 0 && ++cs == slen) cs = 0;
+		if (++dcol == al) dcol = 0;
+	}
+	cp_async_wait_all();
+	{ /* H(nl-1, al-1): in the last strip, the lane holding row nl-1 keeps the last column in hm */
+		const int rl = nl - 1 - i0;
+		if (rl >= 0 && rl < R) {
+#pragma unroll
+			for (int r = 0; r < R; ++r)
+				if (r == rl) J->score = MODE == 0 ? hm[r] >> 4 : hm[r];
+		}
+	}
+	__syncwarp();
+}
+
+/* The claim order of the shared jobs' strips, `units`: by k / S (S strips in the job), in nb
+ * buckets, so that every job advances through its strips at the pace that ends them all
+ * together and the strips of a job come in order (nb >= S: two strips of a job never share a
+ * bucket; order inside a bucket is free).  One CTA: histogram, scan, scatter -- 30 us for the
+ * 82,000 strips of a wave of the batched workload. */
+__global__ void __launch_bounds__(1024) k_strip_order(const plk_job_t *__restrict__ jobs,
+		const int32_t *__restrict__ order, int n, int hs, int nb, int2 *__restrict__ units)
+{
+	extern __shared__ __align__(16) int32_t s_hist[];
+	__shared__ int32_t s_part[1024];
+	const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+	for (int x = tid; x < nb; x += 1024) s_hist[x] = 0;
+	__syncthreads();
+	for (int q = warp; q < n; q += 32) {
+		const unsigned S = (unsigned)(jobs[order[q]].nl - 2 + hs - 1) / (unsigned)hs;
+		for (unsigned k = lane; k < S; k += 32) atomicAdd(&s_hist[k * (unsigned)nb / S], 1);
+	}
+	__syncthreads();
+	const int per = nb / 1024;
+	int acc = 0;
+	for (int x = 0; x < per; ++x) acc += s_hist[tid * per + x];
+	s_part[tid] = acc;
+	__syncthreads();
+	for (int off = 1; off < 1024; off <<= 1) {
+		const int v = tid >= off ? s_part[tid - off] : 0;
+		__syncthreads();
+		s_part[tid] += v;
+		__syncthreads();
+	}
+	int run = s_part[tid] - acc;
+	for (int x = 0; x < per; ++x) {
+		const int h = s_hist[tid * per + x];
+		s_hist[tid * per + x] = run, run += h;
+	}
+	__syncthreads();
+	for (int q = warp; q < n; q += 32) {
+		const int j = order[q];
+		const unsigned S = (unsigned)(jobs[j].nl - 2 + hs - 1) / (unsigned)hs;
+		for (unsigned k = lane; k < S; k += 32) units[atomicAdd(&s_hist[k * (unsigned)nb / S], 1)] = make_int2(j, (int)k);
+	}
+}
+
+/* Persistent DP kernel: the warps take strips of the shared jobs until that queue is empty,
+ * then solo jobs (sorted by decreasing size on the host: small ones fill the end).  With fewer
+ * strips than warps only `active` warps of a CTA take them, which spreads the strips over the
+ * SMs. */
 template <int MODE, int R>
 __global__ void __launch_bounds__(32 * PLK_WARPS_PER_CTA, R == 8 ? 2 : 3)
-k_splice_dp(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_coop, int n_coop,
+k_splice_dp(plk_job_t *__restrict__ jobs, const int2 *__restrict__ units, int n_units, int active,
 		const int32_t *__restrict__ order_solo, int n_solo, int32_t *counters,
 		const uint8_t *__restrict__ prep, uint16_t *__restrict__ trace, int32_t *__restrict__ ring,
-		int64_t ring_stride, plk_params_t P)
+		int64_t ring_stride, int32_t *__restrict__ sring, plk_params_t P)
 {
 	__shared__ DpShared sh;
 	for (int x = threadIdx.x; x < 22 * 22; x += blockDim.x) { /* sct[b*22 + a] = s(a, b), scaled and tagged in mode 0 */
@@ -496,15 +702,13 @@ k_splice_dp(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_coop
 	}
 	__syncthreads();
 	const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-	for (;;) {
-		if (threadIdx.x == 0) sh.job = atomicAdd(&counters[0], 1);
-		__syncthreads();
-		const int idx = sh.job;
-		__syncthreads();
-		if (idx >= n_coop) break;
-		dp_job<MODE, PLK_WARPS_PER_CTA, R>(jobs + order_coop[idx], prep, trace,
-				ring + (int64_t)blockIdx.x * PLK_WARPS_PER_CTA * ring_stride, sh, P, threadIdx.x, wib);
-		__syncthreads();
+	while (wib < active) {
+		int idx = 0;
+		if (lane == 0) idx = atomicAdd(&counters[0], 1);
+		idx = __shfl_sync(FULL, idx, 0);
+		if (idx >= n_units) break;
+		const int2 u = units[idx];
+		dp_strip<MODE, R>(jobs + u.x, u.y, prep, trace, sring, counters, sh, P, lane, wib);
 	}
 	int32_t *myring = ring + ((int64_t)blockIdx.x * PLK_WARPS_PER_CTA + wib) * ring_stride;
 	for (;;) {
@@ -512,7 +716,7 @@ k_splice_dp(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_coop
 		if (lane == 0) idx = atomicAdd(&counters[1], 1);
 		idx = __shfl_sync(FULL, idx, 0);
 		if (idx >= n_solo) break;
-		dp_job<MODE, 1, R>(jobs + order_solo[idx], prep, trace, myring, sh, P, lane, wib);
+		dp_job<MODE, R>(jobs + order_solo[idx], prep, trace, myring, sh, P, lane, wib);
 		__syncwarp();
 	}
 }
@@ -550,9 +754,7 @@ k_splice_dp(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_coop
  * the traceback converts such a word to the layout of the other modes.
  */
 struct DpSharedPair {
-	int32_t slot[2][PLK_WARPS_PER_CTA][PLK_RING_INTS];
-	int32_t job;
-	int32_t pre[PLK_WARPS_PER_CTA][PLK_RING_INTS] __attribute__((aligned(16)));
+	int32_t pre[PLK_WARPS_PER_CTA][2][PLK_RING_INTS] __attribute__((aligned(16)));
 	uint8_t rows[PLK_WARPS_PER_CTA][2][2][3][ROWBLK] __attribute__((aligned(16)));  /* [warp][job][parity][array] */
 };
 #define PAIR_SCT_WORDS (22 * 22 * 22)   /* [protein residue][codon residue of job 1][of job 2] */
@@ -656,16 +858,16 @@ __device__ __forceinline__ void store_trace_pair(uint16_t *pa, uint16_t *pb, con
 	*(typename TraceVec<R>::T*)pb = *(const typename TraceVec<R>::T*)wb;
 }
 
-/* One pair of jobs on a wavefront of NW warps; the structure of dp_job with packed values. */
-template <int NW, int R>
+/* One pair of jobs on one warp; the structure of dp_job with packed values. */
+template <int R>
 __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *__restrict__ JB,
 		const uint8_t *__restrict__ prep, uint16_t *__restrict__ trace, int32_t *__restrict__ myring,
 		DpSharedPair &sh, const uint32_t *__restrict__ sct2, const PairK &K, const plk_params_t &P,
 		const int L, const int wib)
 {
-	constexpr int NL = 32 * NW, HS = NL * R;
+	constexpr int NL = 32, HS = NL * R;
 	const unsigned NEG = K.F2;
-	const int lane = L & 31, w = L >> 5;
+	const int lane = L;
 	const int nl = JA->nl, al = JA->al, slen = JA->slen;
 	const uint8_t *nasA = prep + JA->prep_off, *aas = nasA + nl;
 	const int8_t *donA = (const int8_t*)(aas + al), *accA = donA + nl + 1;
@@ -675,7 +877,7 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 	const int nr = nl - 2, nstrip = (nr + HS - 1) / HS;
 	const int Pc = al > NL ? al : NL + 1;
 	const int total = nstrip * Pc + NL - 1;
-	int32_t *pre = sh.pre[wib];
+	int32_t *pre = sh.pre[wib][0];
 	uint8_t (*rowA)[3][ROWBLK] = sh.rows[wib][0], (*rowB)[3][ROWBLK] = sh.rows[wib][1];
 	const unsigned r2h = P.pair_b * 0x10001u, r2f = (unsigned)(P.pair_b - P.fs) * 0x10001u;
 
@@ -690,8 +892,8 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 	for (int r = 0; r < R; ++r) ip[r] = lh[r] = ic[r] = hm[r] = NEG, cp[r] = 0, gi[r] = 0;
 #pragma unroll
 	for (int r = 0; r < R + 2; ++r) dn[r] = ac[r] = 0;
-	stage_rows<R>(rowA[0], nasA, donA, accA, nl, 2 + w * 32 * R, lane);
-	stage_rows<R>(rowB[0], nasB, donB, accB, nl, 2 + w * 32 * R, lane);
+	stage_rows<R>(rowA[0], nasA, donA, accA, nl, 2, lane);
+	stage_rows<R>(rowB[0], nasB, donB, accB, nl, 2, lane);
 	if (L == 0) {
 #pragma unroll
 		for (int q = 0; q < 9; ++q) pre[q] = (int32_t)NEG;
@@ -703,10 +905,10 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 		if (__shfl_sync(FULL, c, 0) == 0) {
 			cp_async_wait_all();
 			__syncwarp();
-			const int kn = (s - 32 * w) / Pc + 1;
+			const int kn = s / Pc + 1;
 			if (kn < nstrip) {
-				stage_rows<R>(rowA[kn & 1], nasA, donA, accA, nl, 2 + kn * HS + w * 32 * R, lane);
-				stage_rows<R>(rowB[kn & 1], nasB, donB, accB, nl, 2 + kn * HS + w * 32 * R, lane);
+				stage_rows<R>(rowA[kn & 1], nasA, donA, accA, nl, 2 + kn * HS, lane);
+				stage_rows<R>(rowB[kn & 1], nasB, donB, accB, nl, 2 + kn * HS, lane);
 			}
 		}
 		unsigned in[9];
@@ -714,8 +916,8 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
 		const bool started = c >= 0 && k < nstrip;
 		if (lane == 0 && started) {
-			if (w == 0) cp_async_wait_all();
-			const int32_t *p = w == 0 ? pre : sh.slot[(s - 1) & 1][wib - 1];
+			cp_async_wait_all();
+			const int32_t *p = pre;
 			const int4 v0 = *(const int4*)p, v1 = *(const int4*)(p + 4);
 			in[0] = v0.x, in[1] = v0.y, in[2] = v0.z, in[3] = v0.w;
 			in[4] = v1.x, in[5] = v1.y, in[6] = v1.z, in[7] = v1.w, in[8] = p[8];
@@ -779,14 +981,7 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
-		if (NW > 1) {
-			if (lane == 31) {
-				int32_t *sl = sh.slot[s & 1][wib];
-#pragma unroll
-				for (int q = 0; q < 9; ++q) sl[q] = (int32_t)o[q];
-			}
-			__syncthreads();
-		} else __syncwarp();
+		__syncwarp();
 		++c;
 		if (c > 0) {
 			if (++cs == slen) cs = 0;
@@ -809,12 +1004,120 @@ __device__ __forceinline__ void dp_pair(plk_job_t *__restrict__ JA, plk_job_t *_
 	}
 }
 
+/* One strip of a shared pair; dp_strip with packed values. */
+template <int R>
+__device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, const int ja, const int k,
+		const uint8_t *__restrict__ prep, uint16_t *__restrict__ trace, int32_t *__restrict__ sring, int32_t *ctl,
+		DpSharedPair &sh, const uint32_t *__restrict__ sct2, const PairK &K, const plk_params_t &P, const int lane,
+		const int wib)
+{
+	constexpr int HS = 32 * R;
+	const unsigned NEG = K.F2;
+	const plk_job_t *JA = jobs + ja, *JB = jobs + JA->pair;
+	const int nl = JA->nl, al = JA->al, slen = JA->slen;
+	const uint8_t *aas = prep + JA->prep_off + nl;
+	const int64_t toff = (int64_t)k * al * HS + lane * R;
+	uint16_t *trA = trace + JA->trace_off + toff, *trB = trace + JB->trace_off + toff;
+	int32_t *rout = sring + JA->ring_off + (int64_t)(k & 1) * al * PLK_RING_INTS;
+	const int rdif = (k & 1 ? -al : al);  /* columns from rout to the half that strip k-1 writes */
+	const bool more = k + 1 < (nl - 2 + HS - 1) / HS;
+	int32_t (*pre)[PLK_RING_INTS] = sh.pre[wib];
+	const unsigned r2h = P.pair_b * 0x10001u, r2f = (unsigned)(P.pair_b - P.fs) * 0x10001u;
+	const int i0 = 2 + k * HS + lane * R;
+
+	strip_begin(pre, rout + (int64_t)rdif * PLK_RING_INTS, k, (int)NEG, lane);
+	unsigned ip[R], lh[R], ic[R], hm[R], gi[R], dn[R + 2], ac[R + 2], o[9];
+	int cp[R];
+	unsigned ah1 = NEG, ah2 = NEG, ah3 = NEG;
+#pragma unroll
+	for (int q = 0; q < 9; ++q) o[q] = NEG;
+	{
+		const uint8_t *nasA = prep + JA->prep_off, *nasB = prep + JB->prep_off;
+		const int8_t *donA = (const int8_t*)(nasA + nl + al), *accA = donA + nl + 1;
+		const int8_t *donB = (const int8_t*)(nasB + nl + al), *accB = donB + nl + 1;
+#pragma unroll
+		for (int r = 0; r < R; ++r) {
+			const int i = i0 + r, ca = i < nl ? nasA[i] : 0, cb = i < nl ? nasB[i] : 0;
+			cp[r] = ca * 22 + cb;
+			gi[r] = pk16(-(ca == 20 ? P.fs : P.ge), -(cb == 20 ? P.fs : P.ge));
+			ip[r] = lh[r] = ic[r] = hm[r] = NEG;
+		}
+#pragma unroll
+		for (int r = 0; r < R + 2; ++r) {
+			const int pd = i0 - 1 + r, pa = i0 - 2 + r;
+			dn[r] = pk16(pd <= nl ? -donA[pd] : 0, pd <= nl ? -donB[pd] : 0);
+			ac[r] = pk16(pa <= nl ? -accA[pa] : 0, pa <= nl ? -accB[pa] : 0);
+		}
+	}
+	const bool rows_in = i0 < nl;
+	int cs = 0, dcol = 0;  /* dcol: s modulo al, the trace diagonal of every lane in step s */
+	for (int s = 0; s < al + 31; ++s) {
+		const int c = s - lane;
+		unsigned in[9];
+#pragma unroll
+		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
+		if (lane == 0 && s < al) {
+			int v[9];
+			if (!ring_take(pre[s & 1], rout + (int64_t)(rdif + s) * PLK_RING_INTS, k, ctl, v))
+				jobs[ja].status = jobs[jobs[ja].pair].status = -3;
+#pragma unroll
+			for (int q = 0; q < 9; ++q) in[q] = (unsigned)v[q];
+			if (k > 0 && s + 1 < al) ring_fetch(pre[(s + 1) & 1], rout + (int64_t)(rdif + s + 1) * PLK_RING_INTS);
+		}
+		const bool live = (unsigned)c < (unsigned)al && rows_in;
+		const bool any_seg = __any_sync(FULL, live && cs == 0);
+		if (live) {
+			const bool seg = cs == 0, row2 = c == 0 && i0 == 2;
+			const uint32_t *srow = sct2 + 484 * aas[c];
+			unsigned hn[R], z[R];
+			const unsigned go_e = seg ? 0x80008000u : K.GOn, seg_i = seg ? 0x80008000u : 0u;
+			if (any_seg) {
+				const unsigned goe_e = seg ? K.GOEn : 0x80008000u, ge_e = seg ? K.GEn : 0x80008000u;
+#pragma unroll
+				for (int r = 0; r < R; ++r)
+					ic[r] = __viaddmax_s16x2(ic[r], K.GEn, __viaddmax_s16x2(ip[r], ge_e, __viaddmax_s16x2(lh[r], goe_e, NEG)));
+			} else {
+#pragma unroll
+				for (int r = 0; r < R; ++r) ic[r] = __viaddmax_s16x2(ic[r], K.GEn, NEG);
+			}
+			cells_pair<R>(in, hm, ah1, ah2, ah3, row2, r2h, r2f, srow, cp, gi, dn, ac, ip, lh, ic, K, P, go_e, seg_i,
+					o, z, hn);
+			store_trace_pair<R>(trA + (int64_t)dcol * HS, trB + (int64_t)dcol * HS, z);
+			if (lane == 31 && more) {
+				int v[9];
+#pragma unroll
+				for (int q = 0; q < 9; ++q) v[q] = (int)o[q];
+				ring_put(rout + (int64_t)c * PLK_RING_INTS, k + 1, v);
+			}
+#pragma unroll
+			for (int r = 0; r < R; ++r) hm[r] = hn[r];
+			ah1 = in[0], ah2 = in[1], ah3 = in[2];
+		}
+		__syncwarp();
+		if (c >= 0 && ++cs == slen) cs = 0;
+		if (++dcol == al) dcol = 0;
+	}
+	cp_async_wait_all();
+	{ /* H(nl-1, al-1) of both jobs, unbiased */
+		const int rl = nl - 1 - i0;
+		if (rl >= 0 && rl < R) {
+#pragma unroll
+			for (int r = 0; r < R; ++r)
+				if (r == rl) {
+					jobs[ja].score = (int)(hm[r] & 0xffffu) - P.pair_b;
+					jobs[jobs[ja].pair].score = (int)(hm[r] >> 16) - P.pair_b;
+				}
+		}
+	}
+	__syncwarp();
+}
+
 template <int R>
 __global__ void __launch_bounds__(32 * PLK_WARPS_PER_CTA, R == 8 ? 2 : 3)
-k_splice_pair(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_coop, int n_coop,
+k_splice_pair(plk_job_t *__restrict__ jobs, const int2 *__restrict__ units, int n_units, int active,
 		const int32_t *__restrict__ order_solo, int n_solo, int32_t *counters,
 		const uint8_t *__restrict__ prep, uint16_t *__restrict__ trace, int32_t *__restrict__ ring,
-		int64_t ring_stride, plk_params_t P)
+		int64_t ring_stride, int32_t *__restrict__ sring, plk_params_t P)
 {
 	__shared__ DpSharedPair sh;
 	extern __shared__ __align__(16) uint32_t pair_sct[];  /* [a][ca][cb] = s(ca, a) | s(cb, a) << 16 */
@@ -829,16 +1132,13 @@ k_splice_pair(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_co
 	K.ONE = 0x00010001u;
 	__syncthreads();
 	const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-	for (;;) {
-		if (threadIdx.x == 0) sh.job = atomicAdd(&counters[0], 1);
-		__syncthreads();
-		const int idx = sh.job;
-		__syncthreads();
-		if (idx >= n_coop) break;
-		plk_job_t *J = jobs + order_coop[idx];
-		dp_pair<PLK_WARPS_PER_CTA, R>(J, jobs + J->pair, prep, trace,
-				ring + (int64_t)blockIdx.x * PLK_WARPS_PER_CTA * ring_stride, sh, pair_sct, K, P, threadIdx.x, wib);
-		__syncthreads();
+	while (wib < active) {
+		int idx = 0;
+		if (lane == 0) idx = atomicAdd(&counters[0], 1);
+		idx = __shfl_sync(FULL, idx, 0);
+		if (idx >= n_units) break;
+		const int2 u = units[idx];
+		dp_strip_pair<R>(jobs, u.x, u.y, prep, trace, sring, counters, sh, pair_sct, K, P, lane, wib);
 	}
 	int32_t *myring = ring + ((int64_t)blockIdx.x * PLK_WARPS_PER_CTA + wib) * ring_stride;
 	for (;;) {
@@ -847,7 +1147,7 @@ k_splice_pair(plk_job_t *__restrict__ jobs, const int32_t *__restrict__ order_co
 		idx = __shfl_sync(FULL, idx, 0);
 		if (idx >= n_solo) break;
 		plk_job_t *J = jobs + order_solo[idx];
-		dp_pair<1, R>(J, jobs + J->pair, prep, trace, myring, sh, pair_sct, K, P, lane, wib);
+		dp_pair<R>(J, jobs + J->pair, prep, trace, myring, sh, pair_sct, K, P, lane, wib);
 		__syncwarp();
 	}
 }
@@ -886,13 +1186,13 @@ __device__ __forceinline__ void tb_push(TbOut &T, uint32_t op, int len)
 #define TB_WARPS 8
 
 /* the R trace words of chunk ch (R rows of one lane of a strip) in column col, into w[0..R) */
-__device__ __forceinline__ void tb_load_chunk(const uint16_t *__restrict__ tr, int R, int nlanes, int al, int ch, int col,
+__device__ __forceinline__ void tb_load_chunk(const uint16_t *__restrict__ tr, int R, int al, int ch, int col,
 		uint16_t (&w)[8])
 {
-	const int ra = ch * R, hs = nlanes * R, k = ra / hs, t = ch % nlanes;
+	const int k = ch / 32, t = ch % 32;
 	int d = col + t;
 	if (d >= al) d %= al;
-	const uint16_t *src = tr + (((int64_t)k * al + d) * nlanes + t) * R;
+	const uint16_t *src = tr + (((int64_t)k * al + d) * 32 + t) * R;
 	if (R == 8) {
 		const uint4 v = *(const uint4*)src;
 		*(uint4*)w = v;
@@ -921,7 +1221,7 @@ __device__ __forceinline__ void tb_norm8(uint16_t (&w)[8], const bool pair)
 /* the highest row <= i of column j whose extension bit is clear, among the 32*C R-row chunks
  * down from chunk ch_top (lane l reads chunks l, l + 32, ...); -1 when none is */
 template <int C>
-__device__ __forceinline__ int tb_scan(const uint16_t *__restrict__ tr, const int R, const int nlanes, const int al,
+__device__ __forceinline__ int tb_scan(const uint16_t *__restrict__ tr, const int R, const int al,
 		const int ch_top, const int lane, const int j, const int i, const int bit, const bool pair)
 {
 	int end_row = -1;
@@ -929,7 +1229,7 @@ __device__ __forceinline__ int tb_scan(const uint16_t *__restrict__ tr, const in
 #pragma unroll
 	for (int m = 0; m < C; ++m) {
 		const int ch = ch_top - lane - 32 * m;
-		if (ch >= 0) tb_load_chunk(tr, R, nlanes, al, ch, j, w[m]);
+		if (ch >= 0) tb_load_chunk(tr, R, al, ch, j, w[m]);
 	}
 #pragma unroll
 	for (int m = 0; m < C; ++m) {
@@ -959,7 +1259,6 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 	const uint16_t *tr = trace + J->trace_off;
 	TbOut T;  /* lane 0's */
 	T.out = tmp + J->tmp_off, T.cur = 0, T.n = 0;
-	const int nlanes = 32 * J->nw;
 	const bool pair = J->mode == 3;
 	int i = nl - 1, j = al - 1, last = 0;
 	while (i >= 2 && j >= 0) {
@@ -971,12 +1270,12 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 			const int g = qc - dq, col = jc - dc;
 			if (g >= 0 && col >= 0) {
 				__align__(16) uint16_t w[8];
-				if (R == 8) tb_load_chunk(tr, 8, nlanes, al, g, col, w);
+				if (R == 8) tb_load_chunk(tr, 8, al, g, col, w);
 				else {
-					/* chunks 2g and 2g+1 sit in the same strip (nlanes is even) */
+					/* chunks 2g and 2g+1 sit in the same strip */
 					__align__(8) uint16_t w2[8];
-					tb_load_chunk(tr, 4, nlanes, al, 2 * g, col, w);
-					tb_load_chunk(tr, 4, nlanes, al, 2 * g + 1, col, w2);
+					tb_load_chunk(tr, 4, al, 2 * g, col, w);
+					tb_load_chunk(tr, 4, al, 2 * g + 1, col, w2);
 					*(uint2*)(w + 4) = *(const uint2*)w2;
 				}
 				tb_norm8(w, pair);
@@ -1022,8 +1321,8 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 			const int ch_top = (i - 2) / R, bit = tb_ext_bit(last);
 			const int op = last == 3 ? NS_CIGAR_N : (last == 4 ? NS_CIGAR_U : NS_CIGAR_V);
 			int end_row = -1;
-			if (wide) end_row = tb_scan<4>(tr, R, nlanes, al, ch_top, lane, j, i, bit, pair);
-			else end_row = tb_scan<1>(tr, R, nlanes, al, ch_top, lane, j, i, bit, pair);
+			if (wide) end_row = tb_scan<4>(tr, R, al, ch_top, lane, j, i, bit, pair);
+			else end_row = tb_scan<1>(tr, R, al, ch_top, lane, j, i, bit, pair);
 			const int low = max(2, (ch_top - (wide ? 127 : 31)) * R + 2);
 			wide = 1;
 			if (end_row >= low) { /* the run ends at end_row: its step clears the state (and moves j for U/V) */
@@ -1131,23 +1430,42 @@ extern "C" int plk_dp_ctas_per_sm(int32_t mode, int32_t rows)
 	return mode == 1 ? dp_occupancy<1, 8>() : mode == 2 ? dp_occupancy<2, 8>() : dp_occupancy<0, 8>();
 }
 
-extern "C" int plk_splice_dp(plk_job_t *jobs, const int32_t *order_coop, int32_t n_coop, const int32_t *order_solo,
-		int32_t n_solo, int32_t *counters, const uint8_t *prep, uint16_t *trace, int32_t *ring,
-		int64_t ring_stride_ints, int32_t n_ctas, int32_t mode, int32_t rows, const plk_params_t *p, void *stream)
+extern "C" int plk_splice_dp(plk_job_t *jobs, const plk_dp_group_t *G, const int32_t *order, void *units,
+		int32_t *counters, const uint8_t *prep, uint16_t *trace, int32_t *ring, int64_t ring_stride_ints, int32_t *sring,
+		int32_t n_ctas, const plk_params_t *p, void *stream)
 {
-	if (n_coop + n_solo <= 0) return 0;
+	const int32_t n_units = G->n_units, n_solo = G->n_solo, rows = G->rows, mode = G->mode;
+	const int32_t *order_solo = order + G->n_shared;
+	if (n_units + n_solo <= 0) return 0;
 	if (rows != 4 && rows != 8) return (int)cudaErrorInvalidValue;
 	cudaStream_t st = (cudaStream_t)stream;
-	cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(int32_t), st);
+	cudaError_t e = cudaMemsetAsync(counters, 0, 4 * sizeof(int32_t), st);  /* strip ticket, solo ticket, abort */
 	if (e != cudaSuccess) return (int)e;
-	const dim3 grid(n_ctas), block(32 * PLK_WARPS_PER_CTA);
-#define DP_LAUNCH(M, RR) k_splice_dp<M, RR><<<grid, block, 0, st>>>(jobs, order_coop, n_coop, order_solo, n_solo, \
-		counters, prep, trace, ring, ring_stride_ints, *p)
-	if (mode == 3) { /* pairs: order_* hold the first job of each pair (jobs[q].pair: the second) */
-		if (rows == 4) k_splice_pair<4><<<grid, block, PAIR_SMEM, st>>>(jobs, order_coop, n_coop, order_solo, n_solo,
-				counters, prep, trace, ring, ring_stride_ints, *p);
-		else k_splice_pair<8><<<grid, block, PAIR_SMEM, st>>>(jobs, order_coop, n_coop, order_solo, n_solo,
-				counters, prep, trace, ring, ring_stride_ints, *p);
+	int active = PLK_WARPS_PER_CTA, ctas = n_ctas;
+	if (n_units > 0) {
+		int nb = 1024;
+		while (nb < G->max_strips) nb <<= 1;
+		if (nb > PLK_MAX_STRIPS) return (int)cudaErrorInvalidValue;
+		/* no stale tag may match: this group's part of the ring starts at zero */
+		if ((e = cudaMemsetAsync(sring + G->ring_off, 0, sizeof(int32_t) * (size_t)G->ring_ints, st)) != cudaSuccess) return (int)e;
+		if (nb * 4 > 40 * 1024 && (e = cudaFuncSetAttribute(k_strip_order, cudaFuncAttributeMaxDynamicSharedMemorySize,
+				PLK_MAX_STRIPS * 4)) != cudaSuccess) return (int)e;
+		k_strip_order<<<1, 1024, (size_t)nb * 4, st>>>(jobs, order, G->n_shared, 32 * rows, nb, (int2*)units);
+		if ((e = cudaGetLastError()) != cudaSuccess) return (int)e;
+		__sync_fetch_and_add(&g_launches, 1ull);
+		active = (n_units + n_ctas - 1) / n_ctas;
+		if (active > PLK_WARPS_PER_CTA) active = PLK_WARPS_PER_CTA;
+		if (n_solo == 0 && n_units < ctas) ctas = n_units;
+	} else active = 0;
+	const dim3 grid(ctas), block(32 * PLK_WARPS_PER_CTA);
+	const int2 *u = (const int2*)units;
+#define DP_LAUNCH(M, RR) k_splice_dp<M, RR><<<grid, block, 0, st>>>(jobs, u, n_units, active, order_solo, n_solo, \
+		counters, prep, trace, ring, ring_stride_ints, sring, *p)
+	if (mode == 3) { /* pairs: order holds the first job of each pair (jobs[q].pair: the second) */
+		if (rows == 4) k_splice_pair<4><<<grid, block, PAIR_SMEM, st>>>(jobs, u, n_units, active, order_solo, n_solo,
+				counters, prep, trace, ring, ring_stride_ints, sring, *p);
+		else k_splice_pair<8><<<grid, block, PAIR_SMEM, st>>>(jobs, u, n_units, active, order_solo, n_solo,
+				counters, prep, trace, ring, ring_stride_ints, sring, *p);
 	} else if (rows == 4) {
 		if (mode == 1) DP_LAUNCH(1, 4); else if (mode == 2) DP_LAUNCH(2, 4); else DP_LAUNCH(0, 4);
 	} else {
