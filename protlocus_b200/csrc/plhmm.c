@@ -26,32 +26,71 @@ struct pl_hmm_profile_s {
 	uint8_t codon[64];     /* the same, on the host */
 };
 
+/* Columns a lane (2-8) when the paired 16-bit kernel can take the profile, else 0.  With no
+ * transition above 0 a state is at most bound = m * (largest emission); a transition below
+ * -(bound + emax + 1) or an emission below -(bound + 1) then sends every state to the DP's
+ * clamp at 0 as that floor does, and with 2 * bound + emax + 2 <= 32767 no sum of a state and
+ * the two wraps. */
+static int pl_hmm_cols(int32_t m, const int16_t *emit, const int16_t *trans, int32_t *t_floor, int32_t *e_floor)
+{
+	int64_t bound;
+	int32_t emax = 0, cols, tiles = (m + PLK_HMM_TILE - 1) / PLK_HMM_TILE;
+	size_t x;
+	for (x = 0; x < (size_t)m * 20; ++x) if (emit[x] > emax) emax = emit[x];
+	for (x = 0; x < (size_t)m * 7; ++x) if (trans[x] > 0) return 0;
+	bound = (int64_t)m * emax;
+	if (2 * bound + emax + 2 > 32767) return 0;
+	*t_floor = -(int32_t)(bound + emax + 1), *e_floor = -(int32_t)(bound + 1);
+	cols = plk_hmm_smem_bytes(tiles * PLK_HMM_TILE, 8) > 0 ? (m + 32 * tiles - 1) / (32 * tiles) : 8;
+	return cols < 2 ? 2 : cols;
+}
+
 PL_EXPORT pl_hmm_profile_t *pl_hmm_profile_create(int32_t device, int32_t m, const int16_t *emit,
 		const int16_t *trans, const uint8_t *codon_alpha)
 {
 	pl_hmm_profile_t *p;
 	int16_t *e = 0;
+	uint32_t *e32 = 0;
 	int32_t *t = 0;
-	int32_t mpad, j, k;
+	int32_t mpad, j, k, cols, t_floor = 0, e_floor = 0;
 	if (m <= 0 || !emit || !trans || !codon_alpha) { pl_set_error("pl_hmm_profile_create: empty profile"); return 0; }
 	for (k = 0; k < 64; ++k)
 		if (codon_alpha[k] > 20) { pl_set_error("codon_alpha[%d] = %d (HMMER columns 0-19, 20 = none)", k, codon_alpha[k]); return 0; }
 	mpad = (m + PLK_HMM_TILE - 1) / PLK_HMM_TILE * PLK_HMM_TILE;
 	p = (pl_hmm_profile_t*)calloc(1, sizeof(*p));
-	e = (int16_t*)calloc((size_t)21 * mpad, sizeof(int16_t));
+	e = (int16_t*)calloc((size_t)21 * mpad, sizeof(uint32_t));  /* either kernel's table */
 	t = (int32_t*)malloc(sizeof(int32_t) * 7 * (size_t)mpad);
 	if (!p || !e || !t) { pl_set_error("out of host memory"); goto fail; }
-	for (j = 0; j < m; ++j) /* column j holds profile position j (the DP's column j+1) */
-		for (k = 0; k < 20; ++k) e[(size_t)k * mpad + j] = emit[(size_t)j * 20 + k];
-	for (k = 0; k < 7; ++k)
-		for (j = 0; j < mpad; ++j) t[(size_t)k * mpad + j] = j < m ? trans[(size_t)j * 7 + k] : -(1 << 28);
+	cols = pl_hmm_cols(m, emit, trans, &t_floor, &e_floor);
+	if (cols == 0) {
+		for (j = 0; j < m; ++j) /* column j holds profile position j (the DP's column j+1) */
+			for (k = 0; k < 20; ++k) e[(size_t)k * mpad + j] = emit[(size_t)j * 20 + k];
+		for (k = 0; k < 7; ++k)
+			for (j = 0; j < mpad; ++j) t[(size_t)k * mpad + j] = j < m ? trans[(size_t)j * 7 + k] : -(1 << 28);
+	} else {
+		e32 = (uint32_t*)e;
+		const uint32_t none = ((uint32_t)t_floor & 0xffffu) * 0x10001u;
+		for (j = 0; j < 7 * mpad; ++j) t[j] = (int32_t)none;
+		for (j = 0; j < m; ++j) { /* the slot of column j in the paired kernel's tables */
+			const size_t x = (size_t)(j / (32 * cols)) * PLK_HMM_TILE + (size_t)(j % (32 * cols) / cols) * 8 + j % cols;
+			for (k = 0; k < 20; ++k) {
+				const int32_t v = emit[(size_t)j * 20 + k];
+				e32[(size_t)k * mpad + x] = (uint32_t)(v < e_floor ? e_floor : v) & 0xffffu;
+			}
+			for (k = 0; k < 7; ++k) {
+				const int32_t v = trans[(size_t)j * 7 + k];
+				t[(size_t)k * mpad + x] = (int32_t)(((uint32_t)(v < t_floor ? t_floor : v) & 0xffffu) * 0x10001u);
+			}
+		}
+	}
+	p->k.cols = cols, p->k.hi = 65536;
 	p->device = device, p->k.m = m, p->k.mpad = mpad;
 	memcpy(p->codon, codon_alpha, 64);
 	CK(cudaSetDevice(device));
-	CK(cudaMalloc((void**)&p->k.emit_t, sizeof(int16_t) * 21 * (size_t)mpad));
+	CK(cudaMalloc((void**)&p->k.emit_t, (cols ? sizeof(uint32_t) : sizeof(int16_t)) * 21 * (size_t)mpad));
 	CK(cudaMalloc((void**)&p->k.trans_t, sizeof(int32_t) * 7 * (size_t)mpad));
 	CK(cudaMalloc((void**)&p->codon_dev, 64));
-	CK(cudaMemcpy((void*)p->k.emit_t, e, sizeof(int16_t) * 21 * (size_t)mpad, cudaMemcpyHostToDevice));
+	CK(cudaMemcpy((void*)p->k.emit_t, e, (cols ? sizeof(uint32_t) : sizeof(int16_t)) * 21 * (size_t)mpad, cudaMemcpyHostToDevice));
 	CK(cudaMemcpy((void*)p->k.trans_t, t, sizeof(int32_t) * 7 * (size_t)mpad, cudaMemcpyHostToDevice));
 	CK(cudaMemcpy(p->codon_dev, codon_alpha, 64, cudaMemcpyHostToDevice));
 	free(e), free(t);
@@ -132,21 +171,23 @@ static int pl_hmm_plan(pl_engine_t *e, int32_t n, const int32_t *len, int64_t **
 static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, const uint8_t *nt_dev,
 		const int32_t *off, const int32_t *len, int32_t *score_dev, cudaStream_t st)
 {
-	int64_t *row_off, rows_total, cells = 0;
-	int32_t *order, max_rows, ctas, q;
+	int64_t *row_off, rows_total, cells = 0, edge_rows;
+	int32_t *order, max_rows, ctas, units, q;
 	if (n <= 0) return 1;
 	if (!p) { pl_set_error("no profile"); return 0; }
 	if (p->device != e->device) { pl_set_error("profile on device %d, engine on device %d", p->device, e->device); return 0; }
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
+	edge_rows = ((int64_t)max_rows + 3) / 4 * 4 + 4;  /* the paired kernel walks rows in fours */
 	for (q = 0; q < n; ++q) cells += (int64_t)(len[q] >= 3 ? len[q] / 3 : 0) * p->k.m;
-	ctas = plk_hmm_ctas_per_sm(p->k.mpad);
+	ctas = plk_hmm_ctas_per_sm(&p->k);
 	if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
 	ctas *= e->n_sm;
-	if ((int64_t)ctas * plk_hmm_warps_per_cta() > n) ctas = (n + plk_hmm_warps_per_cta() - 1) / plk_hmm_warps_per_cta();
+	units = p->k.cols ? (n + 1) / 2 : n;  /* the paired kernel takes two regions a warp */
+	if ((int64_t)ctas * plk_hmm_warps_per_cta() > units) ctas = (units + plk_hmm_warps_per_cta() - 1) / plk_hmm_warps_per_cta();
 	if (!dbuf_ensure(&e->h_off, sizeof(int32_t) * (size_t)n) || !dbuf_ensure(&e->h_len, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rowoff, sizeof(int64_t) * (size_t)n) || !dbuf_ensure(&e->h_order, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rows, (size_t)(rows_total > 0 ? rows_total : 16)) || !dbuf_ensure(&e->h_counter, 64) ||
-			!dbuf_ensure(&e->h_edge, (size_t)16 * 2 * (size_t)(max_rows + 1) * (size_t)ctas * plk_hmm_warps_per_cta()))
+			!dbuf_ensure(&e->h_edge, (size_t)16 * 2 * (size_t)edge_rows * (size_t)ctas * plk_hmm_warps_per_cta()))
 		return 0;
 	CK(cudaMemcpyAsync(e->h_off.p, off, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->h_len.p, len, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
@@ -159,7 +200,7 @@ static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, cons
 	PL_TIME(e, st, 0);
 	PL_TIME(e, st, 1);
 	CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
-			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, (int64_t)max_rows + 1, ctas,
+			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, edge_rows, ctas,
 			score_dev, st));
 	PL_TIME(e, st, 1);
 	CK(cudaStreamSynchronize(st));
@@ -194,7 +235,7 @@ PL_EXPORT int pl_hmm_score_device(pl_engine_t *e, const pl_hmm_profile_t *p, int
 PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *const *ps, int32_t n_prof, int32_t n,
 		const uint8_t *nt, const int32_t *off, const int32_t *len, int32_t *score_dev, void *stream)
 {
-	int64_t *row_off, rows_total, cells = 0, rows_sum = 0;
+	int64_t *row_off, rows_total, cells = 0, rows_sum = 0, edge_rows;
 	int32_t *order, max_rows, q, k, s, warps;
 	const uint8_t *codon = 0;
 	cudaStream_t st;
@@ -206,6 +247,7 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	CK(cudaSetDevice(e->device));
 	st = stream ? (cudaStream_t)stream : e->stream;
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
+	edge_rows = ((int64_t)max_rows + 3) / 4 * 4 + 4;  /* the paired kernel walks rows in fours */
 	for (q = 0; q < n; ++q) rows_sum += len[q] >= 3 ? len[q] / 3 : 0;
 	warps = plk_hmm_warps_per_cta();
 	for (s = 0; s < PL_HMM_STREAMS; ++s)
@@ -225,11 +267,12 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	PL_TIME(e, st, 1);
 	for (k = 0; k < n_prof; ++k) {
 		const pl_hmm_profile_t *p = ps[k];
-		int32_t ctas = plk_hmm_ctas_per_sm(p->k.mpad);
+		int32_t ctas = plk_hmm_ctas_per_sm(&p->k), units;
 		cudaStream_t sk;
 		if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
 		ctas *= e->n_sm;
-		if ((int64_t)ctas * warps > n) ctas = (n + warps - 1) / warps;
+		units = p->k.cols ? (n + 1) / 2 : n;
+		if ((int64_t)ctas * warps > units) ctas = (units + warps - 1) / warps;
 		if (!codon || memcmp(codon, p->codon, 64) != 0) {  /* the rows of this codon table, then fork again */
 			if (codon) {  /* every launch reading the previous rows has finished */
 				for (s = 0; s < PL_HMM_STREAMS; ++s) {
@@ -244,10 +287,10 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 			codon = p->codon;
 		}
 		s = k % PL_HMM_STREAMS, sk = e->h_st[s];
-		if (!dbuf_ensure(&e->h_edge_s[s], (size_t)16 * 2 * (size_t)(max_rows + 1) * (size_t)ctas * warps)) return 0;
+		if (!dbuf_ensure(&e->h_edge_s[s], (size_t)16 * 2 * (size_t)edge_rows * (size_t)ctas * warps)) return 0;
 		CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
 				(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p + 16 * s, e->h_edge_s[s].p,
-				(int64_t)max_rows + 1, ctas, score_dev + (int64_t)k * n, sk));
+				edge_rows, ctas, score_dev + (int64_t)k * n, sk));
 		cells += rows_sum * p->k.m;
 	}
 	for (s = 0; s < PL_HMM_STREAMS; ++s) {  /* join */

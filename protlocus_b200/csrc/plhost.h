@@ -54,7 +54,7 @@ struct pl_engine_s {
 	dbuf_t h_off, h_len, h_rowoff, h_rows, h_order, h_counter, h_edge, h_nt, h_score;
 	/* several profiles at once: concurrent launches on PL_HMM_STREAMS streams, each with its
 	 * own queue counter and edge buffer */
-#define PL_HMM_STREAMS 4
+#define PL_HMM_STREAMS 8
 	cudaStream_t h_st[PL_HMM_STREAMS];
 	cudaEvent_t h_ev[PL_HMM_STREAMS + 1];
 	dbuf_t h_edge_s[PL_HMM_STREAMS];

@@ -90,12 +90,18 @@ typedef struct {
 
 /* a profile of the integer HMM DP on the device (hmm.c:14-22 tables, re-laid out) */
 typedef struct {
-	const int16_t *emit_t;   /* [21][mpad]: emissions by HMMER column (row 20: zeros, no emission), column j-1 */
+	const void *emit_t;      /* [21][mpad]: emissions by HMMER column (row 20: zeros, no emission), column j-1;
+	                            int16, paired kernel: uint32 with the value in the low half */
 	const int32_t *trans_t;  /* [7][mpad]: m->m, m->i, m->d, i->m, i->i, d->m, d->d of column j-1; -2^28 beyond m */
-	int32_t m, mpad;         /* profile length, padded to the 256-column tile */
+	int32_t m, mpad;         /* profile length; table width, 256 per tile */
+	int32_t cols;            /* > 0: columns a lane of the paired kernel, whose tables hold column
+	                            j-1 at tile * 256 + lane * 8 + c and each transition in both halves;
+	                            0: the 32-bit kernel, 8 columns a lane */
+	uint32_t hi;             /* 65536, read as a kernel constant: a shift would issue on the ALU pipe */
 } plk_hmm_prof_t;
 #define PLK_HMM_TILE 256
-#define PLK_HMM_SMEM_MAX (96 * 1024)  /* emissions staged in shared memory up to mpad = 2048 */
+#define PLK_HMM_SMEM_MAX (96 * 1024)   /* emissions staged in shared memory up to mpad = 2048, */
+#define PLK_HMM_SMEM_PAIR (172 * 1024) /* in the paired kernel's 32-bit words too */
 
 /* bytes after the last job's preparation scratch that the DP may read (its row
  * inputs are copied in whole 16-byte chunks) */
@@ -162,9 +168,9 @@ int plk_hmm_codons(const uint8_t *nt, const int32_t *off, const int32_t *len, co
 int plk_hmm_dp(const plk_hmm_prof_t *p, const uint8_t *rows, const int64_t *row_off, const int32_t *len,
 		const int32_t *order, int32_t n, int32_t *counter, void *edge, int64_t edge_stride_rows, int32_t n_ctas,
 		int32_t *score, void *stream);
-int plk_hmm_ctas_per_sm(int32_t mpad);
+int plk_hmm_ctas_per_sm(const plk_hmm_prof_t *p);
 int plk_hmm_warps_per_cta(void);
-int plk_hmm_smem_bytes(int32_t mpad);
+int plk_hmm_smem_bytes(int32_t mpad, int32_t cols);  /* 0: read from global memory */
 /* gapless prefilter: one warp per candidate; steps accumulates the extension steps walked */
 int plk_gapless(const uint8_t *packed, int64_t bases, const uint8_t *queries, int64_t query_aa, const void *cand,
 		int32_t n_cand, const void *anchors, int64_t n_anchors, int32_t block_width, int32_t kmer, int32_t xdrop,
