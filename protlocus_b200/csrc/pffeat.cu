@@ -5,17 +5,32 @@
  *
  *  1. the protein's aa 5-mers go into a shared-memory hash table (4096 slots, first
  *     occurrence kept) and its aa 3-mers into 256 composition bins;
- *  2. the window is translated in chunks of 4096 codon ends (all three frames: every
- *     position is the end of a codon) into shared memory; each codon end adds its
- *     window 3-mer to 256 more bins and looks its 5-mer up in the table: a hit is an
- *     anchor (window position, protein position);
- *  3. the anchors are sorted by position (bitonic, shared memory) and one warp chains
- *     them: the longest chain increasing in both coordinates whose nucleotide gap is
- *     not shorter than 3x the residue gap minus 60 (frameshift slack);
+ *  2. the window is translated (all three frames: every position is the end of a
+ *     codon); each codon end adds its window 3-mer to 256 more bins and looks its
+ *     5-mer up in the table: a hit is an anchor (window position, protein position).
+ *     The scan is the work (24,000 positions a candidate).  Each warp takes a
+ *     contiguous part of the window, a lane 16 consecutive positions of it from one
+ *     aligned 16-byte load, and everything between the bases and the two lookups stays
+ *     in registers: the codes and residues before a lane's own come from the lane (or
+ *     the step) before by shuffles, so the scan has no barrier.  The lookup tables sit
+ *     in shared memory (as kernel constants their divergent reads serialised), and a
+ *     65,536-bit map of the protein's 5-mers, 0.6 % full for a 420-residue protein,
+ *     sends few warps to the hash table;
+ *  3. the anchors are sorted by position and chained: the longest chain increasing in
+ *     both coordinates whose nucleotide gap is not shorter than 3x the residue gap
+ *     minus 60 (frameshift slack).  A lane holds one anchor of a block of 32: the
+ *     eight warps take the predecessors before the block among them, then one warp
+ *     the block's own, each final anchor broadcast to the later ones (no reduction per
+ *     anchor); the chain's sums come by pointer jumping instead of a walk;
  *  4. features: the 512 composition bins (scaled so a uniform composition is 1) and 20
  *     scalars of the anchors and the best chain (counts, coverage, span, frame
  *     changes, the window positions where the protein would start and end); the chain
  *     ends are also returned as integers for window tightening.
+ *
+ * Measured, 16,384 candidates of 2,048 proteins (393 M positions): the kernel 4.6 -> 1.2 ms
+ * (tables and scan in bytes 4.6 -> 2.3, the chain without a reduction per anchor 1.8, no
+ * branch per position 1.2); it issues on 65 % of the slots, the rest mostly waits on the
+ * barriers around the chain.
  *
  * Feature row layout (bf16, F_DIM = 576 columns): [0,256) protein 3-mer bins,
  * [256,512) window 3-mer bins, [512,532) scalars, [532,576) zero.
@@ -31,32 +46,31 @@ namespace {
 
 constexpr int THREADS = 256;
 constexpr int HSLOTS = 4096;
-constexpr int CH = 4096;
 constexpr int MAXA = 1024;
 constexpr int F_DIM = PLK_PF_FDIM;
 constexpr uint8_t BAD = 255;
 
 struct FeatSmem {
-	int32_t hkey[HSLOTS];
-	int32_t hpos[HSLOTS];
+	union {
+		struct { int32_t hkey[HSLOTS], hpos[HSLOTS]; };
+		struct { /* the chain, once the scan is done */
+			int32_t p[MAXA], r[MAXA], f[MAXA], up[2][MAXA], sum[2][MAXA], part[THREADS / 32][32];
+		} c;
+	};
 	int32_t bins[512];
 	int64_t akey[MAXA];
-	int32_t f[MAXA], prev[MAXA];
-	uint8_t aab[CH + 16];
+	uint32_t map[2048];            /* word hmul(code) >> 21, bit code & 31 of every 5-mer in the table */
+	uint8_t nt4[256], aa20[256], codon[64];
 	int32_t n_anchor, tot_p, tot_w;
 	int32_t chain[8];
 };
 
-__device__ __forceinline__ uint32_t h5(uint32_t code) { return (code * 2654435761u) >> 20; }          /* 12 bits */
+__device__ __forceinline__ uint32_t hmul(uint32_t code) { return code * 2654435761u; }
+__device__ __forceinline__ uint32_t h5(uint32_t h) { return h >> 20; }                                /* slot: 12 bits */
 __device__ __forceinline__ uint32_t h3(uint32_t code) { return ((code * 40503u) >> 8) & 255u; }
 
-__device__ __forceinline__ uint8_t codon_aa(const uint8_t *nt, int64_t p, const plk_pf_tabs_t &T)
-{
-	const uint8_t a = T.nt4[nt[p - 2]], b = T.nt4[nt[p - 1]], c = T.nt4[nt[p]];
-	if ((a | b | c) > 3) return BAD;
-	const uint8_t x = T.codon[a * 16 + b * 4 + c];
-	return x < 20 ? x : BAD;
-}
+/* bit 7 of a word's four bytes, in order */
+__device__ __forceinline__ uint32_t high_bits(const uint32_t w) { return (((w >> 7) & 0x01010101u) * 0x10204080u) >> 28; }
 
 __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 {
@@ -69,8 +83,16 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 	const int32_t nl = C.nl, al = C.al;
 	const uint8_t *nt = A.nt + C.nt_off;
 	const uint8_t *aa = A.aa + C.aa_off;
-	const plk_pf_tabs_t &T = A.tabs;
-
+	for (int i = tid; i < 256; i += THREADS) {
+		const uint8_t c = A.tabs.nt4[i];
+		S.nt4[i] = c > 3 ? 0x80 : c;  /* bit 7: no base */
+		S.aa20[i] = A.tabs.aa20[i];
+	}
+	for (int i = tid; i < 64; i += THREADS) {
+		const uint8_t x = A.tabs.codon[i];
+		S.codon[i] = x < 20 ? x : BAD;
+	}
+	for (int i = tid; i < 2048; i += THREADS) S.map[i] = 0;
 	for (int i = tid; i < HSLOTS; i += THREADS) S.hkey[i] = 0, S.hpos[i] = 0x7fffffff;
 	for (int i = tid; i < 512; i += THREADS) S.bins[i] = 0;
 	if (tid == 0) S.n_anchor = 0, S.tot_p = 0, S.tot_w = 0;
@@ -83,7 +105,7 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 		bool ok = true;
 		const int w = p >= 4 ? 5 : p + 1;
 		for (int k = 0; k < w; ++k) {
-			const uint8_t x = T.aa20[aa[p - k]];
+			const uint8_t x = S.aa20[aa[p - k]];
 			r[k] = x < 20 ? x : BAD;
 			if (r[k] == BAD) ok = false;
 		}
@@ -93,7 +115,9 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 		}
 		if (p >= 4 && ok) {
 			const uint32_t code = (((r[4] * 20u + r[3]) * 20u + r[2]) * 20u + r[1]) * 20u + r[0];
-			uint32_t s = h5(code);
+			const uint32_t h = hmul(code);
+			uint32_t s = h5(h);
+			atomicOr(&S.map[h >> 21], 1u << (code & 31));
 			for (int t = 0; t < HSLOTS; ++t, s = (s + 1) & (HSLOTS - 1)) {
 				const int32_t old = atomicCAS(&S.hkey[s], 0, (int32_t)code + 1);
 				if (old == 0 || old == (int32_t)code + 1) { atomicMin(&S.hpos[s], p); break; }
@@ -103,99 +127,188 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 	atomicAdd(&S.tot_p, cnt3);
 	__syncthreads();
 
-	/* 2. window scan */
+	/* 2. window scan, in groups of 16 positions P = p + a0 that start at 16-byte boundaries of the
+	 * bases.  Warp w takes groups [gb, ge); its first step starts a group early, uncounted, for
+	 * the codes and residues that reach into the part */
 	int cntw = 0;
-	for (int64_t cs = 0; cs < nl; cs += CH) {
-		/* aab[j] = residue of the codon ending at cs - 12 + j */
-		for (int j = tid; j < CH + 12; j += THREADS) {
-			const int64_t p = cs - 12 + j;
-			S.aab[j] = (p >= 2 && p < nl) ? codon_aa(nt, p, T) : BAD;
-		}
-		__syncthreads();
-		for (int j = 12 + tid; j < CH + 12; j += THREADS) {
-			const int64_t p = cs - 12 + j;
-			if (p >= nl) break;
-			const uint8_t a0 = S.aab[j], a1 = S.aab[j - 3], a2 = S.aab[j - 6];
-			if (a0 == BAD || a1 == BAD || a2 == BAD) continue;
-			atomicAdd(&S.bins[256 + h3((uint32_t)a2 * 400u + a1 * 20u + a0)], 1);
-			++cntw;
-			const uint8_t a3 = S.aab[j - 9], a4 = S.aab[j - 12];
-			if (a3 == BAD || a4 == BAD) continue;
-			const uint32_t code = (((a4 * 20u + a3) * 20u + a2) * 20u + a1) * 20u + a0;
-			uint32_t s = h5(code);
-			for (int t = 0; t < HSLOTS; ++t, s = (s + 1) & (HSLOTS - 1)) {
-				const int32_t key = S.hkey[s];
-				if (key == 0) break;
-				if (key == (int32_t)code + 1) {
-					const int idx = atomicAdd(&S.n_anchor, 1);
-					if (idx < MAXA) S.akey[idx] = (p << 20) | (int64_t)S.hpos[s];  /* both coordinates are k-mer ends */
-					break;
+	{
+		const int a0 = (int)((uintptr_t)nt & 15);
+		const uint4 *ntv = reinterpret_cast<const uint4 *>(nt - a0);
+		const int ng = (int)(((int64_t)nl + a0 + 15) / 16), gb = (int)((int64_t)ng * warp / (THREADS / 32)),
+				ge = (int)((int64_t)ng * (warp + 1) / (THREADS / 32));
+		/* of the position group before lane 0's: 2 codes with their marks, 12 residues */
+		uint32_t pc = 0x30000000u, p1 = ~0u, p2 = ~0u, p3 = ~0u;
+		for (int g0 = gb - 1; gb < ge && g0 < ge; g0 += 32) {
+			const int g = g0 + lane;
+			const int64_t p0 = 16 * (int64_t)g - a0;  /* the group's first position in the window */
+			uint32_t x[4];
+			if (p0 >= 0 && p0 + 16 <= nl && g < ge) {
+				const uint4 q4 = __ldg(ntv + g);
+				x[0] = q4.x, x[1] = q4.y, x[2] = q4.z, x[3] = q4.w;
+			}
+			/* codes: two bits each, the first position highest; bad: bit k = position k has no base */
+			uint32_t cw = 0, bad = 0, any = 0x80;
+			if (p0 >= 0 && p0 + 16 <= nl && g < ge) {
+				any = 0;
+#pragma unroll
+				for (int k = 0; k < 16; ++k) {
+					const uint32_t t = S.nt4[__byte_perm(x[k >> 2], 0, 0x4440 + (k & 3))];
+					cw = cw * 4 + t, any |= t;
+				}
+			}
+			if (any & 0x80) { /* an N, or the window's ends: one position at a time */
+				cw = 0;
+				for (int k = 0; k < 16; ++k) {
+					const int64_t p = p0 + k;
+					const uint32_t t = p >= 0 && p < nl && g < ge ? S.nt4[nt[p]] : 0x80u;
+					cw = cw * 4 + (t & 3), bad |= (t >> 7) << k;
+				}
+			}
+			/* residues of the 16 codons: the two codes before come from the lane before */
+			const uint32_t last = (cw & 15) | (bad >> 14) << 28;
+			uint32_t before = __shfl_up_sync(0xffffffffu, last, 1);
+			if (lane == 0) before = pc;
+			pc = __shfl_sync(0xffffffffu, last, 31);
+			const uint32_t bb = bad << 2 | before >> 28, badc = bb | bb >> 1 | bb >> 2;  /* bit k: the codon ending at k */
+			uint32_t v[28], o[4];
+#pragma unroll
+			for (int k = 0; k < 16; ++k) {
+				const uint32_t idx = k < 2 ? ((before & 15) << (2 * k + 2) | cw >> (30 - 2 * k)) & 63 : cw >> (30 - 2 * k) & 63;
+				v[12 + k] = S.codon[idx];
+				o[k >> 2] = k & 3 ? o[k >> 2] + (v[12 + k] << (8 * (k & 3))) : v[12 + k];
+			}
+			uint32_t rb = high_bits(o[0]) | high_bits(o[1]) << 4 | high_bits(o[2]) << 8 | high_bits(o[3]) << 12;
+			rb |= badc & 0xffffu;
+			/* the 12 residues before and their marks (a byte with bit 7) */
+			const uint32_t m1 = (rb >> 4 & 15) * 0x00204081u & 0x01010101u, m2 = (rb >> 8 & 15) * 0x00204081u & 0x01010101u,
+					m3 = (rb >> 12 & 15) * 0x00204081u & 0x01010101u;
+			const uint32_t s1 = o[1] | m1 << 7, s2 = o[2] | m2 << 7, s3 = o[3] | m3 << 7;
+			uint32_t b1 = __shfl_up_sync(0xffffffffu, s1, 1), b2 = __shfl_up_sync(0xffffffffu, s2, 1),
+					b3 = __shfl_up_sync(0xffffffffu, s3, 1);
+			if (lane == 0) b1 = p1, b2 = p2, b3 = p3;
+			p1 = __shfl_sync(0xffffffffu, s1, 31), p2 = __shfl_sync(0xffffffffu, s2, 31), p3 = __shfl_sync(0xffffffffu, s3, 31);
+			const uint32_t m = high_bits(b1) | high_bits(b2) << 4 | high_bits(b3) << 8 | rb << 12;  /* bit i: v[i] is none */
+			const uint32_t bad3 = m | m << 3 | m << 6, bad5 = bad3 | m << 9 | m << 12;
+			if (g < gb || g >= ge || (bad3 >> 12 & 0xffffu) == 0xffffu) continue;
+			cntw += __popc(~bad3 & 0x0ffff000u);
+			uint32_t pr[28];
+#pragma unroll
+			for (int k = 0; k < 12; ++k) v[k] = __byte_perm(k < 4 ? b1 : k < 8 ? b2 : b3, 0, 0x4440 + (k & 3));
+#pragma unroll
+			for (int i = 3; i < 28; ++i) pr[i] = v[i - 3] * 20u + v[i];
+			uint32_t hits = 0;  /* bit i: the map has the 5-mer ending at v[i] */
+#pragma unroll
+			for (int i = 12; i < 28; ++i) {
+				const uint32_t tri = v[i - 6] * 400u + pr[i];
+				if (!(bad3 >> i & 1)) atomicAdd(&S.bins[256 + h3(tri)], 1);
+				const uint32_t code = pr[i - 9] * 8000u + tri, w = S.map[hmul(code) >> 21];
+				hits |= __funnelshift_r(w, w, code - i) & (1u << i);
+			}
+			hits &= ~bad5;
+			while (hits) {  /* few lanes have one: the 5-mer again, from its bytes */
+				const int i = __ffs(hits) - 1;
+				hits &= hits - 1;
+				uint32_t code = 0;
+#pragma unroll
+				for (int k = 4; k >= 0; --k) {
+					const int at = i - 3 * k;  /* byte of b1 b2 b3 o[0] .. o[3] */
+					const uint32_t w = at < 4 ? b1 : at < 8 ? b2 : at < 12 ? b3 : at < 16 ? o[0] : at < 20 ? o[1] : at < 24 ? o[2] : o[3];
+					code = code * 20u + (w >> (8 * (at & 3)) & 255);
+				}
+				uint32_t sl = h5(hmul(code));
+				for (int t = 0; t < HSLOTS; ++t, sl = (sl + 1) & (HSLOTS - 1)) {
+					const int32_t key = S.hkey[sl];
+					if (key == 0) break;
+					if (key == (int32_t)code + 1) {
+						const int at = atomicAdd(&S.n_anchor, 1);
+						/* both coordinates are k-mer ends */
+						if (at < MAXA) S.akey[at] = ((p0 + i - 12) << 20) | (int64_t)S.hpos[sl];
+						break;
+					}
 				}
 			}
 		}
-		__syncthreads();
 	}
 	atomicAdd(&S.tot_w, cntw);
 	__syncthreads();
 
-	/* 3. sort the kept anchors by (position, protein position) and chain them */
+	/* 3. sort the kept anchors by (position, protein position) -- all keys differ -- and chain them */
 	const int na_all = S.n_anchor, na = na_all < MAXA ? na_all : MAXA;
-	int np2 = 1;
-	while (np2 < na) np2 <<= 1;
-	for (int i = na + tid; i < np2; i += THREADS) S.akey[i] = INT64_MAX;
-	__syncthreads();
-	for (int k = 2; k <= np2; k <<= 1)
-		for (int j = k >> 1; j > 0; j >>= 1) {
-			for (int i = tid; i < np2; i += THREADS) {
-				const int l = i ^ j;
-				if (l > i) {
-					const int64_t a = S.akey[i], b = S.akey[l];
-					const bool up = (i & k) == 0;
-					if ((a > b) == up) S.akey[i] = b, S.akey[l] = a;
+	if (na <= THREADS) { /* an anchor per thread: its rank by counting */
+		int rank = 0;
+		const int64_t key = tid < na ? S.akey[tid] : 0;
+		if (tid < na)
+			for (int k = 0; k < na; ++k) rank += S.akey[k] < key;
+		if (tid < na) S.c.p[rank] = (int32_t)(key >> 20), S.c.r[rank] = (int32_t)(key & 0xFFFFF);
+		__syncthreads();
+	} else {
+		int np2 = 1;
+		while (np2 < na) np2 <<= 1;
+		for (int i = na + tid; i < np2; i += THREADS) S.akey[i] = INT64_MAX;
+		__syncthreads();
+		for (int k = 2; k <= np2; k <<= 1)
+			for (int j = k >> 1; j > 0; j >>= 1) {
+				for (int i = tid; i < np2; i += THREADS) {
+					const int l = i ^ j;
+					if (l > i) {
+						const int64_t a = S.akey[i], b = S.akey[l];
+						const bool up = (i & k) == 0;
+						if ((a > b) == up) S.akey[i] = b, S.akey[l] = a;
+					}
 				}
+				__syncthreads();
 			}
-			__syncthreads();
+		for (int i = tid; i < na; i += THREADS) S.c.p[i] = (int32_t)(S.akey[i] >> 20), S.c.r[i] = (int32_t)(S.akey[i] & 0xFFFFF);
+		__syncthreads();
+	}
+	for (int b0 = 0; b0 < na; b0 += 32) {
+		const int j = b0 + lane;
+		const int32_t pj = j < na ? S.c.p[j] : 0, rj = j < na ? S.c.r[j] : 0;  /* lanes past the end take nothing: r >= 4 */
+		int32_t best = 0;  /* f * 2048 + k + 1 of the best predecessor: ties to the largest k */
+		for (int k = warp; k < b0; k += THREADS / 32) {
+			const int32_t pk = S.c.p[k], rk = S.c.r[k];
+			if (pk < pj && rk < rj && pj - pk >= 3 * (rj - rk) - 60) best = max(best, S.c.f[k] * 2048 + k + 1);
 		}
+		S.c.part[warp][lane] = best;
+		__syncthreads();
+		if (warp == 0) {
+			for (int w = 1; w < THREADS / 32; ++w) best = max(best, S.c.part[w][lane]);
+			for (int k = 0; k < 32; ++k) {
+				const int32_t fk = (__shfl_sync(0xffffffffu, best, k) >> 11) + 1, pk = __shfl_sync(0xffffffffu, pj, k),
+						rk = __shfl_sync(0xffffffffu, rj, k);
+				if (k < lane && pk < pj && rk < rj && pj - pk >= 3 * (rj - rk) - 60) best = max(best, fk * 2048 + b0 + k + 1);
+			}
+			if (j < na) {
+				const int32_t u = best ? (best & 2047) - 1 : j;  /* a chain's first anchor points at itself */
+				S.c.f[j] = (best >> 11) + 1;
+				S.c.up[0][j] = u;
+				/* its link to the one before: a frame change (high half) and the residues it covers */
+				S.c.sum[0][j] = u == j ? 0 : ((pj % 3 != S.c.p[u] % 3) << 16) + min(5, rj - S.c.r[u]);
+			}
+		}
+		__syncthreads();
+	}
+	int buf = 0;
+	for (int d = 1; d < na; d <<= 1, buf ^= 1) { /* sums over the links back to the chain's start */
+		for (int j = tid; j < na; j += THREADS) {
+			const int u = S.c.up[buf][j];
+			S.c.sum[buf ^ 1][j] = S.c.sum[buf][j] + S.c.sum[buf][u];
+			S.c.up[buf ^ 1][j] = S.c.up[buf][u];
+		}
+		__syncthreads();
+	}
 	if (warp == 0) {
-		for (int j = 0; j < na; ++j) {
-			const int64_t kj = S.akey[j];
-			const int64_t pj = kj >> 20;
-			const int32_t rj = (int32_t)(kj & 0xFFFFF);
-			int32_t best = 0;  /* f * 2048 + k + 1 of the best predecessor */
-			for (int k = lane; k < j; k += 32) {
-				const int64_t kk = S.akey[k];
-				const int64_t pk = kk >> 20;
-				const int32_t rk = (int32_t)(kk & 0xFFFFF);
-				if (pk < pj && rk < rj && (pj - pk) >= 3LL * (rj - rk) - 60) {
-					const int32_t v = S.f[k] * 2048 + k + 1;
-					best = v > best ? v : best;
-				}
-			}
+		int32_t top = 0;  /* the first anchor with the largest f */
+		for (int j = lane; j < na; j += 32) top = max(top, S.c.f[j] * 2048 + 2047 - j);
 #pragma unroll
-			for (int o = 16; o >= 1; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-			if (lane == 0) {
-				S.f[j] = best ? (best >> 11) + 1 : 1;
-				S.prev[j] = best ? (best & 2047) - 1 : -1;
-			}
-			__syncwarp();
-		}
+		for (int o = 16; o >= 1; o >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, o));
 		if (lane == 0) {
-			int jb = -1, fb = 0;
-			for (int j = 0; j < na; ++j) if (S.f[j] > fb) fb = S.f[j], jb = j;
-			int32_t len = 0, fc = 0, cov = 0, first_p = -1, last_p = -1, first_r = -1, last_r = -1, nxt_r = -1, nxt_p = -1;
-			for (int j = jb; j >= 0; j = S.prev[j]) {
-				const int32_t pj = (int32_t)(S.akey[j] >> 20), rj = (int32_t)(S.akey[j] & 0xFFFFF);
-				if (len == 0) last_p = pj, last_r = rj;
-				else {
-					if ((nxt_p % 3) != (pj % 3)) ++fc;
-					cov += min(5, nxt_r - rj);
-				}
-				first_p = pj, first_r = rj, nxt_p = pj, nxt_r = rj;
-				++len;
-			}
-			if (len > 0) cov += 5;
-			S.chain[0] = len, S.chain[1] = fc, S.chain[2] = cov;
-			S.chain[3] = first_p, S.chain[4] = last_p, S.chain[5] = first_r, S.chain[6] = last_r;
+			const int jb = 2047 - (top & 2047), first = na ? S.c.up[buf][jb] : 0;
+			S.chain[0] = na ? top >> 11 : 0;
+			S.chain[1] = na ? S.c.sum[buf][jb] >> 16 : 0;
+			S.chain[2] = na ? (S.c.sum[buf][jb] & 0xffff) + 5 : 0;
+			S.chain[3] = na ? S.c.p[first] : -1, S.chain[4] = na ? S.c.p[jb] : -1;
+			S.chain[5] = na ? S.c.r[first] : -1, S.chain[6] = na ? S.c.r[jb] : -1;
 		}
 	}
 	__syncthreads();
