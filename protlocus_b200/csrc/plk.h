@@ -237,7 +237,10 @@ typedef struct {
 } plk_seed_args_t;
 int plk_seed_sketch(const plk_seed_args_t *a, void *stream);
 int plk_seed_take(const plk_seed_args_t *a, void *stream);
-int plk_seed_emit(const plk_seed_args_t *a, void *stream);
+int plk_seed_emit(const plk_seed_args_t *a, const int32_t *list, int32_t n_list, void *stream);
+#define PLK_SEED_CLASSES 4
+#define PLK_SEED_CLASS(c) (2048 << (c))
+int plk_seed_anchors(const plk_seed_args_t *a, const int32_t *list, int32_t n_list, int32_t cls, uint64_t *out, void *stream);
 /* profiles: every state's offered groups; the windows' seeds appended to each protein's own */
 int plk_seed_hmm_alts(const plk_seed_args_t *a, void *stream);
 int plk_seed_hmm_enum(const plk_seed_args_t *a, void *stream);

@@ -105,6 +105,14 @@ static int64_t pl_seed_hmm_slots(int32_t n, const int32_t *len, const pl_seed_hm
 	return t;
 }
 
+/* the class of plk_seed_anchors that holds n anchors, PLK_SEED_CLASSES past the largest */
+static int pl_seed_class(int64_t n)
+{
+	int c = 0;
+	while (c < PLK_SEED_CLASSES && n > PLK_SEED_CLASS(c)) ++c;
+	return c;
+}
+
 /* the batch's anchors: into the host array a (when they fit a_cap), or left on the device
  * (a_dev != 0: *a_dev at the engine's sorted array); h with seed_max > 0: HMM-profile queries */
 static int64_t pl_seed_run(pl_engine_t *e, const pl_seed_index_t *x, int32_t n, const uint8_t *seq, int64_t seq_len,
@@ -114,7 +122,7 @@ static int64_t pl_seed_run(pl_engine_t *e, const pl_seed_index_t *x, int32_t n, 
 	const int rescue = o && o->repeat_cap > 0, hmm = h && h->seed_max > 0;
 	const int32_t max_occ = o ? o->max_occ : 0;
 	plk_seed_args_t A;
-	int64_t *na = 0, *soff = 0, total = 0, ret = -1, n_slot;
+	int64_t *na = 0, *soff = 0, *pack = 0, total = 0, ret = -1, n_slot;
 	int32_t q;
 	size_t tmp_bytes = 0;
 	cudaStream_t st;
@@ -222,17 +230,47 @@ static int64_t pl_seed_run(pl_engine_t *e, const pl_seed_index_t *x, int32_t n, 
 	ret = total;
 	if (a_dev) *a_dev = 0;
 	if (total == 0 || (!a_dev && total > a_cap)) goto done;  /* a_off only: the caller grows a to a_off[n] */
-	if (!dbuf_ensure(&e->s_anc, sizeof(uint64_t) * (size_t)total) || !dbuf_ensure(&e->s_anc2, sizeof(uint64_t) * (size_t)total))
-		goto fail;
-	CK(cudaMemcpyAsync(e->s_aoff.p, a_off, sizeof(int64_t) * (size_t)(n + 1), cudaMemcpyHostToDevice, st));
-	A.a_off = (const int64_t*)e->s_aoff.p, A.anchors = (uint64_t*)e->s_anc.p;
-	PL_TIME(e, st, 1);
-	CKK(plk_seed_emit(&A, st));
-	CKK(plk_seed_sort((const uint64_t*)e->s_anc.p, (uint64_t*)e->s_anc2.p, total, n, (const int64_t*)e->s_aoff.p, 0, 0,
-			&tmp_bytes, st));
-	if (!dbuf_ensure(&e->s_tmp, tmp_bytes > 0 ? tmp_bytes : 16)) goto fail;
-	CKK(plk_seed_sort((const uint64_t*)e->s_anc.p, (uint64_t*)e->s_anc2.p, total, n, (const int64_t*)e->s_aoff.p, 0,
-			e->s_tmp.p, &tmp_bytes, st));
+	{ /* by anchor count: the classes sorted in shared memory, then the proteins past them, whose
+	   * anchors go through memory and the segmented sort */
+		int32_t cnt[PLK_SEED_CLASSES + 1], pos[PLK_SEED_CLASSES + 1], n_big, c;
+		int32_t *list;
+		int64_t *seg;
+		memset(cnt, 0, sizeof(cnt));
+		for (q = 0; q < n; ++q) ++cnt[pl_seed_class(na[q])];
+		n_big = cnt[PLK_SEED_CLASSES];
+		pack = (int64_t*)malloc(sizeof(int64_t) * (size_t)(n + 1 + 2 * n_big) + sizeof(int32_t) * (size_t)n);
+		if (!pack) { pl_set_error("out of host memory"); goto fail; }
+		seg = pack + n + 1, list = (int32_t*)(seg + 2 * n_big);
+		memcpy(pack, a_off, sizeof(int64_t) * (size_t)(n + 1));
+		for (c = 0, pos[0] = 0; c < PLK_SEED_CLASSES; ++c) pos[c + 1] = pos[c] + cnt[c];
+		for (q = 0; q < n; ++q) {
+			c = pl_seed_class(na[q]);
+			if (c == PLK_SEED_CLASSES) {
+				const int32_t i = pos[c] - (n - n_big);
+				seg[i] = a_off[q], seg[n_big + i] = a_off[q + 1];
+			}
+			list[pos[c]++] = q;
+		}
+		if (!dbuf_ensure(&e->s_aoff, sizeof(int64_t) * (size_t)(n + 1 + 2 * n_big) + sizeof(int32_t) * (size_t)n) ||
+				!dbuf_ensure(&e->s_anc2, sizeof(uint64_t) * (size_t)total) ||
+				(n_big > 0 && !dbuf_ensure(&e->s_anc, sizeof(uint64_t) * (size_t)total)))
+			goto fail;
+		CK(cudaMemcpyAsync(e->s_aoff.p, pack, sizeof(int64_t) * (size_t)(n + 1 + 2 * n_big) + sizeof(int32_t) * (size_t)n,
+				cudaMemcpyHostToDevice, st));
+		A.a_off = (const int64_t*)e->s_aoff.p, A.anchors = (uint64_t*)e->s_anc.p;
+		seg = (int64_t*)e->s_aoff.p + n + 1, list = (int32_t*)(seg + 2 * n_big);
+		PL_TIME(e, st, 1);
+		for (c = PLK_SEED_CLASSES - 1; c >= 0; --c)
+			CKK(plk_seed_anchors(&A, list + pos[c] - cnt[c], cnt[c], c, (uint64_t*)e->s_anc2.p, st));
+		if (n_big > 0) {
+			CKK(plk_seed_emit(&A, list + (n - n_big), n_big, st));
+			CKK(plk_seed_sort((const uint64_t*)e->s_anc.p, (uint64_t*)e->s_anc2.p, total, n_big, seg, seg + n_big, 0, &tmp_bytes,
+					st));
+			if (!dbuf_ensure(&e->s_tmp, tmp_bytes > 0 ? tmp_bytes : 16)) goto fail;
+			CKK(plk_seed_sort((const uint64_t*)e->s_anc.p, (uint64_t*)e->s_anc2.p, total, n_big, seg, seg + n_big, e->s_tmp.p,
+					&tmp_bytes, st));
+		}
+	}
 	PL_TIME(e, st, 1);
 	if (a_dev) *a_dev = (const uint64_t*)e->s_anc2.p;
 	else CK(cudaMemcpyAsync(a, e->s_anc2.p, sizeof(uint64_t) * (size_t)total, cudaMemcpyDeviceToHost, st));
@@ -247,10 +285,10 @@ done:
 		}
 		e->acc_dp_launches += e->n_ev / 2;
 	}
-	free(na), free(soff);
+	free(na), free(soff), free(pack);
 	return ret;
 fail:
-	free(na), free(soff);
+	free(na), free(soff), free(pack);
 	return -1;
 }
 

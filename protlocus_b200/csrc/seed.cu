@@ -12,15 +12,17 @@
  *                  in position order, their bucket sizes (32 lookups in flight), the cap
  *                  (the 25 % and 75 % order statistics of the sizes by a warp radix
  *                  select) and the anchor count.
- *   k_seed_emit    one warp per protein: 32 seeds at a time, their kept buckets laid out by
- *                  a warp scan, the lanes copy the blocks as block << 32 | position.
+ *   k_seed_anchors one CTA per protein of at most 16,384 anchors: the blocks of its kept
+ *                  buckets as block << 32 | position into shared memory (32 seeds at a time
+ *                  per warp, laid out by a warp scan), sorted there, written once.
+ *   k_seed_emit    the larger proteins' anchors to memory, for the segmented sort.
  * HMM-profile queries (the query the profile's consensus, mp_sketch_query with a profile,
  * map.c:332-343) add the profile-derived seeds of mp_sketch_hmm (sketch.c:40-118) before
  * the cap: k_seed_hmm_alts (a thread per match state: its offered groups), k_seed_hmm_enum
  * (a warp per protein, a lane per window: the seeds appended after the protein's own), a
  * segmented sort and k_seed_unique (duplicates removed, then the cap as in the sketch).
- * The anchors of each protein are then sorted (cub::DeviceSegmentedSort, ascending 64-bit
- * keys: equal keys are equal values, so any sort leaves the reference's array).
+ * The anchors of each protein are sorted ascending as 64-bit keys (equal keys are equal
+ * values, so any sort leaves the reference's array).
  */
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -63,8 +65,13 @@ __device__ __forceinline__ int64_t sd_warp_sum(int64_t v)
  * values that share the bits chosen so far and have a 0 next are counted */
 __device__ uint32_t sd_select(const uint32_t *v, const int32_t n, int64_t k, const int lane)
 {
-	uint32_t prefix = 0, mask = 0;
-	for (int bit = 31; bit >= 0; --bit) {
+	uint32_t prefix = 0, top = 0;
+	for (int32_t j = lane; j < n; j += 32) top |= v[j];
+#pragma unroll
+	for (int o = 16; o >= 1; o >>= 1) top |= __shfl_xor_sync(0xffffffffu, top, o);
+	const int bits = 32 - __clz(top);  /* no value has a bit above these */
+	uint32_t mask = bits < 32 ? ~0u << bits : 0;
+	for (int bit = bits - 1; bit >= 0; --bit) {
 		const uint32_t m = mask | 1u << bit;
 		int64_t c = 0;
 		for (int32_t j = lane; j < n; j += 32) c += (v[j] & m) == prefix;
@@ -189,59 +196,218 @@ __global__ void __launch_bounds__(256) k_seed_take(plk_seed_args_t A)
 	if (lane == 0) A.n_anchor[q] = n_base + n_res;
 }
 
-#define SD_EMIT_WARPS 8
-__global__ void __launch_bounds__(32 * SD_EMIT_WARPS) k_seed_emit(plk_seed_args_t A)
+/* what a warp holds of 32 seeds: exclusive scan of their takes, their buckets */
+struct SdGroup {
+	int64_t st[32], sz[32];
+	int32_t pre[33];
+	uint32_t pos[32];
+};
+
+/* seeds j0 .. j0+31 of a protein into G; returns their anchors */
+__device__ __forceinline__ int32_t sd_group(const plk_seed_args_t &A, SdGroup &G, const uint64_t *sd, const int32_t *take,
+		const int32_t n, const int32_t j0, const int lane)
 {
-	__shared__ int64_t s_pre[SD_EMIT_WARPS][33], s_st[SD_EMIT_WARPS][32];
-	__shared__ uint32_t s_pos[SD_EMIT_WARPS][32];
-	__shared__ int64_t s_sz[SD_EMIT_WARPS][32];
+	const int32_t j = j0 + lane;
+	int64_t st = 0, sz = 0;
+	int32_t tk = 0;
+	uint32_t pos = 0;
+	if (j < n) {
+		const int64_t b = (int64_t)(sd[j] >> 32);
+		st = A.ki[b];
+		sz = (b + 1 < A.n_bucket ? A.ki[b + 1] : A.n_kb) - st;
+		tk = take[j];
+		pos = (uint32_t)sd[j];
+	}
+	int32_t inc = tk;
+#pragma unroll
+	for (int o = 1; o < 32; o <<= 1) {
+		const int32_t t = __shfl_up_sync(0xffffffffu, inc, o);
+		if (lane >= o) inc += t;
+	}
+	__syncwarp();
+	G.pre[lane] = inc - tk, G.st[lane] = st, G.pos[lane] = pos, G.sz[lane] = sz;
+	if (lane == 31) G.pre[32] = inc;
+	__syncwarp();
+	return __shfl_sync(0xffffffffu, inc, 31);
+}
+
+/* anchor t of the group: the seed is the last one whose offset is at most t; a whole bucket,
+ * or take of its blocks evenly spaced (map.c:390-393) */
+__device__ __forceinline__ uint64_t sd_anchor(const plk_seed_args_t &A, const SdGroup &G, const int32_t t)
+{
+	int lo = 0;
+#pragma unroll
+	for (int h = 16; h >= 1; h >>= 1) if (G.pre[lo + h] <= t) lo += h;
+	const int64_t u = t - G.pre[lo], bsz = G.sz[lo], btk = G.pre[lo + 1] - G.pre[lo];
+	const int64_t o = btk == bsz ? u : u * bsz / btk + bsz / (2 * btk);
+	return (uint64_t)__ldg(A.kb + G.st[lo] + o) << 32 | G.pos[lo];
+}
+
+/* one warp per protein of the list: its anchors to memory, unsorted */
+#define SD_EMIT_WARPS 8
+__global__ void __launch_bounds__(32 * SD_EMIT_WARPS) k_seed_emit(plk_seed_args_t A, const int32_t *list, int32_t n_list)
+{
+	__shared__ SdGroup s_g[SD_EMIT_WARPS];
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-	const int64_t q = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-	if (q >= A.n) return;  /* whole warps */
+	const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+	if (i >= n_list) return;  /* whole warps */
+	const int32_t q = list[i];
 	const uint64_t *sd = A.seeds + A.soff[q];
 	const int32_t n = A.n_seed[q];
 	const int32_t *take = A.take + A.soff[q];
 	uint64_t *a = A.anchors + A.a_off[q];
 	int64_t k = 0;
-	/* 32 seeds at a time: their buckets' starts and sizes (0 past the cap) side by side, an
-	 * exclusive scan of the sizes, then every lane copies blocks of any of the 32 seeds
-	 * (the seed of output t: the last one whose offset is at most t) */
 	for (int32_t j0 = 0; j0 < n; j0 += 32) {
-		const int32_t j = j0 + lane;
-		int64_t st = 0, sz = 0, tk = 0;
-		uint32_t pos = 0;
-		if (j < n) {
-			const int64_t b = (int64_t)(sd[j] >> 32);
-			st = A.ki[b];
-			sz = (b + 1 < A.n_bucket ? A.ki[b + 1] : A.n_kb) - st;
-			tk = take[j];
-			pos = (uint32_t)sd[j];
+		const int32_t total = sd_group(A, s_g[w], sd, take, n, j0, lane);
+		for (int32_t t = lane; t < total; t += 32) a[k + t] = sd_anchor(A, s_g[w], t);
+		k += total;
+	}
+}
+
+/* One CTA of T threads per protein of the list, each with at most T * PER anchors: emitted into
+ * shared memory and sorted there, so that they cross HBM once (emission, the segmented sort's
+ * read and write were 3.5 times the traffic and a radix sort's passes).  A genome's blocks
+ * spread a protein's anchors thinly, so one distribution over B buckets of equal width between
+ * the smallest and the largest block leaves one or two keys a bucket, which a thread sorts by
+ * insertion; a gene's cluster of up to 128 keys is ranked by a warp, and where a bucket holds
+ * more (or more than SD_BIG of them are large) the CTA sorts all keys by a bitonic network.
+ * Any order the seeds and the buckets come in is taken.  10,000 proteins, 26.5 M anchors:
+ * emission and sort 2.16 -> 0.58 ms. */
+#define SD_BIG 256
+template <int T, int PER>
+__global__ void __launch_bounds__(T) k_seed_anchors(plk_seed_args_t A, const int32_t *list, uint64_t *__restrict__ out)
+{
+	constexpr int NMAX = T * PER, B = NMAX / 2;
+	extern __shared__ __align__(16) uint64_t s_key[];  /* [NMAX], then uint32 [B + 1] */
+	uint32_t *s_cnt = (uint32_t*)(s_key + NMAX);
+	__shared__ SdGroup s_g[T / 32];
+	__shared__ uint32_t s_mn, s_mx, s_part[T / 32], s_big[SD_BIG];
+	__shared__ int32_t s_n, s_nbig;
+	const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+	const int32_t q = list[blockIdx.x];
+	const int32_t n = (int32_t)(A.a_off[q + 1] - A.a_off[q]);
+	if (n <= 0) return;
+	if (tid == 0) s_n = 0, s_nbig = 0, s_mn = 0xffffffffu, s_mx = 0;
+	for (int x = tid; x <= B; x += T) s_cnt[x] = 0;
+	__syncthreads();
+	{ /* emission: the groups of 32 seeds in any order */
+		const uint64_t *sd = A.seeds + A.soff[q];
+		const int32_t *take = A.take + A.soff[q], ns = A.n_seed[q];
+		for (int32_t j0 = 32 * w; j0 < ns; j0 += T) {
+			const int32_t total = sd_group(A, s_g[w], sd, take, ns, j0, lane);
+			int32_t k = 0;
+			if (lane == 0) k = atomicAdd(&s_n, total);
+			k = __shfl_sync(0xffffffffu, k, 0);
+			for (int32_t t = lane; t < total; t += 32)
+				if (k + t < NMAX) s_key[k + t] = sd_anchor(A, s_g[w], t);
 		}
-		int64_t inc = tk;
+	}
+	__syncthreads();
+	uint64_t key[PER];
+	uint32_t mn = 0xffffffffu, mx = 0;
+#pragma unroll
+	for (int i = 0; i < PER; ++i) {
+		key[i] = tid + i * T < n ? s_key[tid + i * T] : 0;
+		if (tid + i * T < n) mn = min(mn, (uint32_t)(key[i] >> 32)), mx = max(mx, (uint32_t)(key[i] >> 32));
+	}
+#pragma unroll
+	for (int o = 16; o >= 1; o >>= 1) {
+		mn = min(mn, __shfl_xor_sync(0xffffffffu, mn, o));
+		mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+	}
+	if (lane == 0) atomicMin(&s_mn, mn), atomicMax(&s_mx, mx);
+	__syncthreads();
+	mn = s_mn, mx = s_mx;
+	/* bucket of a block: d * B / range rounded down, the block itself where B covers the range */
+	const uint64_t range = (uint64_t)mx - mn + 1;
+	const uint32_t scale = range > B ? (uint32_t)(((uint64_t)B << 32) / range) : 0;
+	uint32_t at[PER];
+#pragma unroll
+	for (int i = 0; i < PER; ++i)
+		if (tid + i * T < n) {
+			const uint32_t d = (uint32_t)(key[i] >> 32) - mn, b = scale ? __umulhi(d, scale) : d;
+			at[i] = atomicAdd(&s_cnt[b], 1) << 16 | b;  /* its place in bucket b: n <= 16384, B <= 8192 */
+		}
+	__syncthreads();
+	{ /* exclusive scan of the counts, B / T of them a thread */
+		constexpr int C = B / T;
+		uint32_t c[C], sum = 0;
+#pragma unroll
+		for (int x = 0; x < C; ++x) c[x] = s_cnt[tid * C + x], sum += c[x];
+		uint32_t inc = sum;
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
-			const int64_t t = __shfl_up_sync(0xffffffffu, inc, o);
+			const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
 			if (lane >= o) inc += t;
 		}
-		const int64_t total = __shfl_sync(0xffffffffu, inc, 31);
-		s_pre[w][lane] = inc - tk, s_st[w][lane] = st, s_pos[w][lane] = pos, s_sz[w][lane] = sz;
-		if (lane == 31) s_pre[w][32] = total;  /* s_pre[lo + 1] - s_pre[lo]: seed lo's take */
-		__syncwarp();
-		for (int64_t t = lane; t < total; t += 32) {
-			int lo = 0, hi = 31;
-			while (lo < hi) {
-				const int mid = (lo + hi + 1) >> 1;
-				if (s_pre[w][mid] <= t) lo = mid;
-				else hi = mid - 1;
-			}
-			const int64_t u = t - s_pre[w][lo], bsz = s_sz[w][lo], btk = s_pre[w][lo + 1] - s_pre[w][lo];
-			/* a whole bucket, or take of its blocks evenly spaced (map.c:390-393) */
-			const int64_t o = btk == bsz ? u : u * bsz / btk + bsz / (2 * btk);
-			a[k + t] = (uint64_t)A.kb[s_st[w][lo] + o] << 32 | s_pos[w][lo];
-		}
-		k += total;
-		__syncwarp();
+		if (lane == 31) s_part[w] = inc;
+		__syncthreads();
+		uint32_t base = 0;
+		for (int x = 0; x < w; ++x) base += s_part[x];
+		base += inc - sum;
+#pragma unroll
+		for (int x = 0; x < C; ++x) s_cnt[tid * C + x] = base, base += c[x];
+		if (tid == T - 1) s_cnt[B] = base;
 	}
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < PER; ++i)
+		if (tid + i * T < n) s_key[s_cnt[at[i] & 0xffffu] + (at[i] >> 16)] = key[i];
+	__syncthreads();
+	for (int b = tid; b < B; b += T) {
+		const int s0 = (int)s_cnt[b], m = (int)s_cnt[b + 1] - s0;
+		if (m <= 1) continue;
+		if (m > 12) {
+			const int x = atomicAdd(&s_nbig, 1);
+			if (x < SD_BIG) s_big[x] = (uint32_t)b;
+			continue;
+		}
+		for (int i = 1; i < m; ++i) {
+			const uint64_t v = s_key[s0 + i];
+			int j = i;
+			for (; j > 0 && s_key[s0 + j - 1] > v; --j) s_key[s0 + j] = s_key[s0 + j - 1];
+			s_key[s0 + j] = v;
+		}
+	}
+	__syncthreads();
+	bool bad = s_nbig > SD_BIG;
+	if (!bad)
+		for (int x = w; x < s_nbig; x += T / 32) { /* ranks by counting, four keys a lane; equal keys by place */
+			const int s0 = (int)s_cnt[s_big[x]], m = (int)s_cnt[s_big[x] + 1] - s0;
+			if (m > 128) { bad = true; continue; }
+			uint64_t v[4];
+			int r[4];
+#pragma unroll
+			for (int i = 0; i < 4; ++i) v[i] = lane + 32 * i < m ? s_key[s0 + lane + 32 * i] : 0, r[i] = 0;
+			for (int j = 0; j < m; ++j) {
+				const uint64_t u = s_key[s0 + j];
+#pragma unroll
+				for (int i = 0; i < 4; ++i) r[i] += u < v[i] || (u == v[i] && j < lane + 32 * i);
+			}
+			__syncwarp();
+#pragma unroll
+			for (int i = 0; i < 4; ++i) if (lane + 32 * i < m) s_key[s0 + r[i]] = v[i];
+			__syncwarp();
+		}
+	if (__syncthreads_or(bad)) {
+		int np2 = 1;
+		while (np2 < n) np2 <<= 1;  /* at most NMAX, a power of two */
+		for (int i = n + tid; i < np2; i += T) s_key[i] = ~0ull;
+		__syncthreads();
+		for (int k = 2; k <= np2; k <<= 1)
+			for (int j = k >> 1; j > 0; j >>= 1) {
+				for (int i = tid; i < np2; i += T) {
+					const int l = i ^ j;
+					if (l > i) {
+						const uint64_t a = s_key[i], c = s_key[l];
+						if ((a > c) == ((i & k) == 0)) s_key[i] = c, s_key[l] = a;
+					}
+				}
+				__syncthreads();
+			}
+	}
+	uint64_t *o = out + A.a_off[q];
+	for (int i = tid; i < n; i += T) o[i] = s_key[i];
 }
 
 /* HMM-profile queries: one thread per match state, its offered groups (seed_hmm.cuh) */
@@ -359,13 +525,40 @@ extern "C" int plk_seed_take(const plk_seed_args_t *a, void *stream)
 	return (int)cudaGetLastError();
 }
 
-extern "C" int plk_seed_emit(const plk_seed_args_t *a, void *stream)
+extern "C" int plk_seed_emit(const plk_seed_args_t *a, const int32_t *list, int32_t n_list, void *stream)
 {
-	if (a->n <= 0) return 0;
-	k_seed_emit<<<(unsigned)(((int64_t)a->n * 32 + 32 * SD_EMIT_WARPS - 1) / (32 * SD_EMIT_WARPS)), 32 * SD_EMIT_WARPS, 0,
-			(cudaStream_t)stream>>>(*a);
+	if (n_list <= 0) return 0;
+	k_seed_emit<<<(unsigned)(((int64_t)n_list * 32 + 32 * SD_EMIT_WARPS - 1) / (32 * SD_EMIT_WARPS)), 32 * SD_EMIT_WARPS, 0,
+			(cudaStream_t)stream>>>(*a, list, n_list);
 	plk_add_launches(1);
 	return (int)cudaGetLastError();
+}
+
+template <int T, int PER>
+static int seed_anchors(const plk_seed_args_t *a, const int32_t *list, int32_t n_list, uint64_t *out, cudaStream_t st)
+{
+	const int smem = 8 * T * PER + 4 * (T * PER / 2 + 4);
+	cudaError_t e = cudaFuncSetAttribute(k_seed_anchors<T, PER>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	if (e != cudaSuccess) return (int)e;
+	k_seed_anchors<T, PER><<<(unsigned)n_list, T, smem, st>>>(*a, list, out);
+	plk_add_launches(1);
+	return (int)cudaGetLastError();
+}
+
+/* the sorted anchors of the list's proteins, each at most PLK_SEED_CLASS(cls) of them, into out */
+extern "C" int plk_seed_anchors(const plk_seed_args_t *a, const int32_t *list, int32_t n_list, int32_t cls, uint64_t *out,
+		void *stream)
+{
+	cudaStream_t st = (cudaStream_t)stream;
+	if (n_list <= 0) return 0;
+	/* the least shared memory that holds a class: 23 to 187 KB a CTA */
+	switch (cls) {
+	case 0: return seed_anchors<256, 8>(a, list, n_list, out, st);
+	case 1: return seed_anchors<256, 16>(a, list, n_list, out, st);
+	case 2: return seed_anchors<512, 16>(a, list, n_list, out, st);
+	case 3: return seed_anchors<1024, 16>(a, list, n_list, out, st);
+	default: return (int)cudaErrorInvalidValue;
+	}
 }
 
 /* per-segment ascending sort of keys_in into keys_out, segment i at [seg_off[i],
