@@ -4,20 +4,26 @@
  * scores, bit for bit).
  *
  * One warp per candidate.  For each anchor (at most 32, nasw-cuda.cu:1174):
- *   seed    the warp loads the oriented bases of the anchor's block (plus the
- *           k-mer's reach) into shared memory once, translates every codon end
- *           of the window once, and each lane scores its deltas from the staged
- *           residues: kmer shared-memory lookups per delta instead of 3*kmer
- *           scattered genome reads.  The best seed is a warp max over the key
- *           (score << 32 | ~delta), so ties go to the smaller target end as in
- *           the reference's reduction;
+ *   seed    the residue of every codon end of the block (plus the k-mer's reach) goes
+ *           into shared memory once, twelve a lane: three aligned words of the packed
+ *           genome hold their 14 bases, and three bases, as they lie in the genome,
+ *           index a 4096-entry residue table (one per strand).  A lane then scores
+ *           eight neighbouring deltas from 24 staged bytes against the scores of the
+ *           k-mer's query residues, copied to a row each.  The best seed is a warp max
+ *           over score * 8192 + (8191 - delta), so ties go to the smaller target end as
+ *           in the reference's reduction;
  *   extend  left, then right: 32 steps at a time, one per lane, with warp
  *           prefix sums of the step scores and prefix maxima of the running
  *           score; the first step that leaves the sequence or breaks the X-drop
  *           ends the walk, and the best prefix (first step reaching it) is the
  *           reference's left_best / left_len (nasw-cuda.cu:1229-1252).
- * Lane 0 then sorts the segments and sums them greedily with the overlap rule
- * of nasw-cuda.cu:1259-1293.
+ * The warp then ranks the segments and sums them greedily with the overlap rule
+ * of nasw-cuda.cu:1259-1293, a segment per lane.
+ *
+ * Bound by instruction issue (base by base with 64-bit bounds, and six scattered
+ * query reads per delta, an anchor cost some 3,000 warp instructions).  131,072
+ * candidates of 8 anchors, 256-wide blocks: 4.4 -> 1.64 ms.
+ *
  * Every index is bounds-checked against the buffer sizes, so malformed
  * candidates read as missing bases / residues instead of faulting.
  */
@@ -69,56 +75,87 @@ __device__ __forceinline__ int gl_query(const GlArgs &A, const ns_gpu_gapless_ca
 	return a >= 0 && a < A.query_aa ? __ldg(A.queries + a) : 0;
 }
 
-/* One side of the X-drop extension, 32 steps per round.  dir = -1: left, +1: right.
+/* bytes of a warp's staged residues: whole rounds of twelve, and the eight-byte reads past the last delta */
+__host__ __device__ __forceinline__ int gl_stride(const int block_width, const int kmer)
+{
+	return (block_width + 3 * (kmer - 1) + 24 + 15) / 16 * 16;
+}
+
+/* the 16 packed bits from base a on (a nibble each), a within the genome's bytes */
+__device__ __forceinline__ unsigned gl_nibbles(const GlArgs &A, const int64_t a)
+{
+	const uint8_t *p = A.packed + (a >> 1);
+	return ((unsigned)__ldg(p) | (unsigned)__ldg(p + 1) << 8) >> ((int)(a & 1) * 4);
+}
+
+struct GlCand {
+	ns_gpu_gapless_candidate_t C;
+	const uint8_t *q;      /* its query, when all of it lies in the buffer */
+	const uint8_t *tab;    /* residue table of its strand */
+	int64_t lo, hi;        /* target positions whose codon end lies inside target and genome with the
+	                        * bytes that gl_nibbles reads: [lo, hi) */
+};
+
+__device__ __forceinline__ int gl_q(const GlArgs &A, const GlCand &G, const int pos)
+{
+	const int v = G.q ? __ldg(G.q + pos) : gl_query(A, G.C, pos);
+	return v < A.asize ? v : A.asize - 1;
+}
+
+/* residue of the codon ending at te (any te) */
+__device__ __forceinline__ int gl_res(const GlArgs &A, const GlCand &G, const uint8_t *codon, const int64_t te)
+{
+	if (te >= G.lo && te < G.hi) {
+		const int64_t a = G.C.target_offset + (G.C.reverse ? G.C.target_length - 1 - te : te - 2);
+		return G.tab[gl_nibbles(A, a) & 0xfffu];
+	}
+	return min(gl_aa(A, G.C, codon, te), 31);
+}
+
+/* One side of the X-drop extension, 32 steps per round.  DIR = -1: left, +1: right.
  * Returns best (>= 0) and sets len (steps up to the first step reaching it). */
-__device__ int gl_extend(const GlArgs &A, const ns_gpu_gapless_candidate_t &C, const uint8_t *codon,
-		const int *sm, const int lane, const int dir, const int qend, const int64_t te0, int &len, int &walked)
+template <int DIR>
+__device__ __forceinline__ int gl_extend(const GlArgs &A, const GlCand &G, const uint8_t *codon, const int *sm, const int lane,
+		const int qend, const int64_t te0, int &len, unsigned &walked)
 {
 	int carry = 0, best = 0, blen = 0, st = 0;
 	const int kmer = A.kmer;
-	walked = 0;
 	for (;;) {
 		const int step = st + lane + 1;
 		int pos;
 		int64_t te;
 		bool valid;
-		if (dir < 0) {
+		if (DIR < 0) {
 			pos = qend - kmer - (step - 1);
 			te = te0 - (int64_t)(kmer - 1 + step) * 3;
 			valid = pos >= 0 && te - 2 >= 0;
 		} else {
 			pos = qend + step;
 			te = te0 + (int64_t)step * 3;
-			valid = pos < C.query_length && te < C.target_length;
+			valid = pos < G.C.query_length && te < G.C.target_length;
 		}
 		int v = 0;
-		if (valid) {
-			const int a = gl_aa(A, C, codon, te), q = gl_query(A, C, pos);
-			v = sm[a * A.asize + (q < A.asize ? q : A.asize - 1)];
-		}
-		int incl = v;
+		if (valid) v = sm[gl_res(A, G, codon, te) * A.asize + gl_q(A, G, pos)];
+		int running = v;
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
-			const int x = __shfl_up_sync(FULL, incl, o);
-			if (lane >= o) incl += x;
+			const int x = __shfl_up_sync(FULL, running, o);
+			if (lane >= o) running += x;
 		}
-		const int running = carry + incl;
+		running += carry;
 		const unsigned inval = __ballot_sync(FULL, !valid);
 		const int first_invalid = inval ? __ffs(inval) - 1 : 32;
-		int rmax = lane < first_invalid ? running : INT_MIN;
+		int rmax = lane < first_invalid ? running : INT_MIN;  /* maximum of the round up to this step */
 #pragma unroll
 		for (int o = 1; o < 32; o <<= 1) {
 			const int x = __shfl_up_sync(FULL, rmax, o);
 			if (lane >= o) rmax = max(rmax, x);
 		}
-		const int bestv = max(best, rmax);
-		const unsigned brk = __ballot_sync(FULL, lane < first_invalid && bestv - running > A.xdrop);
+		const unsigned brk = __ballot_sync(FULL, lane < first_invalid && max(best, rmax) - running > A.xdrop);
 		const int first_brk = brk ? __ffs(brk) - 1 : 32;
 		const int stop = min(first_invalid, first_brk + 1);  /* steps processed in this round */
-		int m = lane < stop ? running : INT_MIN;
-#pragma unroll
-		for (int o = 16; o >= 1; o >>= 1) m = max(m, __shfl_xor_sync(FULL, m, o));
-		if (m > best) { /* strict improvement: the first step reaching it */
+		const int m = __shfl_sync(FULL, rmax, stop > 0 ? stop - 1 : 0);
+		if (stop > 0 && m > best) { /* strict improvement: the first step reaching it */
 			const unsigned at = __ballot_sync(FULL, lane < stop && running == m);
 			blen = st + __ffs(at);
 			best = m;
@@ -132,92 +169,186 @@ __device__ int gl_extend(const GlArgs &A, const ns_gpu_gapless_candidate_t &C, c
 	return best;
 }
 
+/* residues of the window's codon ends base .. base + win - 1 into saa, twelve per lane and round */
+__device__ __forceinline__ void gl_stage(const GlArgs &A, const GlCand &G, const uint8_t *codon, uint8_t *saa, const int64_t base,
+		const int win, const int lane)
+{
+	const bool words = ((uintptr_t)A.packed & 3) == 0;
+	for (int x0 = 12 * lane; x0 < win; x0 += 384) {
+		const int64_t te = base + x0;
+		/* their 14 bases from genome position a on, in three words that must lie in the buffer */
+		const int64_t a = G.C.target_offset + (G.C.reverse ? G.C.target_length - 1 - (te + 11) : te - 2), w = a >> 3;
+		uint32_t o[3];
+		if (words && te >= G.lo && te + 11 < G.hi && (w + 3) * 8 <= A.bases) {
+			const uint32_t *p = reinterpret_cast<const uint32_t*>(A.packed) + w;
+			const uint32_t p0 = __ldg(p), p1 = __ldg(p + 1), p2 = __ldg(p + 2);
+			const unsigned sh = (unsigned)(a & 7) * 4;
+			const uint32_t v0 = __funnelshift_r(p0, p1, sh), v1 = __funnelshift_r(p1, p2, sh);
+			uint32_t t[12];
+#pragma unroll
+			for (int i = 0; i < 12; ++i) t[i] = G.tab[(i < 8 ? __funnelshift_r(v0, v1, 4 * i) : v1 >> (4 * i - 32)) & 0xfffu];
+#pragma unroll
+			for (int i = 0; i < 3; ++i) o[i] = t[4 * i] + (t[4 * i + 1] << 8) + (t[4 * i + 2] << 16) + (t[4 * i + 3] << 24);
+			if (G.C.reverse) { /* the codon ends run down the genome */
+				const uint32_t z = __byte_perm(o[2], 0, 0x0123);
+				o[1] = __byte_perm(o[1], 0, 0x0123), o[2] = __byte_perm(o[0], 0, 0x0123), o[0] = z;
+			}
+		} else {
+			o[0] = o[1] = o[2] = 0;
+			for (int i = 0; i < 12; ++i) {
+				const uint32_t r = (uint32_t)gl_res(A, G, codon, te + i) << (8 * (i & 3));
+				if (i < 4) o[0] |= r;
+				else if (i < 8) o[1] |= r;
+				else o[2] |= r;
+			}
+		}
+		uint32_t *d = reinterpret_cast<uint32_t*>(saa + x0);
+		d[0] = o[0], d[1] = o[1], d[2] = o[2];
+	}
+}
+
+/* K: the k-mer length, compiled in for the mapper's 5, 6 and 7 (0: any length) */
+template <int K>
 __global__ void __launch_bounds__(32 * GL_WARPS) k_gapless(GlArgs A, const int8_t *__restrict__ mat,
 		const uint8_t *__restrict__ codon_g)
 {
 	extern __shared__ __align__(16) uint8_t gl_smem[];
 	__shared__ int sm[32 * 32];
 	__shared__ uint8_t codon[64];
+	__shared__ uint8_t tab[2][4096];  /* residue of three bases as they lie in the genome, read forward / on the other strand */
+	__shared__ int prof[GL_WARPS][K > 0 ? K : 1][32];
 	__shared__ int seg[GL_WARPS][3][GL_MAX_ANCHORS];
 	const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-	for (int x = threadIdx.x; x < A.asize * A.asize; x += blockDim.x) sm[x] = mat[x];
+	for (int x = threadIdx.x; x < 32 * 32; x += blockDim.x) sm[x] = x < A.asize * A.asize ? mat[x] : 0;
 	for (int x = threadIdx.x; x < 64; x += blockDim.x) codon[x] = codon_g[x];
 	__syncthreads();
-	const int win = A.block_width + 3 * (A.kmer - 1);       /* codon ends of one anchor's seed scan */
-	const int stride = (win + 2 + 15) / 16 * 16;               /* bytes of one staging array */
-	uint8_t *sb = gl_smem + (size_t)wib * 2 * stride;          /* bases of the window */
-	uint8_t *saa = sb + stride;                                /* residue of each codon end */
+	for (int x = threadIdx.x; x < 4096; x += blockDim.x) {
+		const int n0 = x & 15, n1 = x >> 4 & 15, n2 = x >> 8;
+		const bool ok = n0 < 4 && n1 < 4 && n2 < 4;
+		tab[0][x] = ok ? min((int)codon[n0 << 4 | n1 << 2 | n2], 31) : 20;
+		tab[1][x] = ok ? min((int)codon[(3 - n2) << 4 | (3 - n1) << 2 | (3 - n0)], 31) : 20;
+	}
+	__syncthreads();
+	const int kmer = K > 0 ? K : A.kmer;
+	const int win = A.block_width + 3 * (kmer - 1);            /* codon ends of one anchor's seed scan */
+	uint8_t *saa = gl_smem + (size_t)wib * gl_stride(A.block_width, kmer);
+	for (int x = lane; x < gl_stride(A.block_width, kmer); x += 32) saa[x] = 0;  /* bytes past the window stay residue 0 */
+	__syncwarp();
 	unsigned long long walked_sum = 0;
 	for (int ci = blockIdx.x * GL_WARPS + wib; ci < A.n_cand; ci += gridDim.x * GL_WARPS) {
-		const ns_gpu_gapless_candidate_t C = A.cand[ci];
-		const int na = C.anchor_count < GL_MAX_ANCHORS ? C.anchor_count : GL_MAX_ANCHORS;
+		GlCand G;
+		G.C = A.cand[ci];
+		const int64_t ql = G.C.query_length;
+		G.q = G.C.query_offset >= 0 && G.C.query_offset + ql <= A.query_aa ? A.queries + G.C.query_offset : 0;
+		G.tab = tab[G.C.reverse ? 1 : 0];
+		{ /* codon ends with all three bases inside the target, and their nibbles' two bytes in the genome */
+			const int64_t off = G.C.target_offset, tl = G.C.target_length;
+			G.lo = 2, G.hi = tl;
+			if (G.C.reverse) { /* bases off + tl - 1 - te .. + 2, the last byte one further */
+				G.lo = max(G.lo, off + tl + 3 - A.bases), G.hi = min(G.hi, off + tl);
+			} else { /* bases off + te - 2 .. off + te */
+				G.lo = max(G.lo, 2 - off), G.hi = min(G.hi, A.bases - off - 2);
+			}
+		}
+		const int na = G.C.anchor_count < GL_MAX_ANCHORS ? G.C.anchor_count : GL_MAX_ANCHORS;
 		int n_seg = 0;
 		for (int ai = 0; ai < na; ++ai) {
-			const int64_t aidx = (int64_t)C.anchor_offset + ai;
+			const int64_t aidx = (int64_t)G.C.anchor_offset + ai;
 			if (aidx < 0 || aidx >= A.n_anchors) break;
 			const ns_gpu_gapless_anchor_t an = A.anchors[aidx];
 			const int qe = an.query_end;
-			if (!(qe >= A.kmer - 1 && qe < C.query_length)) continue;
-			/* seed: stage bases [base-2, base+win) and translate every codon end once */
-			const int64_t base = an.target_block - (int64_t)3 * (A.kmer - 1);
-			for (int x = lane; x < win + 2; x += 32) sb[x] = (uint8_t)gl_base(A, C, base - 2 + x);
-			__syncwarp();
-			for (int x = lane; x < win; x += 32) {
-				const int b0 = sb[x], b1 = sb[x + 1], b2 = sb[x + 2];
-				saa[x] = b0 < 4 && b1 < 4 && b2 < 4 ? codon[b0 << 4 | b1 << 2 | b2] : 20;
+			if (!(qe >= kmer - 1 && qe < G.C.query_length)) continue;
+			const int64_t tb = an.target_block;
+			gl_stage(A, G, codon, saa, tb - (int64_t)3 * (kmer - 1), win, lane);
+			if (K > 0) {
+#pragma unroll
+				for (int k = 0; k < K; ++k)
+					prof[wib][k][lane] = lane < A.asize ? sm[lane * A.asize + gl_q(A, G, qe - K + 1 + k)] : 0;
 			}
 			__syncwarp();
-			long long key = LLONG_MIN;
-			for (int d = lane; d < A.block_width; d += 32) {
-				const int64_t te = an.target_block + d;
-				if (te - (int64_t)(A.kmer - 1) * 3 - 2 < 0 || te >= C.target_length) continue;
-				int s = 0;
-				for (int k = 0; k < A.kmer; ++k) {
-					const int q = gl_query(A, C, qe - A.kmer + 1 + k);
-					s += sm[saa[d + 3 * k] * A.asize + (q < A.asize ? q : A.asize - 1)];
+			/* deltas whose k-mer lies in the target */
+			const int64_t dl = (int64_t)(kmer - 1) * 3 + 2 - tb, dh = G.C.target_length - tb;
+			const int d_lo = dl > 0 ? (int)min(dl, (int64_t)A.block_width) : 0;
+			const int d_hi = dh < A.block_width ? (int)max(dh, (int64_t)0) : A.block_width;
+			int key = INT_MIN;  /* score * 8192 + (8191 - delta): scores are below 64 * 128, deltas below 8192 */
+			if (K > 0) {
+				for (int d0 = 8 * lane; d0 < d_hi; d0 += 256) {
+					constexpr int NB = 8 + 3 * (K > 0 ? K - 1 : 0), NW = (NB + 7) / 8 * 2;
+					uint32_t w[NW];
+#pragma unroll
+					for (int i = 0; i < NW; i += 2) {
+						const uint2 x = *reinterpret_cast<const uint2*>(saa + d0 + 4 * i);
+						w[i] = x.x, w[i + 1] = x.y;
+					}
+					int r[NB];
+#pragma unroll
+					for (int i = 0; i < NB; ++i) r[i] = (int)__byte_perm(w[i >> 2], 0, 0x4440 + (i & 3));
+#pragma unroll
+					for (int j = 0; j < 8; ++j) {
+						int sc = 0;
+#pragma unroll
+						for (int k = 0; k < K; ++k) sc += prof[wib][k][r[j + 3 * k]];
+						const int d = d0 + j;
+						if (d >= d_lo && d < d_hi) key = max(key, sc * 8192 + 8191 - d);
+					}
 				}
-				const long long kk = (long long)s * 4294967296ll + (long long)(0xFFFFFFFFu - (unsigned)d);
-				key = max(key, kk);
+			} else {
+				for (int d = lane; d < d_hi; d += 32) {
+					if (d < d_lo) continue;
+					int sc = 0;
+					for (int k = 0; k < kmer; ++k) sc += sm[saa[d + 3 * k] * A.asize + gl_q(A, G, qe - kmer + 1 + k)];
+					key = max(key, sc * 8192 + 8191 - d);
+				}
 			}
 #pragma unroll
 			for (int o = 16; o >= 1; o >>= 1) key = max(key, __shfl_xor_sync(FULL, key, o));
 			__syncwarp();
-			if (key == LLONG_MIN) continue;  /* no valid target end in the block */
-			const int seed = (int)(key >> 32);
-			const int64_t te = an.target_block + (int64_t)(0xFFFFFFFFu - (unsigned)(key & 0xFFFFFFFFll));
-			int ll, rl, wl, wr;
-			const int lb = gl_extend(A, C, codon, sm, lane, -1, qe, te, ll, wl);
-			const int rb = gl_extend(A, C, codon, sm, lane, +1, qe, te, rl, wr);
-			walked_sum += (unsigned long long)(wl + wr);
+			if (key == INT_MIN) continue;  /* no valid target end in the block */
+			const int seed = key >> 13;
+			const int64_t te = tb + (8191 - (key & 8191));
+			int ll, rl;
+			unsigned wk = 0;
+			const int lb = gl_extend<-1>(A, G, codon, sm, lane, qe, te, ll, wk);
+			const int rb = gl_extend<1>(A, G, codon, sm, lane, qe, te, rl, wk);
+			walked_sum += wk;
 			if (lane == 0) {
 				seg[wib][0][n_seg] = seed + lb + rb;
-				seg[wib][1][n_seg] = qe - (A.kmer - 1) - ll;
+				seg[wib][1][n_seg] = qe - (kmer - 1) - ll;
 				seg[wib][2][n_seg] = qe + rl;
 			}
 			++n_seg;
 		}
 		__syncwarp();
-		if (lane == 0) { /* nasw-cuda.cu:1259-1293: stable sort by score, greedy overlap-scaled sum */
-			int ss[GL_MAX_ANCHORS], qs[GL_MAX_ANCHORS], qq[GL_MAX_ANCHORS], n = 0, total = 0;
+		{ /* nasw-cuda.cu:1259-1293: stable sort by score, greedy overlap-scaled sum */
+			int total = 0;
+			const int my = lane < n_seg ? seg[wib][0][lane] : INT_MIN;
+			int rank = 0;
 			for (int i = 0; i < n_seg; ++i) {
-				const int sc = seg[wib][0][i];
-				int j;
-				for (j = n; j > 0 && ss[j - 1] < sc; --j) ss[j] = ss[j - 1], qs[j] = qs[j - 1], qq[j] = qq[j - 1];
-				ss[j] = sc, qs[j] = seg[wib][1][i], qq[j] = seg[wib][2][i], ++n;
+				const int x = __shfl_sync(FULL, my, i);
+				rank += x > my || (x == my && i < lane);
 			}
-			for (int i = 0; i < n; ++i) {
-				const int len = qq[i] - qs[i] + 1;
-				int overlap = 0;
-				if (i > 0 && ss[i] < A.xdrop) break;
-				for (int j = 0; j < i; ++j) {
-					const int s = max(qs[i], qs[j]), e = min(qq[i], qq[j]);
-					if (ss[j] != INT_MIN && e >= s) overlap += e - s + 1;
-				}
-				if (overlap >= len) { ss[i] = INT_MIN; continue; }
-				if (overlap > 0) total += (int)((long long)ss[i] * (len - overlap) / len);
-				else total += ss[i];
+			const int b = lane < n_seg ? seg[wib][1][lane] : 0, e = lane < n_seg ? seg[wib][2][lane] : 0;
+			__syncwarp();
+			if (lane < n_seg) seg[wib][0][rank] = my, seg[wib][1][rank] = b, seg[wib][2][rank] = e;
+			__syncwarp();
+			const int ss = lane < n_seg ? seg[wib][0][lane] : 0, qs = lane < n_seg ? seg[wib][1][lane] : 0,
+					qq = lane < n_seg ? seg[wib][2][lane] : 0;
+			unsigned out = 0;  /* segments that earlier ones cover: they take part no more */
+			for (int i = 0; i < n_seg; ++i) {
+				const int si = __shfl_sync(FULL, ss, i), bi = __shfl_sync(FULL, qs, i), ei = __shfl_sync(FULL, qq, i);
+				const int len = ei - bi + 1;
+				if (i > 0 && si < A.xdrop) break;
+				const int s0 = max(bi, qs), e0 = min(ei, qq);
+				int overlap = lane < i && !(out >> lane & 1) && e0 >= s0 ? e0 - s0 + 1 : 0;
+				if (__ballot_sync(FULL, overlap > 0)) {
+#pragma unroll
+					for (int o = 16; o >= 1; o >>= 1) overlap += __shfl_xor_sync(FULL, overlap, o);
+				} else overlap = 0;
+				if (overlap >= len) { out |= 1u << i; continue; }
+				if (overlap > 0) total += (int)((long long)si * (len - overlap) / len);
+				else total += si;
 			}
-			A.scores[ci] = n_seg ? total : INT_MIN;
+			if (lane == 0) A.scores[ci] = n_seg ? total : INT_MIN;
 		}
 		__syncwarp();
 	}
@@ -226,8 +357,7 @@ __global__ void __launch_bounds__(32 * GL_WARPS) k_gapless(GlArgs A, const int8_
 
 extern "C" int plk_gapless_smem_bytes(int32_t block_width, int32_t kmer)
 {
-	const int win = block_width + 3 * (kmer - 1);
-	return GL_WARPS * 2 * ((win + 2 + 15) / 16 * 16);
+	return GL_WARPS * gl_stride(block_width, kmer);
 }
 
 extern "C" int plk_gapless(const uint8_t *packed, int64_t bases, const uint8_t *queries, int64_t query_aa,
@@ -242,15 +372,17 @@ extern "C" int plk_gapless(const uint8_t *packed, int64_t bases, const uint8_t *
 	A.anchors = (const ns_gpu_gapless_anchor_t*)anchors, A.n_anchors = n_anchors;
 	A.block_width = block_width, A.kmer = kmer, A.xdrop = xdrop, A.asize = asize, A.scores = scores, A.steps = steps;
 	const int smem = plk_gapless_smem_bytes(block_width, kmer);
-	cudaError_t e = cudaFuncSetAttribute(k_gapless, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+	void (*f)(GlArgs, const int8_t*, const uint8_t*) = kmer == 6 ? k_gapless<6> : kmer == 5 ? k_gapless<5> :
+			kmer == 7 ? k_gapless<7> : k_gapless<0>;
+	cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
 	if (e != cudaSuccess) return (int)e;
 	int per_sm = 0;
-	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_gapless, 32 * GL_WARPS, smem);
+	e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, f, 32 * GL_WARPS, smem);
 	if (e != cudaSuccess) return (int)e;
 	int64_t grid = (int64_t)(per_sm > 0 ? per_sm : 1) * n_sm;
 	const int64_t need = (n_cand + GL_WARPS - 1) / GL_WARPS;
 	if (grid > need) grid = need;
-	k_gapless<<<(unsigned)grid, 32 * GL_WARPS, smem, (cudaStream_t)stream>>>(A, mat_dev, codon_dev);
+	f<<<(unsigned)grid, 32 * GL_WARPS, smem, (cudaStream_t)stream>>>(A, mat_dev, codon_dev);
 	plk_add_launches(1);
 	return (int)cudaGetLastError();
 }
