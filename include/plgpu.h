@@ -707,7 +707,7 @@ int pl_ps_gapped_device(pl_engine_t *e, const pl_ps_job_t *jobs, int32_t n, cons
  * query's anchors are blockId << 32 | queryPos, sorted ascending, as mp_chain
  * takes them; the arguments of mp_chain are the fields of pl_chain_opt_t.  The
  * chaining DP (the score f, predecessor p and peak v of every anchor,
- * chain.c:183-208) runs on the device, one warp per query; the backtrack and
+ * chain.c:183-208) runs on the device, one thread per query; the backtrack and
  * compaction (chain.c:8-110) run on the host's cores.
  * ------------------------------------------------------------------------- */
 typedef struct {

@@ -3,14 +3,22 @@
  * of mp_chain): for every anchor i of a query, the best chain score f[i] ending
  * there, its predecessor p[i] and the peak score v[i] along that chain.
  *
- * One thread per query (the host orders queries longest first, so the longest
- * start in the first warps).  The loop over predecessors is the reference's,
+ * Two kernels.  k_chain_score computes comput_sc of every anchor against the 32
+ * before it, a lane per pair.  k_chain_fill walks one query per thread, one such
+ * thread per warp (the host orders queries longest first, so the longest start
+ * first).  The loop over predecessors is the reference's,
  * statement for statement: a running best (strictly greater wins, so the nearest j
  * keeps a tie), a skip counter that rises on a non-improving predecessor already
  * marked by this anchor (t[j] == i), falls on an improving one (floored at 0) and
  * ends the loop when it passes max_skip, and a mark t[p[j]] = i after every scored
  * j.  Queries are independent, so thousands of them fill the GPU; within a query
  * the order of comparisons is the reference's and the results are bit-exact.
+ * Different queries' loops share neither trip counts nor branches, so 32 of them
+ * in a warp ran their paths one after the other and left two warps an SM (8.3 ms
+ * for 10,000 queries, 1.2 M anchors); a warp each is bound by issue, and scoring a
+ * pair was 80 of its 110 instructions on a single lane: 5.5 ms, with the scores
+ * taken from the rows 2.9 + 0.09, the loop's records read four ahead and its branches
+ * turned into selects 2.2 + 0.09.
  * Scores (comput_sc, chain.c:112-152) use the reference's float operations one at
  * a time, rounded to nearest as the CPU build rounds them (no fused multiply-add).
  */
@@ -23,7 +31,7 @@ extern "C" void plk_add_launches(uint64_t n);
 
 namespace {
 
-constexpr int CHAIN_THREADS = 64;
+constexpr int CHAIN_THREADS = 128, CHAIN_STRIDE = 32;
 constexpr int BLOCK_BONUS = 2;  /* MP_BLOCK_BONUS (protlocus.h:47) */
 
 /* log2 approximation of the reference (mppriv.h:143-151), valid for x >= 2: the
@@ -80,50 +88,105 @@ __device__ __forceinline__ int chain_score(uint64_t ai, uint64_t aj, const plk_c
 	return sc;
 }
 
-/* One thread per query: the reference's sequential loop over predecessors, with its
+/* rows[(r0 + i) * 32 + k] = the score of chaining anchor i - 1 - k before anchor i, k < 32, for the
+ * queries order[first ..]: a CTA per query, a warp per anchor */
+__global__ void __launch_bounds__(CHAIN_THREADS) k_chain_score(plk_chain_args_t A)
+{
+	const int q = A.order[blockIdx.x];
+	if (q < 0 || q >= A.n_all) return;  /* k_chain_fill reports it */
+	const int64_t base = A.off[q];
+	const int n = A.n[q], lane = threadIdx.x & 31;
+	if (base < 0 || n < 0 || base + n > A.n_a) return;
+	const uint64_t *__restrict__ a = A.a + base;
+	int32_t *row = A.rows + (A.row0[blockIdx.x] << 5);
+	for (int i = threadIdx.x >> 5; i < n; i += CHAIN_THREADS / 32) {
+		const int j = i - 1 - lane;
+		if (j >= 0) row[((int64_t)i << 5) + lane] = chain_score(a[i], a[j], A);
+	}
+}
+
+/* One query per thread: the reference's sequential loop over predecessors, with its
  * early exit, skip counter and marks, so the order of every comparison is the
- * reference's.  Every per-query index is checked against the query's length; a bad
- * one records the site and the query (err[0], err[1]) and the access is skipped. */
+ * reference's.  Per anchor a record {f, p, t, v}.  Every per-query index is checked against the
+ * query's length; a bad one records the site and the query (err[0], err[1]) and the access is
+ * skipped. */
 __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_fill(plk_chain_args_t A)
 {
-	const int qi = blockIdx.x * CHAIN_THREADS + threadIdx.x;
+	if (threadIdx.x % CHAIN_STRIDE) return;
+	const int qi = (blockIdx.x * CHAIN_THREADS + threadIdx.x) / CHAIN_STRIDE;
 	if (qi >= A.n_q) return;
 	const int q = A.order[qi];
-	if (q < 0 || q >= A.n_q) { atomicExch(A.err, 1); return; }
+	if (q < 0 || q >= A.n_all) { atomicExch(A.err, 1); return; }
 	const int64_t base = A.off[q];
 	const int n = A.n[q];
 	if (base < 0 || n < 0 || base + n > A.n_a) { atomicExch(A.err, 2), atomicExch(A.err + 1, q); return; }
 	const uint64_t *__restrict__ a = A.a + base;
-	int32_t *f = A.f + base, *p = A.p + base, *v = A.v + base, *t = A.t + base;
+	const int32_t *__restrict__ rows = A.rows + (A.row0[qi] << 5);
+	int32_t *f = A.f + base, *p = A.p + base, *v = A.v + base;
+	int4 *rec = (int4*)A.rec + base;
 #define CHK(x, site) ((unsigned)(x) < (unsigned)n ? true : (atomicExch(A.err, (site)), atomicExch(A.err + 1, q), false))
-	for (int k = 0; k < n; ++k) t[k] = 0;
 	int st = 0, hi = -1, hf = 0;
 	unsigned long long pairs = 0;
 	for (int i = 0; i < n; ++i) {
 		const uint64_t ai = a[i];
+		const int32_t *row = rows + ((int64_t)i << 5);
+		if (i + 2 < n) { /* the next anchors' row and the anchors, on their way from L2 */
+			asm volatile("prefetch.global.L1 [%0];" :: "l"(row + 64));
+			asm volatile("prefetch.global.L1 [%0];" :: "l"(a + min(i + 16, n - 1)));
+		}
 		int max_f = A.kmer, max_j = -1, n_skip = 0;
 		while (st < i && (((ai >> 32) - (a[st] >> 32)) << A.bbit) > (uint64_t)(int64_t)A.max_dist_x) ++st;
 		if (hi >= 0 && hi >= st && CHK(hi, 12)) { /* the best anchor so far, even beyond the skip limit */
-			const int s = hf + chain_score(ai, a[hi], A);
+			const int s = hf + (i - 1 - hi < 32 ? row[i - 1 - hi] : chain_score(ai, a[hi], A));
 			if (s > max_f) max_f = s, max_j = hi;
 		} else hf = 0, hi = -1;
 		if (i - st > A.max_iter) st = i - A.max_iter;
-		for (int j = i - 1; j >= st; --j) {
-			int s = chain_score(ai, a[j], A);
-			++pairs;
-			if (s == INT_MIN) continue;
-			s += f[j];
-			if (s > max_f) {
-				max_f = s, max_j = j;
-				if (n_skip > 0) --n_skip;
-			} else if (t[j] == i) {
-				if (++n_skip > A.max_skip) break;
+		int j = i - 1;
+		bool more = true;
+		/* predecessor j with its record and score (INT_MIN: they cannot chain), as selects: live = the
+		 * loop still runs; marked is whether the predecessor of j was marked */
+#define CHAIN_STEP(r, sc, live, marked) do { \
+			const bool ok = (live) && (sc) != INT_MIN; \
+			const int s = (sc) + (r).x; \
+			const bool better = ok && s > max_f, skip = ok && !better && (r).z == i; \
+			n_skip = better ? max(n_skip - 1, 0) : n_skip + skip; \
+			more = more && !(skip && n_skip > A.max_skip); \
+			max_f = better ? s : max_f, max_j = better ? j : max_j; \
+			marked = ok && more && (r).y >= 0; \
+			if (marked && CHK((r).y, 14)) rec[(r).y].z = i; \
+		} while (0)
+		const int near = st > i - 32 ? st : i - 32;  /* predecessors whose scores are in the row */
+		while (more && j >= near) {
+			/* j counts down from i - 1 in fours.  The four records are read before any of their marks
+			 * is set (read one by one each waited for the mark before it: 2.9 against 2.6 ms); a mark
+			 * on a later one of the four goes to its copy too */
+			const int4 s4 = *(const int4*)(row + (i - 1 - j));
+			const int sc[4] = {s4.x, s4.y, s4.z, s4.w}, j0 = j;
+			int4 r[4];
+#pragma unroll
+			for (int u = 0; u < 4; ++u) r[u] = rec[j0 - u >= 0 ? j0 - u : 0];
+#pragma unroll
+			for (int u = 0; u < 4; ++u) {
+				const bool live = more && j >= near;
+				bool marked;
+				CHAIN_STEP(r[u], sc[u], live, marked);
+#pragma unroll
+				for (int x = u + 1; x < 4; ++x) r[x].z = marked && r[u].y == j0 - x ? i : r[x].z;
+				j -= live;
 			}
-			const int pj = p[j];
-			if (pj >= 0 && CHK(pj, 14)) t[pj] = i;
 		}
-		f[i] = max_f, p[i] = max_j;
-		v[i] = max_j >= 0 && CHK(max_j, 16) && v[max_j] > max_f ? v[max_j] : max_f;
+		for (; more && j >= st; --j) {
+			const int sc = chain_score(ai, a[j], A);
+			const int4 r = rec[j];
+			bool marked;
+			CHAIN_STEP(r, sc, true, marked);
+		}
+#undef CHAIN_STEP
+		pairs += (unsigned)(i - 1 - j);
+		int pk = max_f;
+		if (max_j >= 0 && CHK(max_j, 16)) pk = max(pk, rec[max_j].w);
+		rec[i] = make_int4(max_f, max_j, 0, pk);
+		f[i] = max_f, p[i] = max_j, v[i] = pk;
 		if (hf < max_f) hf = max_f, hi = i;
 	}
 #undef CHK
@@ -132,13 +195,15 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_fill(plk_chain_args_t A
 
 } /* namespace */
 
-extern "C" int plk_chain_fill(const plk_chain_args_t *a, int32_t n_ctas, void *stream)
+extern "C" int plk_chain_fill(const plk_chain_args_t *a, void *stream)
 {
 	if (a->n_q <= 0) return 0;
 	cudaStream_t st = (cudaStream_t)stream;
-	k_chain_fill<<<n_ctas, CHAIN_THREADS, 0, st>>>(*a);
-	plk_add_launches(1);
+	k_chain_score<<<a->n_q, CHAIN_THREADS, 0, st>>>(*a);
+	cudaError_t e = cudaGetLastError();
+	if (e != cudaSuccess) return (int)e;
+	constexpr int per = CHAIN_THREADS / CHAIN_STRIDE;
+	k_chain_fill<<<(a->n_q + per - 1) / per, CHAIN_THREADS, 0, st>>>(*a);
+	plk_add_launches(2);
 	return (int)cudaGetLastError();
 }
-
-extern "C" int plk_chain_threads_per_cta(void) { return CHAIN_THREADS; }

@@ -200,7 +200,7 @@ PL_EXPORT int pl_chain_finish(const pl_chain_opt_t *opt, int64_t n, const uint64
 void pl_chain_engine_free(pl_engine_t *e)
 {
 	dbuf_free(&e->c_off), dbuf_free(&e->c_n), dbuf_free(&e->c_order), dbuf_free(&e->c_a), dbuf_free(&e->c_f);
-	dbuf_free(&e->c_p), dbuf_free(&e->c_v), dbuf_free(&e->c_t), dbuf_free(&e->c_counter);
+	dbuf_free(&e->c_p), dbuf_free(&e->c_v), dbuf_free(&e->c_rec), dbuf_free(&e->c_rows), dbuf_free(&e->c_row0), dbuf_free(&e->c_counter);
 	if (e->c_host) cudaFreeHost(e->c_host);
 	e->c_host = 0, e->c_host_cap = 0;
 }
@@ -238,13 +238,15 @@ static int pl_chain_cmp_len(const void *x, const void *y)
 	return a < b ? -1 : a > b;
 }
 
+#define PL_CHAIN_ROWS (4LL << 20)  /* anchors whose score rows are held at once: 512 MB */
+
 PL_EXPORT int pl_chain_fill_device(pl_engine_t *e, const pl_chain_opt_t *opt, int32_t n_q, const int64_t *off,
 		const int32_t *n, const uint64_t *a_dev, int64_t n_a, int32_t *f_dev, int32_t *p_dev, int32_t *v_dev,
 		void *stream)
 {
 	pl_chain_opt_t o;
 	plk_chain_args_t A;
-	int64_t *key = 0;
+	int64_t *key = 0, *row0 = 0, rows = 0, max_rows = 0;
 	int32_t *order = 0, q;
 	int ok = 0;
 	cudaStream_t st;
@@ -277,27 +279,44 @@ PL_EXPORT int pl_chain_fill_device(pl_engine_t *e, const pl_chain_opt_t *opt, in
 	st = stream ? (cudaStream_t)stream : e->stream;
 	if (!dbuf_ensure(&e->c_off, sizeof(int64_t) * (size_t)n_q) || !dbuf_ensure(&e->c_n, sizeof(int32_t) * (size_t)n_q) ||
 			!dbuf_ensure(&e->c_order, sizeof(int32_t) * (size_t)n_q) || !dbuf_ensure(&e->c_counter, 64) ||
-			!dbuf_ensure(&e->c_t, sizeof(int32_t) * (size_t)(n_a > 0 ? n_a : 1)))
+			!dbuf_ensure(&e->c_rec, 16 * (size_t)(n_a > 0 ? n_a : 1)))
 		goto fail;
+	/* the score rows, 128 bytes an anchor: launches of as many queries as PL_CHAIN_ROWS holds */
+	row0 = (int64_t*)malloc(sizeof(int64_t) * (size_t)n_q);
+	if (!row0) { pl_set_error("out of host memory"); goto fail; }
+	for (q = 0; q < n_q; ++q) {
+		if (rows > 0 && rows + n[order[q]] > PL_CHAIN_ROWS) rows = 0;
+		row0[q] = rows, rows += n[order[q]];
+		if (rows > max_rows) max_rows = rows;
+	}
+	if (!dbuf_ensure(&e->c_rows, 128 * (size_t)(max_rows > 0 ? max_rows : 1)) ||
+			!dbuf_ensure(&e->c_row0, sizeof(int64_t) * (size_t)n_q))
+		goto fail;
+	CK(cudaMemcpyAsync(e->c_row0.p, row0, sizeof(int64_t) * (size_t)n_q, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->c_off.p, off, sizeof(int64_t) * (size_t)n_q, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->c_n.p, n, sizeof(int32_t) * (size_t)n_q, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->c_order.p, order, sizeof(int32_t) * (size_t)n_q, cudaMemcpyHostToDevice, st));
 	memset(&A, 0, sizeof(A));
-	A.off = (const int64_t*)e->c_off.p, A.n = (const int32_t*)e->c_n.p, A.order = (const int32_t*)e->c_order.p;
-	A.a = a_dev, A.f = f_dev, A.p = p_dev, A.v = v_dev, A.t = (int32_t*)e->c_t.p;
+	A.off = (const int64_t*)e->c_off.p, A.n = (const int32_t*)e->c_n.p;
+	A.a = a_dev, A.f = f_dev, A.p = p_dev, A.v = v_dev, A.rec = e->c_rec.p;
 	A.err = (int32_t*)((char*)e->c_counter.p + 16), A.n_a = n_a;
 	CK(cudaMemsetAsync(A.err, 0, 2 * sizeof(int32_t), st));
-	A.n_q = n_q, A.max_dist_x = o.max_dist_x, A.max_dist_y = o.max_dist_y, A.bw = o.bw, A.max_skip = o.max_skip;
+	A.rows = (int32_t*)e->c_rows.p, A.n_all = n_q;
+	A.max_dist_x = o.max_dist_x, A.max_dist_y = o.max_dist_y, A.bw = o.bw, A.max_skip = o.max_skip;
 	A.max_iter = o.max_iter, A.is_spliced = o.is_spliced, A.kmer = o.kmer, A.bbit = o.bbit, A.coef = o.chn_coef_log;
 	if (e->timing) { /* count the scored predecessors in the scratch block's second half */
 		A.pairs = (unsigned long long*)((char*)e->c_counter.p + 32);
 		CK(cudaMemsetAsync(A.pairs, 0, sizeof(unsigned long long), st));
 	}
 	{
-		const int32_t ctas = (n_q + plk_chain_threads_per_cta() - 1) / plk_chain_threads_per_cta();
+		int32_t q1;
 		e->n_ev = 0;
 		PL_TIME(e, st, 1);
-		CKK(plk_chain_fill(&A, ctas, st));
+		for (q = 0; q < n_q; q = q1) { /* a launch ends where the rows restart (queries without anchors share a row) */
+			for (q1 = q + 1; q1 < n_q && row0[q1] >= row0[q1 - 1] && (row0[q1] > 0 || row0[q1 - 1] + n[order[q1 - 1]] == 0);) ++q1;
+			A.order = (const int32_t*)e->c_order.p + q, A.row0 = (const int64_t*)e->c_row0.p + q, A.n_q = q1 - q;
+			CKK(plk_chain_fill(&A, st));
+		}
 		PL_TIME(e, st, 1);
 	}
 	{ /* the kernel's own index checks: site and query of the last failure */
@@ -321,7 +340,7 @@ PL_EXPORT int pl_chain_fill_device(pl_engine_t *e, const pl_chain_opt_t *opt, in
 	}
 	ok = 1;
 fail:
-	free(key), free(order);
+	free(key), free(order), free(row0);
 	return ok;
 }
 

@@ -82,7 +82,7 @@ struct pl_engine_s {
 	/* prescreen banded alignment */
 	dbuf_t s_jobs, s_pssm, s_orf, s_scr, s_score, s_order;
 	/* anchor chaining */
-	dbuf_t c_off, c_n, c_order, c_a, c_f, c_p, c_v, c_t, c_counter;
+	dbuf_t c_off, c_n, c_order, c_a, c_f, c_p, c_v, c_rec, c_rows, c_row0, c_counter;
 	void *c_host;           /* pinned host buffer for the fill's f and p (grow-only) */
 	size_t c_host_cap;
 	int64_t c_last_pairs;   /* predecessors scored by the last timed fill */

@@ -374,16 +374,18 @@ typedef struct {
 	const int64_t *off;
 	const int32_t *n, *order;
 	const uint64_t *a;
-	int32_t *f, *p, *v, *t;
+	int32_t *f, *p, *v;
+	void *rec;                   /* per anchor 16 bytes of scratch */
+	int32_t *rows;               /* scores against the 32 anchors before, from row row0[i] for query order[i] */
+	const int64_t *row0;
 	unsigned long long *pairs;   /* optional: predecessors scored, summed over queries */
 	int32_t *err;                /* set non-zero by a query whose indices leave their ranges (then skipped) */
-	int64_t n_a;                 /* anchors in a / f / p / v / t */
-	int32_t n_q;
+	int64_t n_a;                 /* anchors in a / f / p / v / rec */
+	int32_t n_q, n_all;          /* queries of this launch, of the batch */
 	int32_t max_dist_x, max_dist_y, bw, max_skip, max_iter, is_spliced, kmer, bbit;
 	float coef;
 } plk_chain_args_t;
-int plk_chain_fill(const plk_chain_args_t *a, int32_t n_ctas, void *stream);
-int plk_chain_threads_per_cta(void);
+int plk_chain_fill(const plk_chain_args_t *a, void *stream);
 
 #ifdef __cplusplus
 }
