@@ -276,16 +276,35 @@ typedef struct {
 	float *Cf; int64_t ldcf;         /* f32 [M x N] */
 	int32_t *err;
 } plk_gemm_t;
-int plk_gemm_smem(int32_t n_tile);
-int plk_gemm_bf16(const plk_gemm_t *a, void *stream);
+/* n <= 4 GEMMs in one launch */
+int plk_gemm_bf16(const plk_gemm_t *a, int32_t n, void *stream);
+/* bias gradients: db[l][n] = the sum of row n of dZT[l] (bf16 [N[l] x B]) */
+typedef struct {
+	const void *dZT[4];
+	float *db[4];
+	int32_t N[4];
+} plk_mlp_bias_t;
+/* parameter tensors of an Adam step */
+typedef struct {
+	float *p, *m, *v;
+	const float *grad;               /* rows ldg apart */
+	void *W, *WT;                    /* bf16 copy [rows x ldw] and its transpose [cols x ldwt], or null */
+	int64_t ldg, ldw, ldwt, flat;  /* flat: place in a model's parameter array */
+	int32_t rows, cols, first;
+	float wd;
+} plk_mlp_tensor_t;
+typedef struct {
+	plk_mlp_tensor_t t[8];
+	int32_t n, pad;
+} plk_mlp_adam_t;
 int plk_mlp_gather(const void *F, int32_t fdim, const int32_t *perm, int64_t n_perm, const int32_t *step,
 		int32_t B, const float *tgt, int32_t tdim, void *X, void *XT, float *T, void *stream);
 int plk_mlp_loss(const float *out, int32_t ldo, const float *T, int32_t B, float pos_w, float box_w,
 		void *dout, int32_t ldd, void *doutT, float *loss_sum, void *stream);
-int plk_mlp_colsum(const void *dZT, int32_t B, int32_t N, float *db, void *stream);
-int plk_mlp_adam(float *p, float *m, float *v, const float *grad, int64_t ldg, int32_t rows, int32_t cols,
-		const int32_t *step, float lr, float b1, float b2, float eps, float wd, void *W, int64_t ldw, void *WT,
-		int64_t ldwt, void *stream);
+int plk_mlp_colsum(const plk_mlp_bias_t *g, int32_t B, void *stream);
+int plk_mlp_adam(const plk_mlp_adam_t *a, const int32_t *step, float lr, float b1, float b2, float eps, void *stream);
+/* all parameters from (load) or to one array */
+int plk_mlp_params(const plk_mlp_adam_t *a, float *flat, int32_t load, void *stream);
 int plk_mlp_step_inc(int32_t *step, float *loss_sum, float *loss_log, int32_t log_cap, void *stream);
 
 /* learned-prefilter features (pffeat.cu) */

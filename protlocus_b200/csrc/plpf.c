@@ -39,7 +39,7 @@ struct pl_pf_model_s {
 	int32_t in_dim, hidden;
 	pf_layer_t L[PF_LAYERS];
 	int32_t *err, *step;
-	float *loss_sum, *loss_log;
+	float *loss_sum, *loss_log, *flat;
 	/* training buffers for batch size tb */
 	int32_t tb;
 	void *X, *XT, *H[3], *HT[3], *dout, *doutT, *dZ[3], *dZT[3];
@@ -87,7 +87,7 @@ PL_EXPORT void pl_pf_model_destroy(pl_pf_model_t *m)
 		cudaFree(y->p), cudaFree(y->m), cudaFree(y->v), cudaFree(y->pb), cudaFree(y->mb), cudaFree(y->vb);
 		cudaFree(y->W), cudaFree(y->WT), cudaFree(y->gW), cudaFree(y->gb);
 	}
-	cudaFree(m->err), cudaFree(m->step), cudaFree(m->loss_sum), cudaFree(m->loss_log);
+	cudaFree(m->err), cudaFree(m->step), cudaFree(m->loss_sum), cudaFree(m->loss_log), cudaFree(m->flat);
 	free(m);
 }
 
@@ -100,50 +100,37 @@ PL_EXPORT int64_t pl_pf_model_size(const pl_pf_model_t *m)
 	return n;
 }
 
-/* bf16 copies of the masters (round to nearest even) */
-static uint16_t f2bf(float f)
+/* the parameter tensors */
+static void pf_tensors(const pl_pf_model_t *m, plk_mlp_adam_t *a)
 {
-	uint32_t u;
-	memcpy(&u, &f, 4);
-	if ((u & 0x7f800000u) == 0x7f800000u) return (uint16_t)(u >> 16);
-	u += 0x7fffu + ((u >> 16) & 1u);
-	return (uint16_t)(u >> 16);
+	int64_t flat = 0;
+	int l;
+	memset(a, 0, sizeof(*a));
+	for (l = 0; l < PF_LAYERS; ++l) {
+		const pf_layer_t *y = &m->L[l];
+		plk_mlp_tensor_t *w = &a->t[2 * l], *b = &a->t[2 * l + 1];
+		w->p = y->p, w->m = y->m, w->v = y->v, w->grad = y->gW, w->ldg = y->in, w->rows = y->out, w->cols = y->in;
+		w->W = y->W, w->ldw = y->in, w->WT = y->WT, w->ldwt = y->out_pad, w->wd = 1e-5f;
+		w->flat = flat, flat += (int64_t)y->out * y->in;
+		b->p = y->pb, b->m = y->mb, b->v = y->vb, b->grad = y->gb, b->ldg = 1, b->rows = y->out, b->cols = 1;
+		b->flat = flat, flat += y->out;
+	}
+	a->n = 2 * PF_LAYERS;
 }
 
+/* all parameters from a host array: one copy up, then the masters, their bf16 copies and the
+ * cleared moments by one kernel */
 static int pf_upload(pl_pf_model_t *m, const float *params)
 {
-	int l;
-	int64_t off = 0;
-	uint16_t *wb = 0, *wt = 0;
-	int ok = 0;
-	for (l = 0; l < PF_LAYERS; ++l) {
-		pf_layer_t *y = &m->L[l];
-		const int64_t nw = (int64_t)y->out * y->in;
-		int64_t r, c;
-		wb = (uint16_t*)malloc(sizeof(uint16_t) * (size_t)nw);
-		wt = (uint16_t*)calloc((size_t)y->in * y->out_pad, sizeof(uint16_t));
-		if (!wb || !wt) { pl_set_error("out of host memory"); goto fail; }
-		for (r = 0; r < y->out; ++r)
-			for (c = 0; c < y->in; ++c) {
-				const uint16_t b = f2bf(params[off + r * y->in + c]);
-				wb[r * y->in + c] = b, wt[c * y->out_pad + r] = b;
-			}
-		CK(cudaMemcpy(y->p, params + off, sizeof(float) * (size_t)nw, cudaMemcpyHostToDevice));
-		CK(cudaMemcpy(y->pb, params + off + nw, sizeof(float) * (size_t)y->out, cudaMemcpyHostToDevice));
-		CK(cudaMemcpy(y->W, wb, sizeof(uint16_t) * (size_t)nw, cudaMemcpyHostToDevice));
-		CK(cudaMemcpy(y->WT, wt, sizeof(uint16_t) * (size_t)y->in * y->out_pad, cudaMemcpyHostToDevice));
-		CK(cudaMemset(y->m, 0, sizeof(float) * (size_t)nw));
-		CK(cudaMemset(y->v, 0, sizeof(float) * (size_t)nw));
-		CK(cudaMemset(y->mb, 0, sizeof(float) * (size_t)y->out));
-		CK(cudaMemset(y->vb, 0, sizeof(float) * (size_t)y->out));
-		free(wb), free(wt), wb = wt = 0;
-		off += nw + y->out;
-	}
-	CK(cudaMemset(m->step, 0, sizeof(int32_t)));
-	ok = 1;
+	plk_mlp_adam_t a;
+	pf_tensors(m, &a);
+	CK(cudaMemcpy(m->flat, params, sizeof(float) * (size_t)pl_pf_model_size(m), cudaMemcpyHostToDevice));
+	CKK(plk_mlp_params(&a, m->flat, 1, 0));
+	CK(cudaMemsetAsync(m->step, 0, sizeof(int32_t), 0));
+	CK(cudaStreamSynchronize(0));
+	return 1;
 fail:
-	free(wb), free(wt);
-	return ok;
+	return 0;
 }
 
 PL_EXPORT int pl_pf_model_set(pl_pf_model_t *m, const float *params, int64_t n)
@@ -156,18 +143,13 @@ PL_EXPORT int pl_pf_model_set(pl_pf_model_t *m, const float *params, int64_t n)
 
 PL_EXPORT int pl_pf_model_get(const pl_pf_model_t *m, float *params, int64_t n)
 {
-	int l;
-	int64_t off = 0;
+	plk_mlp_adam_t a;
 	if (!m || !params || n != pl_pf_model_size(m)) { pl_set_error("parameter count mismatch"); return 0; }
 	CK(cudaSetDevice(m->device));
 	CK(cudaDeviceSynchronize());
-	for (l = 0; l < PF_LAYERS; ++l) {
-		const pf_layer_t *y = &m->L[l];
-		const int64_t nw = (int64_t)y->out * y->in;
-		CK(cudaMemcpy(params + off, y->p, sizeof(float) * (size_t)nw, cudaMemcpyDeviceToHost));
-		CK(cudaMemcpy(params + off + nw, y->pb, sizeof(float) * (size_t)y->out, cudaMemcpyDeviceToHost));
-		off += nw + y->out;
-	}
+	pf_tensors(m, &a);
+	CKK(plk_mlp_params(&a, m->flat, 0, 0));
+	CK(cudaMemcpy(params, m->flat, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost));
 	return 1;
 fail:
 	return 0;
@@ -202,12 +184,14 @@ PL_EXPORT pl_pf_model_t *pl_pf_model_create(int32_t device, int32_t in_dim, int3
 		CK(cudaMalloc((void**)&y->vb, sizeof(float) * (size_t)y->out));
 		CK(cudaMalloc(&y->W, 2 * (size_t)nw));
 		CK(cudaMalloc(&y->WT, 2 * (size_t)y->in * y->out_pad));
+		CK(cudaMemset(y->WT, 0, 2 * (size_t)y->in * y->out_pad));  /* the padding columns stay zero */
 		CK(cudaMalloc((void**)&y->gW, sizeof(float) * (size_t)grow * y->in));
 		CK(cudaMalloc((void**)&y->gb, sizeof(float) * (size_t)y->out));
 	}
 	CK(cudaMalloc((void**)&m->err, sizeof(int32_t)));
 	CK(cudaMalloc((void**)&m->step, sizeof(int32_t)));
 	CK(cudaMalloc((void**)&m->loss_sum, sizeof(float)));
+	CK(cudaMalloc((void**)&m->flat, sizeof(float) * (size_t)pl_pf_model_size(m)));
 	CK(cudaMalloc((void**)&m->loss_log, sizeof(float) * PF_LOG_CAP));
 	CK(cudaMemset(m->err, 0, sizeof(int32_t)));
 	CK(cudaMemset(m->loss_sum, 0, sizeof(float)));
@@ -244,17 +228,13 @@ static int pf_gemm(pl_pf_model_t *m, const void *A, int64_t lda, const void *B, 
 	g.A = A, g.lda = lda, g.B = B, g.ldb = ldb, g.M = M, g.N = N, g.K = K, g.n_tile = n_tile;
 	g.bias = bias, g.relu = relu, g.mask = mask, g.ldm = ldm, g.C = C, g.ldc = ldc, g.CT = CT, g.ldct = ldct;
 	g.Cf = Cf, g.ldcf = ldcf, g.err = m->err;
-	return plk_gemm_bf16(&g, st);
+	return plk_gemm_bf16(&g, 1, st);
 }
 
-/* n_tile for N columns: one tile up to 256, else the largest multiple of 16 <= 256 dividing N */
-static int32_t pf_tile(int32_t N)
-{
-	int32_t t;
-	if (N <= 256) return N;
-	for (t = 256; t >= 16; t -= 16) if (N % t == 0) return t;
-	return 16;
-}
+/* n_tile of an M x N output (N = hidden, 128 or 256): all columns in one tile where the row tiles
+ * make two waves of the SMs, else 64, which gives four times the CTAs for A read four times from
+ * L2 (4096 rows: 32 CTAs or 128) */
+static int32_t pf_tile(int32_t M, int32_t N) { return M / 128 >= 296 ? N : 64; }
 
 /* forward of rows [0, M) of X (bf16 [M x in]) into H[0..2] (and their transposes when HT) and out f32 [M x 16] */
 static int pf_forward(pl_pf_model_t *m, const void *X, int32_t M, void *const *H, void *const *HT, float *out, cudaStream_t st)
@@ -264,7 +244,7 @@ static int pf_forward(pl_pf_model_t *m, const void *X, int32_t M, void *const *H
 	for (l = 0; l < 3; ++l) {
 		const void *in = l == 0 ? X : H[l - 1];
 		const int64_t ld_in = l == 0 ? m->in_dim : h;
-		int e = pf_gemm(m, in, ld_in, m->L[l].W, m->L[l].in, M, h, m->L[l].in, pf_tile(h), m->L[l].pb, 1, 0, 0,
+		int e = pf_gemm(m, in, ld_in, m->L[l].W, m->L[l].in, M, h, m->L[l].in, pf_tile(M, h), m->L[l].pb, 1, 0, 0,
 				H[l], h, HT ? HT[l] : 0, M, 0, 0, st);
 		if (e) return e;
 	}
@@ -327,33 +307,34 @@ static int pf_step(pl_pf_model_t *m, const void *feats, const float *tgt, const 
 		float lr, float pos_w, float box_w, cudaStream_t st)
 {
 	const int32_t B = m->tb, h = m->hidden, in = m->in_dim;
-	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f, wd = 1e-5f;
+	const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+	plk_mlp_adam_t ad;
+	plk_mlp_bias_t bg;
+	plk_gemm_t g[PF_LAYERS];
 	int l, e;
 #define T_(x) do { if ((e = (x)) != 0) return e; } while (0)
 	T_(plk_mlp_gather(feats, in, perm, n_perm, m->step, B, tgt, 4, m->X, m->XT, m->T, st));
 	T_(pf_forward(m, m->X, B, m->H, m->HT, m->out, st));
 	T_(plk_mlp_loss(m->out, PF_OUT, m->T, B, pos_w, box_w, m->dout, PF_OUT_PAD, m->doutT, m->loss_sum, st));
-	/* output layer: gW3 = dout^T . H3 (rows >= 16 of dout^T are zero), db3; dZ2 = (dout . W3) masked by H3 */
-	T_(pf_gemm(m, m->doutT, B, m->HT[2], B, PF_OUT_ROWS, h, B, pf_tile(h), 0, 0, 0, 0, 0, 0, 0, 0, m->L[3].gW, h, st));
-	T_(plk_mlp_colsum(m->doutT, B, PF_OUT, m->L[3].gb, st));
-	T_(pf_gemm(m, m->dout, PF_OUT_PAD, m->L[3].WT, PF_OUT_PAD, B, h, PF_OUT_PAD, pf_tile(h), 0, 0, m->H[2], h,
+	/* dZ2 = (dout . W3) masked by H2, dZ_{l-1} = (dZ_l . W_l) masked by H_{l-1} */
+	T_(pf_gemm(m, m->dout, PF_OUT_PAD, m->L[3].WT, PF_OUT_PAD, B, h, PF_OUT_PAD, pf_tile(B, h), 0, 0, m->H[2], h,
 			m->dZ[2], h, m->dZT[2], B, 0, 0, st));
-	for (l = 2; l >= 0; --l) {
-		/* gW_l = dZ_l^T . (input of layer l); db_l; dZ_{l-1} = (dZ_l . W_l) masked by H_{l-1} */
-		const void *inT = l == 0 ? m->XT : m->HT[l - 1];
-		const int32_t K_in = l == 0 ? in : h;
-		T_(pf_gemm(m, m->dZT[l], B, inT, B, h, K_in, B, pf_tile(K_in), 0, 0, 0, 0, 0, 0, 0, 0, m->L[l].gW, K_in, st));
-		T_(plk_mlp_colsum(m->dZT[l], B, h, m->L[l].gb, st));
-		if (l > 0)
-			T_(pf_gemm(m, m->dZ[l], h, m->L[l].WT, m->L[l].out_pad, B, h, h, pf_tile(h), 0, 0, m->H[l - 1], h,
-					m->dZ[l - 1], h, m->dZT[l - 1], B, 0, 0, st));
-	}
+	for (l = 2; l > 0; --l)
+		T_(pf_gemm(m, m->dZ[l], h, m->L[l].WT, m->L[l].out_pad, B, h, h, pf_tile(B, h), 0, 0, m->H[l - 1], h,
+				m->dZ[l - 1], h, m->dZT[l - 1], B, 0, 0, st));
+	/* gW_l = dZ_l^T . (input of layer l), the output layer's dout^T . H2 (rows >= 16 of dout^T are
+	 * zero), one launch; then all bias gradients */
+	pf_tensors(m, &ad);
+	memset(g, 0, sizeof(g));
 	for (l = 0; l < PF_LAYERS; ++l) {
-		pf_layer_t *y = &m->L[l];
-		T_(plk_mlp_adam(y->p, y->m, y->v, y->gW, y->in, y->out, y->in, m->step, lr, b1, b2, eps, wd, y->W, y->in, y->WT,
-				y->out_pad, st));
-		T_(plk_mlp_adam(y->pb, y->mb, y->vb, y->gb, 1, y->out, 1, m->step, lr, b1, b2, eps, 0.0f, 0, 0, 0, 0, st));
+		g[l].A = l == 3 ? m->doutT : m->dZT[l], g[l].lda = B, g[l].B = l == 0 ? m->XT : m->HT[l - 1], g[l].ldb = B;
+		g[l].M = l == 3 ? PF_OUT_ROWS : h, g[l].N = m->L[l].in, g[l].K = B, g[l].n_tile = 16;
+		g[l].Cf = m->L[l].gW, g[l].ldcf = m->L[l].in, g[l].err = m->err;
+		bg.dZT[l] = g[l].A, bg.db[l] = m->L[l].gb, bg.N[l] = m->L[l].out;
 	}
+	T_(plk_gemm_bf16(g, PF_LAYERS, st));
+	T_(plk_mlp_colsum(&bg, B, st));
+	T_(plk_mlp_adam(&ad, m->step, lr, b1, b2, eps, st));
 	T_(plk_mlp_step_inc(m->step, m->loss_sum, m->loss_log, PF_LOG_CAP, st));
 #undef T_
 	return 0;
@@ -393,7 +374,7 @@ PL_EXPORT int pl_pf_train(pl_pf_model_t *m, const void *feats, const float *targ
 	CK(cudaMemcpyAsync(&step0, m->step, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
 	for (i = 0; i < steps; ++i) CK(cudaGraphLaunch(m->gexec, st));
-	plk_add_launches((uint64_t)steps * 26);
+	plk_add_launches((uint64_t)steps * 13);
 	CK(cudaStreamSynchronize(st));
 	CK(cudaMemcpy(&err, m->err, sizeof(int32_t), cudaMemcpyDeviceToHost));
 	if (err) { pl_set_error("tensor-core GEMM reported a wait timeout"); goto fail; }
@@ -421,7 +402,7 @@ PL_EXPORT int pl_pf_gemm(int32_t device, const void *A, int64_t lda, const void 
 	g.A = A, g.lda = lda, g.B = B, g.ldb = ldb, g.M = M, g.N = N, g.K = K, g.n_tile = n_tile;
 	g.bias = bias, g.relu = relu, g.mask = mask, g.ldm = ldm, g.C = C, g.ldc = ldc, g.CT = CT, g.ldct = ldct;
 	g.Cf = Cf, g.ldcf = ldcf, g.err = err;
-	e = plk_gemm_bf16(&g, stream);
+	e = plk_gemm_bf16(&g, 1, stream);
 	if (e) { pl_set_error("GEMM launch: %s", cudaGetErrorString((cudaError_t)e)); return 0; }
 	return 1;
 }
