@@ -921,6 +921,7 @@ struct ns_gpu_request_s {
 	int8_t sc[22 * 22];
 	uint8_t nt4[256], aa20[256], codon[64];
 	int32_t score, n_cigar, done, success;
+	int32_t taken, waited;      /* in a batch; its submitter is in ns_gpu_wait (counted while queued) */
 	uint32_t *cigar;
 	struct ns_gpu_request_s *next;
 };
@@ -929,12 +930,28 @@ static pthread_mutex_t ns_mu = PTHREAD_MUTEX_INITIALIZER;
 static pthread_cond_t ns_cv_work = PTHREAD_COND_INITIALIZER, ns_cv_done = PTHREAD_COND_INITIALIZER;
 static ns_gpu_request_t *ns_q_head, *ns_q_tail;
 static int32_t ns_q_n;
+/* When a batch is complete.  A request is worth waiting for only while some caller that could
+ * send it is not waiting itself.  So the collection ends before its 2 ms once a caller waits for a
+ * queued request and the queue holds as many requests as were ever outstanding at once around the
+ * last batches: a lone caller, who sends one request and waits, is served at once (2.0 of the
+ * 4.7 ms of a 350-residue protein against a 40 kb window were this wait), T callers get one batch
+ * of T as soon as the last of them is back, and requests sent ahead of any wait are collected as
+ * before. */
+#define NS_PEAKS 8
+static int32_t ns_q_waited, ns_out, ns_out_peak, ns_peaks[NS_PEAKS], ns_peak_at;
 static int ns_ready;
 static pl_engine_t *ns_engine;
 static pthread_t ns_thread;
 static uint64_t ns_dispatches, ns_launches, ns_h2d_ns, ns_kernel_ns, ns_d2h_ns;
 static char ns_msg[1024] = "GPU backend has not been initialized";
 static char ns_dev_name[256] = "none";
+
+static int ns_all_here(void)
+{ /* under ns_mu */
+	int i, peak = 1;
+	for (i = 0; i < NS_PEAKS; ++i) if (peak < ns_peaks[i]) peak = ns_peaks[i];
+	return ns_q_waited > 0 && ns_q_n >= peak;
+}
 
 static uint64_t ns_now_ns(void)
 {
@@ -1002,6 +1019,7 @@ done:
 	if (ok) __sync_fetch_and_add(&ns_dispatches, (uint64_t)n), __sync_fetch_and_add(&ns_launches, 1ull);
 	pthread_mutex_lock(&ns_mu);
 	for (q = 0; q < n; ++q) rq[q]->done = 1;
+	ns_out -= n;
 	pthread_cond_broadcast(&ns_cv_done);
 	pthread_mutex_unlock(&ns_mu);
 	free(jobs), free(res), free(nt), free(aa), free(ss), free(cig);
@@ -1017,12 +1035,12 @@ static void *ns_executor(void *arg)
 		ns_gpu_request_t **pp;
 		pthread_mutex_lock(&ns_mu);
 		while (ns_q_n == 0) pthread_cond_wait(&ns_cv_work, &ns_mu);
-		if (ns_q_n < NS_REQ_MAX_BATCH) { /* let concurrent submitters join the batch */
+		if (ns_q_n < NS_REQ_MAX_BATCH && !ns_all_here()) { /* let concurrent submitters join the batch */
 			struct timespec until;
 			clock_gettime(CLOCK_REALTIME, &until);
 			until.tv_nsec += NS_REQ_WAIT_NS;
 			if (until.tv_nsec >= 1000000000L) until.tv_sec += 1, until.tv_nsec -= 1000000000L;
-			while (ns_q_n < NS_REQ_MAX_BATCH)
+			while (ns_q_n < NS_REQ_MAX_BATCH && !ns_all_here())
 				if (pthread_cond_timedwait(&ns_cv_work, &ns_mu, &until) == ETIMEDOUT) break;
 		}
 		/* take up to 128 requests sharing the first one's options */
@@ -1031,11 +1049,12 @@ static void *ns_executor(void *arg)
 			ns_gpu_request_t *r = *pp;
 			if (n == 0 || ns_same_opt(batch[0], r)) {
 				*pp = r->next, batch[n++] = r, --ns_q_n;
-				r->next = 0;
+				r->next = 0, r->taken = 1, ns_q_waited -= r->waited;
 			} else pp = &r->next;
 		}
 		ns_q_tail = 0;
 		for (pp = &ns_q_head; *pp; pp = &(*pp)->next) ns_q_tail = *pp;
+		ns_peaks[ns_peak_at] = ns_out_peak, ns_peak_at = (ns_peak_at + 1) % NS_PEAKS, ns_out_peak = ns_out;
 		pthread_mutex_unlock(&ns_mu);
 		ns_run_batch(batch, n);
 	}
@@ -1128,6 +1147,7 @@ PL_EXPORT ns_gpu_request_t *ns_gpu_submit(void *km, const char *ns, int32_t nl, 
 	pthread_mutex_lock(&ns_mu);
 	if (ns_q_tail) ns_q_tail->next = r; else ns_q_head = r;
 	ns_q_tail = r, ++ns_q_n;
+	if (++ns_out > ns_out_peak) ns_out_peak = ns_out;
 	pthread_cond_broadcast(&ns_cv_work);
 	pthread_mutex_unlock(&ns_mu);
 	return r;
@@ -1138,6 +1158,10 @@ PL_EXPORT int ns_gpu_wait(ns_gpu_request_t *r, ns_rst_t *rst)
 	int success, k;
 	if (!r) return 0;
 	pthread_mutex_lock(&ns_mu);
+	if (!r->taken) {
+		r->waited = 1, ++ns_q_waited;
+		pthread_cond_broadcast(&ns_cv_work);
+	}
 	while (!r->done) pthread_cond_wait(&ns_cv_done, &ns_mu);
 	pthread_mutex_unlock(&ns_mu);
 	success = r->success;
