@@ -77,6 +77,26 @@ static int pl_xbucket(const plk_ext_job_t *J)
 	return (J->mode / 2 * 4 + J->variant) * 256 + (255 - (lg * 4 + frac > 255 ? 255 : lg * 4 + frac));
 }
 
+/* Pairs (two requests in the halves of one warp's registers, ext.cu) are made of neighbours in this
+ * order: the same number of strips, then the padded column count, so that little of either half's
+ * wave is past its own end; longest first. */
+#define PL_XPBUCKETS (256 * 256)
+static int pl_xpbucket(const plk_ext_job_t *J)
+{
+	const int ns = (J->nl - 2 + 255) / 256, nc = J->ncol >> 2;
+	return (255 - (ns > 255 ? 255 : ns)) * 256 + (255 - (nc > 255 ? 255 : nc));
+}
+
+/* Requests that a pair can hold: a right or left extension without position-specific scores, values
+ * under the pairs' bound over the padded columns, narrow keys, and at least 31 residues (a lane's
+ * next strip then does not reach its padding columns before this one is scanned).  They run in pairs
+ * when the pairs fill the launch's warps PL_XPAIR_FILL times: a pair's wave takes longer than a
+ * single request's, so with fewer the last pairs cost more than the halves save (64-256 residues:
+ * 5,000 requests, 1.4 times, 3.64 ms single and 4.29 paired; 8,192, 2.3 times, 4.87 and 4.41;
+ * 65,536 37.3 and 25.9).  PLGPU_PAIR=0 turns pairs off, engine pairing 2 takes every one. */
+#define PL_XPAIR_MIN_AL 31
+#define PL_XPAIR_FILL 2.0
+
 /* the reference's answer when the DP has no row (nl < 3): the row loop of
  * nasw-sse.c:361 does not run and the column pick of :448-458 reads the
  * initial -32768 row, end_bonus added at al-1 */
@@ -94,7 +114,8 @@ static int pl_ext_run(pl_engine_t *e, const ns_opt_t *opt, const pl_ext_job_t *j
 {
 	plk_params_t P;
 	int32_t *key = 0;   /* bucket counts, then bucket starts */
-	int32_t q, n_dp = 0, max_sub;
+	int32_t *pkey = 0, *hpair = 0;  /* the pairs' buckets and order */
+	int32_t q, n_dp = 0, n_el = 0, n_single = 0, n_pairs = 0, pair_ctas = 0, max_sub, al_cap = 0, bias = 0, can_pair;
 	int64_t prep_total = 0, cells_nominal = 0;
 	unsigned long long cells_run = 0;
 	int ok = 0;
@@ -106,13 +127,14 @@ static int pl_ext_run(pl_engine_t *e, const ns_opt_t *opt, const pl_ext_job_t *j
 	if (n > e->x_m) {
 		free(e->x_hj), free(e->x_horder);
 		e->x_hj = (plk_ext_job_t*)calloc((size_t)n, sizeof(plk_ext_job_t));
-		e->x_horder = (int32_t*)malloc(sizeof(int32_t) * (size_t)n);
+		e->x_horder = (int32_t*)malloc(sizeof(int32_t) * ((size_t)n + 1));
 		e->x_m = e->x_hj && e->x_horder ? n : 0;
 		if (!e->x_m) { pl_set_error("out of host memory"); return 0; }
 	}
 	key = (int32_t*)calloc(PL_XBUCKETS + 1, sizeof(int32_t));
 	if (!key) { pl_set_error("out of host memory"); return 0; }
 	max_sub = pl_max_sub(opt);
+	can_pair = e->pairing && opt->end_bonus >= 0 && opt->end_bonus <= 65535 && pl_pair_limits(opt, max_sub, &al_cap, &bias);
 	for (q = 0; q < n; ++q) {
 		const pl_ext_job_t *x = &jobs[q];
 		plk_ext_job_t *J = &e->x_hj[q];
@@ -145,32 +167,70 @@ static int pl_ext_run(pl_engine_t *e, const ns_opt_t *opt, const pl_ext_job_t *j
 		}
 		J->prep_off = prep_total, prep_total += plk_prep_bytes(x->nl, x->al);
 		cells_nominal += (int64_t)(x->nl - 2) * x->al;
-		++key[pl_xbucket(J) + 1];
+		if (can_pair && J->mode == 0 && J->variant == 0 && kind != 2 && J->al >= PL_XPAIR_MIN_AL && J->ncol <= al_cap) J->pad = 1, ++n_el;
 		++n_dp;
 	}
+	if (n_el > 1) {
+		pair_ctas = plk_ext_ctas_per_sm(3, 0);
+		if (pair_ctas < 1) { pl_set_error("extension DP kernel does not fit on an SM"); goto fail; }
+		pair_ctas *= e->n_sm;
+		if (e->pairing == 2 || n_el / 2 >= PL_XPAIR_FILL * pair_ctas * plk_ext_warps_per_cta()) n_pairs = (n_el + 1) / 2;
+	}
+	if (n_pairs > 0) {
+		pkey = (int32_t*)calloc(PL_XPBUCKETS + 1, sizeof(int32_t));
+		if (!pkey) { pl_set_error("out of host memory"); goto fail; }
+	}
+	for (q = 0; q < n; ++q) {
+		plk_ext_job_t *J = &e->x_hj[q];
+		if (jobs[q].nl < 3) continue;
+		if (J->pad && n_pairs > 0) ++pkey[pl_xpbucket(J) + 1];
+		else J->pad = 0, ++key[pl_xbucket(J) + 1], ++n_single;
+	}
 	for (q = 0; q < PL_XBUCKETS; ++q) key[q + 1] += key[q];
-	for (q = 0; q < n; ++q)
-		if (jobs[q].nl >= 3) e->x_horder[key[pl_xbucket(&e->x_hj[q])]++] = q;
+	if (n_pairs > 0) {
+		for (q = 0; q < PL_XPBUCKETS; ++q) pkey[q + 1] += pkey[q];
+		hpair = e->x_horder + n_single;
+	}
+	for (q = 0; q < n; ++q) {
+		if (jobs[q].nl < 3) continue;
+		if (e->x_hj[q].pad) hpair[pkey[pl_xpbucket(&e->x_hj[q])]++] = q;
+		else e->x_horder[key[pl_xbucket(&e->x_hj[q])]++] = q;
+	}
+	if (n_el & 1 && n_pairs > 0) hpair[n_el] = hpair[n_el - 1];  /* an odd last one goes with itself */
 	if (!dbuf_ensure(&e->x_jobs, sizeof(plk_ext_job_t) * (size_t)n) ||
-			!dbuf_ensure(&e->x_order, sizeof(int32_t) * (size_t)(n_dp > 0 ? n_dp : 1)) ||
+			!dbuf_ensure(&e->x_order, sizeof(int32_t) * (size_t)(n_single + 2 * n_pairs > 0 ? n_single + 2 * n_pairs : 1)) ||
 			!dbuf_ensure(&e->x_counter, 64) || !dbuf_ensure(&e->x_prep, (size_t)(prep_total > 0 ? prep_total : 16)))
 		goto fail;
 	CK(cudaMemcpyAsync(e->x_jobs.p, e->x_hj, sizeof(plk_ext_job_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemsetAsync(e->x_counter.p, 0, 64, st));
 	if (n_dp > 0) {
 		int32_t g0 = 0;
-		CK(cudaMemcpyAsync(e->x_order.p, e->x_horder, sizeof(int32_t) * (size_t)n_dp, cudaMemcpyHostToDevice, st));
+		CK(cudaMemcpyAsync(e->x_order.p, e->x_horder, sizeof(int32_t) * (size_t)(n_single + 2 * n_pairs), cudaMemcpyHostToDevice, st));
 		e->n_ev = 0;
 		PL_TIME(e, st, 0);
 		CKK(plk_ext_prep((const plk_ext_job_t*)e->x_jobs.p, n, nt, aa, ss, (uint8_t*)e->x_prep.p, &P, st));
 		PL_TIME(e, st, 0);
 		++e->x_last_launches;
-		while (g0 < n_dp) { /* one launch per (mode, variant) group */
+		if (n_pairs > 0) {
+			int32_t max_ncol = 1, ctas = pair_ctas;
+			int64_t stride;
+			for (q = 0; q < n_el; ++q) if (e->x_hj[hpair[q]].ncol > max_ncol) max_ncol = e->x_hj[hpair[q]].ncol;
+			if ((int64_t)ctas * plk_ext_warps_per_cta() > n_pairs) ctas = (n_pairs + plk_ext_warps_per_cta() - 1) / plk_ext_warps_per_cta();
+			stride = ((int64_t)max_ncol + 1) * PLK_RING_INTS;
+			if (!dbuf_ensure(&e->x_ring, sizeof(int32_t) * (size_t)(stride * ctas * plk_ext_warps_per_cta()))) goto fail;
+			P.pair_b = bias, P.pair_f = PL_PAIR_F;
+			PL_TIME(e, st, 1);
+			CKK(plk_ext_pair((plk_ext_job_t*)e->x_jobs.p, (const int32_t*)e->x_order.p + n_single, n_pairs,
+					(int32_t*)e->x_counter.p, (const uint8_t*)e->x_prep.p, (int32_t*)e->x_ring.p, stride, ctas, &P, st));
+			PL_TIME(e, st, 1);
+			++e->x_last_launches;
+		}
+		while (g0 < n_single) { /* one launch per (mode, variant) group */
 			const plk_ext_job_t *J0 = &e->x_hj[e->x_horder[g0]];
 			const int mode = J0->mode, variant = J0->variant;
 			int32_t g1 = g0, max_ncol = 1, ctas;
 			int64_t stride;
-			while (g1 < n_dp && e->x_hj[e->x_horder[g1]].mode == mode && e->x_hj[e->x_horder[g1]].variant == variant) {
+			while (g1 < n_single && e->x_hj[e->x_horder[g1]].mode == mode && e->x_hj[e->x_horder[g1]].variant == variant) {
 				if (e->x_hj[e->x_horder[g1]].ncol > max_ncol) max_ncol = e->x_hj[e->x_horder[g1]].ncol;
 				++g1;
 			}
@@ -207,7 +267,7 @@ static int pl_ext_run(pl_engine_t *e, const ns_opt_t *opt, const pl_ext_job_t *j
 	}
 	ok = 1;
 fail:
-	free(key);
+	free(key), free(pkey);
 	return ok;
 }
 

@@ -360,8 +360,7 @@ static double pl_union_ms(double *a, double *b, int n)
  * job of protein length al is admitted when [low bound, high bound] fits between
  * F + 512 and 0x7fff - 512 after biasing; every penalty stays below F so that the
  * floor never wraps under a subtraction. */
-#define PL_PAIR_F 512
-static int pl_pair_limits(const ns_opt_t *opt, int max_sub, int32_t *al_cap, int32_t *bias)
+int pl_pair_limits(const ns_opt_t *opt, int max_sub, int32_t *al_cap, int32_t *bias)
 {
 	int i, s_min = 0;
 	int64_t c_low, per_al, cap;

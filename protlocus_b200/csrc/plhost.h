@@ -107,6 +107,9 @@ void pl_set_error(const char *fmt, ...);
 double pl_coop_ratio(void);
 int32_t pl_r4_rows(void);
 int pl_params(const ns_opt_t *opt, plk_params_t *p, int for_ext);
+/* int16x2 pairs: the longest protein and the bias of the values (plgpu.c); the floor */
+int pl_pair_limits(const ns_opt_t *opt, int max_sub, int32_t *al_cap, int32_t *bias);
+#define PL_PAIR_F 512
 int pl_max_sub(const ns_opt_t *opt);
 void pl_ext_engine_free(pl_engine_t *e);
 void pl_hmm_engine_free(pl_engine_t *e);

@@ -85,7 +85,7 @@ typedef struct {
 	int32_t variant;                 /* bit 0: position-specific scores, bit 1: wide row keys */
 	int32_t nt_len, aa_len, score;   /* outputs */
 	int32_t status;                  /* 0 = ok */
-	int32_t pad;
+	int32_t pad;                     /* 1: runs in a pair (host) */
 } plk_ext_job_t;
 
 /* a profile of the integer HMM DP on the device (hmm.c:14-22 tables, re-laid out) */
@@ -154,6 +154,8 @@ int plk_scan_compact(plk_job_t *jobs, int32_t n_jobs, const uint32_t *tmp, uint3
  * position-specific score buffer (variant bit 0). */
 int plk_ext_prep(const plk_ext_job_t *jobs, int32_t n_jobs, const uint8_t *nt, const uint8_t *aa, const uint8_t *ss,
 		uint8_t *prep, const plk_params_t *p, void *stream);
+int plk_ext_pair(plk_ext_job_t *jobs, const int32_t *order, int32_t n_pairs, int32_t *counter, const uint8_t *prep,
+		int32_t *ring, int64_t ring_stride_ints, int32_t n_ctas, const plk_params_t *p, void *stream);
 int plk_ext_dp(plk_ext_job_t *jobs, const int32_t *order, int32_t n_jobs, int32_t *counter, const uint8_t *prep,
 		const int8_t *pssm, int32_t *ring, int64_t ring_stride_ints, int32_t n_ctas, int32_t mode, int32_t variant,
 		const plk_params_t *p, void *stream);
