@@ -777,7 +777,7 @@ def main_ext(args):
                        "l2": "a 256 MB buffer is written between timed steps", "parallelism": f"{world} independent ranks"},
             "e2e": e2e,
             "gpu_launches": int(launches),
-            "roofline": {"bound": "int", "kernel": "k_ext_dp", "achieved": achieved, "peak": peak,
+            "roofline": {"bound": "int", "kernel": "k_ext_pair", "achieved": achieved, "peak": peak,
                          "unit": "lane-ops/s", "frac": achieved / peak if peak else None, "traffic": None,
                          "ops_per_cell": EXT_OPS_PER_CELL,
                          "dp_kernel_gcups_algorithmic": round(tm["cells"] / dp_s / 1e9, 3) if dp_s > 0 else None,
@@ -1015,12 +1015,13 @@ def main_hmm(args):
                        "l2": "a 256 MB buffer is written between timed steps", "parallelism": f"{world} independent ranks"},
             "e2e": e2e,
             "gpu_launches": int(launches),
-            "roofline": {"bound": "int", "kernel": "k_hmm_dp", "achieved": achieved, "peak": int32_peak,
-                         "unit": "lane-ops/s", "frac": achieved / int32_peak if int32_peak else None, "traffic": None,
+            "roofline": {"bound": "int", "kernel": "k_hmm_pair", "achieved": achieved, "peak": i16x2_peak,
+                         "unit": "lane-ops/s", "frac": achieved / i16x2_peak if i16x2_peak else None, "traffic": None,
                          "ops_per_cell": HMM_OPS_PER_CELL,
                          "dp_kernel_gcups": round(tm["cells"] / dp_s / 1e9, 3) if dp_s > 0 else None,
-                         "peak_source": "measured live: pl_measure_int_peak, int32 add+max chains (%.3g lane-ops/s)"
-                                        % int32_peak,
+                         "peak_source": "measured live: pl_measure_int_peak (int16x2 %.3g, int32 %.3g lane-ops/s; two regions a "
+                                        "warp in int16x2, a profile whose values need 32 bits on k_hmm_dp)"
+                                        % (i16x2_peak, int32_peak),
                          "phase_ms_per_step": {"codons_ms": round(tm["prep_ms"] / args.steps, 3),
                                                "dp_ms": round(tm["dp_ms"] / args.steps, 3)},
                          "api": "pl_hmm_score_many_device: every profile's launch side by side on the engine's HMM "
@@ -1309,7 +1310,7 @@ def main_forward(args):
                     "api": "pl_rc_score_host (C ABI, host buffers), wall clock"},
             "gpu_launches": int(launches),
             "roofline": {"bound": "latency", "kernel": "k_rc_lanes", "achieved": None, "peak": None, "frac": None,
-                         "note": "one peptide per lane; the longest peptide's chains (three dependent logsums per "
+                         "note": "one peptide per lane of seven warps; the longest peptide's chains (three dependent logsums per "
                                  "Backward cell, each a restated glibc expf + log1pf) bound the step"},
             "cpu_baseline": {"value": round(c / secs / 1e9, 4), "unit": "GCUPS", "cores": threads, "kind": "reference",
                              "sample": f"{k} peptides, recheck.c rc_score via kt_for"}}
@@ -1841,12 +1842,12 @@ def main_seed(args):
                         "d2h_bytes_per_step": int(tot) * 8 + n * 8,
                         "api": "pl_seed_anchors_host (C ABI, host buffers), wall clock"},
                 "gpu_launches": int(launches),
-                "roofline": {"bound": "hbm", "kernel": "k_seed_emit + segmented sort",
+                "roofline": {"bound": "hbm", "kernel": "k_seed_anchors (emission and sort in shared memory)",
                              "achieved": round(int(tot) * SEED_BYTES_PER_ANCHOR / k_s / 1e9, 2), "unit": "GB/s",
                              "peak": hbm[0], "frac": round(int(tot) * SEED_BYTES_PER_ANCHOR / k_s / 1e9 / hbm[0], 4),
                              "peak_source": hbm[1], "traffic": None,
-                             "note": "algorithmic bytes: the anchor written and its block id read; the sort's passes "
-                                     "and the per-protein sketch are on top"},
+                             "note": "algorithmic bytes: the anchor written and its block id read; the per-protein sketch "
+                                     "is on top"},
                 "clocks": clk}
         if r is not None:
             line["cpu_baseline"] = {"value": round(r[0], 1), "unit": "anchors/s", "cores": threads, "kind": "reference",
@@ -1995,7 +1996,7 @@ def main_seed_hmm(args):
                         "d2h_bytes_per_step": int(tot) * 8 + n * 8,
                         "api": "pl_seed_anchors_hmm_host (C ABI, host buffers), wall clock"},
                 "gpu_launches": int(launches),
-                "roofline": {"bound": "hbm", "kernel": "k_seed_emit + segmented sorts",
+                "roofline": {"bound": "hbm", "kernel": "k_seed_anchors + the seeds' segmented sort",
                              "achieved": round(int(tot) * SEED_BYTES_PER_ANCHOR / k_s / 1e9, 2), "unit": "GB/s",
                              "peak": hbm[0], "frac": round(int(tot) * SEED_BYTES_PER_ANCHOR / k_s / 1e9 / hbm[0], 4),
                              "peak_source": hbm[1], "traffic": None,
@@ -2115,7 +2116,7 @@ def main_chain(args):
                       "h2d_bytes_per_step": int(a.nbytes + off.nbytes + n.nbytes),
                       "d2h_bytes_per_step": int(8 * n_a), "api": "pl_chain_host (device DP, host backtrack on "
                       f"{os.cpu_count()} threads), wall clock"},
-                     launches, {"bound": "int", "kernel": "k_chain_fill", "achieved": achieved, "peak": int32_peak,
+                     launches, {"bound": "int", "kernel": "k_chain_score + k_chain_fill", "achieved": achieved, "peak": int32_peak,
                                 "unit": "lane-ops/s", "frac": achieved / int32_peak if int32_peak else None,
                                 "traffic": None, "ops_per_pair": CHAIN_OPS_PER_PAIR, "pairs_per_step": pairs,
                                 "kernel_ms_per_step": round(k_s * 1e3, 3),

@@ -17,8 +17,8 @@
  *      budget, by longest-processing-time bin packing so every wave gets a mix
  *      of large and small jobs;
  *   3. in each wave, jobs whose cell count is large compared with the per-warp
- *      share are run by a whole CTA (a 256-lane wavefront), the rest by one
- *      warp each; both queues are sorted by decreasing size.
+ *      share have their strips run side by side by any warps of the GPU, the rest
+ *      run on one warp each; both queues are sorted by decreasing size.
  * There is no CPU fallback: failures are reported as errors.
  */
 #define _POSIX_C_SOURCE 200809L
@@ -458,7 +458,7 @@ static int32_t pl_form_pairs(pl_engine_t *e, const ns_opt_t *opt, int32_t n, int
 }
 
 /* FNV-1a of the launch sequence's shape: sizes, buffers, parameters and, per position of
- * the order array, the wave / launch group / rows / cooperative flag of its job */
+ * the order array, the wave / launch group / rows / shared flag of its job */
 static uint64_t pl_fnv(uint64_t h, const void *p, size_t n)
 {
 	const unsigned char *b = (const unsigned char*)p;
@@ -820,7 +820,7 @@ static double pl_now(void)
 }
 
 /* Autotuner of the batched global DP: runs the batch under every pair of (rows-per-lane
- * bin boundary, cooperative-job ratio) of a small grid, keeps the fastest for this
+ * bin boundary, shared-job ratio) of a small grid, keeps the fastest for this
  * engine and reports it.  The batch should look like the workload (the same length
  * distributions); its results are discarded. */
 PL_EXPORT int pl_engine_autotune(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n,
@@ -933,7 +933,7 @@ static int32_t ns_q_n;
  * send it is not waiting itself.  So the collection ends before its 2 ms once a caller waits for a
  * queued request and the queue holds as many requests as were ever outstanding at once around the
  * last batches: a lone caller, who sends one request and waits, is served at once (2.0 of the
- * 4.7 ms of a 350-residue protein against a 40 kb window were this wait), T callers get one batch
+ * 4.7 ms of a 500-residue protein against 20 kb were this wait), T callers get one batch
  * of T as soon as the last of them is back, and requests sent ahead of any wait are collected as
  * before. */
 #define NS_PEAKS 8

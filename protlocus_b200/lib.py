@@ -466,7 +466,7 @@ class Engine:
         return self.ps_run(self.ps_pack(cands), go, ge)
 
     def set_tuning(self, r4_rows: int = -1, coop_ratio: float = 0.0):
-        """Rows-per-lane bin boundary and cooperative-job ratio of the global DP (see plgpu.h)."""
+        """Rows-per-lane bin boundary and shared-job ratio of the global DP (see plgpu.h)."""
         self.lib.pl_engine_set_tuning(self.h, int(r4_rows), float(coop_ratio))
 
     def tuning(self):

@@ -1,9 +1,9 @@
 """Tuning of the batched global DP per shape class, kept in a JSON file.
 
 pl_engine_autotune picks, for one batch, the rows-per-lane bin boundary (jobs with
-at most r4_rows DP rows take 4 rows per lane, the rest 8) and the cooperative-job
-ratio (a job takes a whole CTA when it holds more than coop_ratio times a warp's
-share of its wave's cells).  The best point depends on the batch's shape: the
+at most r4_rows DP rows take 4 rows per lane, the rest 8) and the shared-job
+ratio (a job's strips run on any warps of the GPU when it holds more than coop_ratio
+times a third of a warp's share of its wave's cells).  The best point depends on the batch's shape: the
 protein lengths, the window lengths and the number of jobs.  A shape class puts
 batches of similar shape together (log2 buckets of the median protein length,
 of the median window length and of the job count), and the JSON file maps each
