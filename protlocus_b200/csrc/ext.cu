@@ -179,78 +179,6 @@ template <> struct KeyOf<true> {
 	static __device__ __forceinline__ int col(long long k) { return (int)(KW - 1 - (k & (KW - 1))); }
 };
 
-/* row-scan state of a request (warp-uniform); last_row: the last row the reference processes, the
- * x-drop row or else nl-1 */
-struct ExtScan { int best_sc, best_row, best_col, M, last_row; };
-
-/* the row scan of strip ks from its rows' (tmp, key) in shared memory; true when the request is done */
-template <typename K, typename KeyS>
-__device__ __forceinline__ bool ext_scan(ExtScan &S, const int ks, const int nl, const int pen_len, const int nstrip,
-		const int xdrop, const int32_t *rts, const KeyS *rkey, const float ie_coef, const int lane)
-{
-	typedef typename K::T KeyT;
-	constexpr int R = PLK_ROWS;
-	const int rb = 2 + ks * EXT_STRIP + lane * R;
-	int tl[R], lp[R], lmax = INT_MIN;
-#pragma unroll
-	for (int r = 0; r < R; ++r) {
-		const int i = rb + r;
-		tl[r] = i < nl ? rts[lane * R + r] - ext_penalty(i - pen_len, ie_coef) : INT_MIN;
-		lmax = max(lmax, tl[r]);
-		lp[r] = lmax;
-	}
-	int incl = lmax;
-#pragma unroll
-	for (int off = 1; off < 32; off <<= 1) {
-		const int v = __shfl_up_sync(FULL, incl, off);
-		if (lane >= off) incl = max(incl, v);
-	}
-	int excl = __shfl_up_sync(FULL, incl, 1);
-	if (lane == 0) excl = INT_MIN;
-	const int base = max(S.M, excl);
-	int br = R;  /* first row of this lane at which the x-drop test fires */
-#pragma unroll
-	for (int r = R - 1; r >= 0; --r)
-		if (tl[r] != INT_MIN && max(base, lp[r]) - tl[r] > xdrop) br = r;
-	const unsigned bm = __ballot_sync(FULL, br < R);
-	const int brk_lane = bm ? __ffs(bm) - 1 : 32;
-	const int brk_r = __shfl_sync(FULL, br, brk_lane & 31);
-	int cmax = INT_MIN;
-#pragma unroll
-	for (int r = 0; r < R; ++r) {
-		const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
-		if (consider) cmax = max(cmax, tl[r]);
-	}
-	int mx = cmax;
-#pragma unroll
-	for (int off = 16; off >= 1; off >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, off));
-	if (mx > S.M) { /* a later row improved the kept maximum: the first row reaching mx */
-		int fr = R;
-		long long fk = 0;
-#pragma unroll
-		for (int r = R - 1; r >= 0; --r) {
-			const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
-			if (consider && tl[r] == mx) fr = r, fk = rkey[lane * R + r];
-		}
-		const unsigned fm = __ballot_sync(FULL, fr < R);
-		const int fl = __ffs(fm) - 1;
-		fr = __shfl_sync(FULL, fr, fl);
-		fk = __shfl_sync(FULL, fk, fl);
-		S.best_row = 2 + ks * EXT_STRIP + fl * R + fr;
-		S.best_sc = K::hi((KeyT)fk);
-		S.best_col = K::col((KeyT)fk);
-		S.M = mx;
-	}
-	if (bm != 0) S.last_row = 2 + ks * EXT_STRIP + brk_lane * R + brk_r;
-	return bm != 0 || ks == nstrip - 1;
-}
-
-/* bias: what the scanned values lie above the scores */
-__device__ __forceinline__ void ext_answer(plk_ext_job_t *J, const ExtScan &S, const int bias)
-{
-	J->nt_len = S.best_row + 1, J->aa_len = S.best_col + 1, J->score = S.best_sc - bias, J->status = S.best_row >= 2 ? 0 : -1;
-}
-
 template <int MODE, bool PSSM, bool WIDE>
 __device__ __forceinline__ void ext_job(plk_ext_job_t *__restrict__ J, const uint8_t *__restrict__ prep,
 		const int8_t *__restrict__ pssm, int32_t *__restrict__ ring, ExtShared &sh, const plk_params_t &P,
@@ -282,8 +210,9 @@ __device__ __forceinline__ void ext_job(plk_ext_job_t *__restrict__ J, const uin
 #pragma unroll
 	for (int r = 0; r < R + 2; ++r) dnn[r] = acn[r] = 0;
 
-	int ks = 0, next_scan = glob ? INT_MAX : 31 + ncol - 1;
-	ExtScan Sc = {NEG, -1, 0, INT_MIN, nl - 1};
+	/* row-scan state (warp-uniform) */
+	int best_sc = NEG, best_row = -1, best_col = 0, M = INT_MIN, ks = 0, next_scan = glob ? INT_MAX : 31 + ncol - 1;
+	int last_row = nl - 1;  /* last row the reference processes: the x-drop row, else nl-1 */
 
 	for (int s = 0; s < total; ++s) {
 		int in[9];
@@ -388,7 +317,59 @@ __device__ __forceinline__ void ext_job(plk_ext_job_t *__restrict__ J, const uin
 		}
 		__syncwarp();
 		if (s == next_scan) { /* lane 31 finished strip ks: scan its rows in order */
-			const bool done = ext_scan<K>(Sc, ks, nl, pen_len, nstrip, xdrop, sh.rts[wib], sh.rkey[wib], P.ie_coef, lane);
+			const int rb = 2 + ks * EXT_STRIP + lane * R;
+			int tl[R], lp[R], lmax = INT_MIN;
+#pragma unroll
+			for (int r = 0; r < R; ++r) {
+				const int i = rb + r;
+				tl[r] = i < nl ? sh.rts[wib][lane * R + r] - ext_penalty(i - pen_len, P.ie_coef) : INT_MIN;
+				lmax = max(lmax, tl[r]);
+				lp[r] = lmax;
+			}
+			int incl = lmax;
+#pragma unroll
+			for (int off = 1; off < 32; off <<= 1) {
+				const int v = __shfl_up_sync(FULL, incl, off);
+				if (lane >= off) incl = max(incl, v);
+			}
+			int excl = __shfl_up_sync(FULL, incl, 1);
+			if (lane == 0) excl = INT_MIN;
+			const int base = max(M, excl);
+			int br = R;  /* first row of this lane at which the x-drop test fires */
+#pragma unroll
+			for (int r = R - 1; r >= 0; --r)
+				if (tl[r] != INT_MIN && max(base, lp[r]) - tl[r] > xdrop) br = r;
+			const unsigned bm = __ballot_sync(FULL, br < R);
+			const int brk_lane = bm ? __ffs(bm) - 1 : 32;
+			const int brk_r = __shfl_sync(FULL, br, brk_lane & 31);
+			int cmax = INT_MIN;
+#pragma unroll
+			for (int r = 0; r < R; ++r) {
+				const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
+				if (consider) cmax = max(cmax, tl[r]);
+			}
+			int mx = cmax;
+#pragma unroll
+			for (int off = 16; off >= 1; off >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, off));
+			if (mx > M) { /* a later row improved the kept maximum: the first row reaching mx */
+				int fr = R;
+				long long fk = 0;
+#pragma unroll
+				for (int r = R - 1; r >= 0; --r) {
+					const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
+					if (consider && tl[r] == mx) fr = r, fk = sh.rkey[wib][lane * R + r];
+				}
+				const unsigned fm = __ballot_sync(FULL, fr < R);
+				const int fl = __ffs(fm) - 1;
+				fr = __shfl_sync(FULL, fr, fl);
+				fk = __shfl_sync(FULL, fk, fl);
+				best_row = 2 + ks * EXT_STRIP + fl * R + fr;
+				best_sc = K::hi((KeyT)fk);
+				best_col = K::col((KeyT)fk);
+				M = mx;
+			}
+			if (bm != 0) last_row = 2 + ks * EXT_STRIP + brk_lane * R + brk_r;
+			const bool done = bm != 0 || ks == nstrip - 1;
 			++ks, next_scan += Pc;
 			__syncwarp();
 			if (done) break;
@@ -406,9 +387,9 @@ __device__ __forceinline__ void ext_job(plk_ext_job_t *__restrict__ J, const uin
 	__syncwarp();
 	if (lane == 0) {
 		if (glob) J->nt_len = nl, J->aa_len = al, J->status = 0;
-		else ext_answer(J, Sc, 0);
+		else J->nt_len = best_row + 1, J->aa_len = best_col + 1, J->score = best_sc, J->status = best_row >= 2 ? 0 : -1;
 		/* algorithmic cells: rows 2..last_row (the rows the reference's loop visits) x al */
-		atomicAdd(cells_acc, (unsigned long long)((int64_t)(Sc.last_row - 1) * al));
+		atomicAdd(cells_acc, (unsigned long long)((int64_t)(last_row - 1) * al));
 	}
 	__syncwarp();
 }
@@ -445,13 +426,86 @@ k_ext_dp(plk_ext_job_t *__restrict__ jobs, const int32_t *__restrict__ order, in
  * column count in the protein's place.  The two differ in everything but the wave: each half has
  * its own residues (two table rows, one already shifted up), segment length, last column and last
  * row; columns and strips past a half's own are computed and not looked at.  What bounds
- * the single kernel is its instructions (57% of the issue slots at the 12 warps per SM that its 164
+ * the single kernel is its instructions (57% of the issue slots at the 12 warps per SM that its 167
  * registers allow, the rest dependences; 16 warps spilled: 36.8 -> 38.5 ms).  65,536 requests
  * of 64-256 residues: 37.3 -> 25.9 ms a batch; 16,384 of 300-600: 25.6 -> 18.0.
  * The geometry and the scan's state stay in shared memory: with them in registers the kernel spilled
  * (28.3 ms).  The row maximum over the padding columns (end_bonus >= 0: over those only) goes to shared memory
  * in the few steps that have any, which leaves its registers to the second key.
  */
+/* row-scan state of a request (warp-uniform); last_row: the last row the reference processes, the
+ * x-drop row or else nl-1 */
+struct ExtScan { int best_sc, best_row, best_col, M, last_row; };
+
+/* the row scan of strip ks from its rows' (tmp, key) in shared memory, as in ext_job, for a pair's
+ * halves; true when the request is done.  (ext_job keeps its own: through this function batches
+ * of a few thousand requests took 1.3% longer.) */
+__device__ __forceinline__ bool ext_scan(ExtScan &S, const int ks, const int nl, const int pen_len, const int nstrip,
+		const int xdrop, const int32_t *rts, const int32_t *rkey, const float ie_coef, const int lane)
+{
+	typedef KeyOf<false> K;
+	constexpr int R = PLK_ROWS;
+	const int rb = 2 + ks * EXT_STRIP + lane * R;
+	int tl[R], lp[R], lmax = INT_MIN;
+#pragma unroll
+	for (int r = 0; r < R; ++r) {
+		const int i = rb + r;
+		tl[r] = i < nl ? rts[lane * R + r] - ext_penalty(i - pen_len, ie_coef) : INT_MIN;
+		lmax = max(lmax, tl[r]);
+		lp[r] = lmax;
+	}
+	int incl = lmax;
+#pragma unroll
+	for (int off = 1; off < 32; off <<= 1) {
+		const int v = __shfl_up_sync(FULL, incl, off);
+		if (lane >= off) incl = max(incl, v);
+	}
+	int excl = __shfl_up_sync(FULL, incl, 1);
+	if (lane == 0) excl = INT_MIN;
+	const int base = max(S.M, excl);
+	int br = R;  /* first row of this lane at which the x-drop test fires */
+#pragma unroll
+	for (int r = R - 1; r >= 0; --r)
+		if (tl[r] != INT_MIN && max(base, lp[r]) - tl[r] > xdrop) br = r;
+	const unsigned bm = __ballot_sync(FULL, br < R);
+	const int brk_lane = bm ? __ffs(bm) - 1 : 32;
+	const int brk_r = __shfl_sync(FULL, br, brk_lane & 31);
+	int cmax = INT_MIN;
+#pragma unroll
+	for (int r = 0; r < R; ++r) {
+		const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
+		if (consider) cmax = max(cmax, tl[r]);
+	}
+	int mx = cmax;
+#pragma unroll
+	for (int off = 16; off >= 1; off >>= 1) mx = max(mx, __shfl_xor_sync(FULL, mx, off));
+	if (mx > S.M) { /* a later row improved the kept maximum: the first row reaching mx */
+		int fr = R;
+		int fk = 0;
+#pragma unroll
+		for (int r = R - 1; r >= 0; --r) {
+			const bool consider = tl[r] != INT_MIN && (lane < brk_lane || (lane == brk_lane && r <= brk_r));
+			if (consider && tl[r] == mx) fr = r, fk = rkey[lane * R + r];
+		}
+		const unsigned fm = __ballot_sync(FULL, fr < R);
+		const int fl = __ffs(fm) - 1;
+		fr = __shfl_sync(FULL, fr, fl);
+		fk = __shfl_sync(FULL, fk, fl);
+		S.best_row = 2 + ks * EXT_STRIP + fl * R + fr;
+		S.best_sc = K::hi(fk);
+		S.best_col = K::col(fk);
+		S.M = mx;
+	}
+	if (bm != 0) S.last_row = 2 + ks * EXT_STRIP + brk_lane * R + brk_r;
+	return bm != 0 || ks == nstrip - 1;
+}
+
+/* bias: what the scanned values lie above the scores */
+__device__ __forceinline__ void ext_answer(plk_ext_job_t *J, const ExtScan &S, const int bias)
+{
+	J->nt_len = S.best_row + 1, J->aa_len = S.best_col + 1, J->score = S.best_sc - bias, J->status = S.best_row >= 2 ? 0 : -1;
+}
+
 /* what one half's wave needs of its request at strip starts and scans */
 struct ExtHalf {
 	const uint8_t *nas;
@@ -530,7 +584,7 @@ __device__ __forceinline__ bool x_scan(ExtHalf &H, const int ks, const int32_t *
 {
 	if (H.done) return true;
 	ExtScan S = H.S;
-	const bool done = ext_scan<KeyOf<false>>(S, ks, H.nl, 3 * H.al, H.nstrip, P.xdrop, rts, rkey, P.ie_coef, lane);
+	const bool done = ext_scan(S, ks, H.nl, 3 * H.al, H.nstrip, P.xdrop, rts, rkey, P.ie_coef, lane);
 	__syncwarp();
 	if (lane == 0) H.S = S, H.done = done;
 	__syncwarp();

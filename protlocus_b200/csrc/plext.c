@@ -170,7 +170,7 @@ static int pl_ext_run(pl_engine_t *e, const ns_opt_t *opt, const pl_ext_job_t *j
 		if (can_pair && J->mode == 0 && J->variant == 0 && kind != 2 && J->al >= PL_XPAIR_MIN_AL && J->ncol <= al_cap) J->pad = 1, ++n_el;
 		++n_dp;
 	}
-	if (n_el > 1) {
+	if (n_el > 1 && (e->pairing == 2 || n_el / 2 >= PL_XPAIR_FILL * e->n_sm * plk_ext_warps_per_cta())) { /* else too few for any occupancy */
 		pair_ctas = plk_ext_ctas_per_sm(3, 0);
 		if (pair_ctas < 1) { pl_set_error("extension DP kernel does not fit on an SM"); goto fail; }
 		pair_ctas *= e->n_sm;
