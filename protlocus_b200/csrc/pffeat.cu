@@ -15,7 +15,8 @@
  *     the step) before by shuffles, so the scan has no barrier.  The lookup tables sit
  *     in shared memory (as kernel constants their divergent reads serialised), and a
  *     65,536-bit map of the protein's 5-mers, 0.6 % full for a 420-residue protein,
- *     sends few warps to the hash table;
+ *     sends few warps to the hash table.  The first 1024 anchors by position are kept:
+ *     when there are more, the warps go over their parts again in order (below);
  *  3. the anchors are sorted by position and chained: the longest chain increasing in
  *     both coordinates whose nucleotide gap is not shorter than 3x the residue gap
  *     minus 60 (frameshift slack).  A lane holds one anchor of a block of 32: the
@@ -62,12 +63,60 @@ struct FeatSmem {
 	uint32_t map[2048];            /* word hmul(code) >> 21, bit code & 31 of every 5-mer in the table */
 	uint8_t nt4[256], aa20[256], codon[64];
 	int32_t n_anchor, tot_p, tot_w;
+	int32_t part_n[THREADS / 32];  /* anchors of each warp's part of the window */
 	int32_t chain[8];
 };
 
 __device__ __forceinline__ uint32_t hmul(uint32_t code) { return code * 2654435761u; }
 __device__ __forceinline__ uint32_t h5(uint32_t h) { return h >> 20; }                                /* slot: 12 bits */
 __device__ __forceinline__ uint32_t h3(uint32_t code) { return ((code * 40503u) >> 8) & 255u; }
+
+/* first protein position of a 5-mer, or -1 */
+__device__ __forceinline__ int32_t lookup5(const FeatSmem &S, const uint32_t code)
+{
+	uint32_t sl = h5(hmul(code));
+	for (int t = 0; t < HSLOTS; ++t, sl = (sl + 1) & (HSLOTS - 1)) {
+		const int32_t key = S.hkey[sl];
+		if (key == 0) break;
+		if (key == (int32_t)code + 1) return S.hpos[sl];
+	}
+	return -1;
+}
+
+/* More anchors than places: the window's first MAXA of them, whatever order the scan met them in
+ * (the warps raced for the places, and a candidate's features could differ from run to run).  Warp w
+ * goes over its positions [lo, hi) again, a position a lane and a step of 32 at a time, and writes its
+ * anchors in order from base, the number that the warps before it hold, until the places are full.
+ * The residues at p - 3 .. p - 12 come from the lanes of this step and the one before; the first
+ * step, before lo, is there for them alone. */
+__device__ __noinline__ void first_anchors(FeatSmem &S, const uint8_t *__restrict__ nt, const int32_t nl, const int64_t lo,
+		const int64_t hi, int base, const int lane)
+{
+	uint32_t prev = BAD;
+	for (int64_t b = lo - 32; b < hi && base < MAXA; b += 32) {
+		const int64_t p = b + lane;
+		uint32_t r = BAD;
+		if (p >= 2 && p < nl) {
+			const uint32_t c0 = S.nt4[nt[p - 2]], c1 = S.nt4[nt[p - 1]], c2 = S.nt4[nt[p]];
+			if (!((c0 | c1 | c2) & 0x80)) r = S.codon[c0 << 4 | c1 << 2 | c2];
+		}
+		uint32_t code = 0;
+		bool ok = p >= lo && p < hi;
+#pragma unroll
+		for (int k = 4; k >= 0; --k) {
+			const uint32_t x = __shfl_sync(0xffffffffu, r, (lane - 3 * k) & 31), y = __shfl_sync(0xffffffffu, prev, (lane - 3 * k) & 31),
+					v = lane >= 3 * k ? x : y;
+			ok = ok && v != BAD;
+			code = code * 20u + v;
+		}
+		const int32_t rp = ok ? lookup5(S, code) : -1;
+		const uint32_t hit = __ballot_sync(0xffffffffu, rp >= 0);
+		const int at = base + __popc(hit & ((1u << lane) - 1));
+		if (rp >= 0 && at < MAXA) S.akey[at] = (p << 20) | (int64_t)rp;
+		base += __popc(hit);
+		prev = r;
+	}
+}
 
 /* bit 7 of a word's four bytes, in order */
 __device__ __forceinline__ uint32_t high_bits(const uint32_t w) { return (((w >> 7) & 0x01010101u) * 0x10204080u) >> 28; }
@@ -130,12 +179,12 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 	/* 2. window scan, in groups of 16 positions P = p + a0 that start at 16-byte boundaries of the
 	 * bases.  Warp w takes groups [gb, ge); its first step starts a group early, uncounted, for
 	 * the codes and residues that reach into the part */
-	int cntw = 0;
+	int cntw = 0, nh = 0;
+	const int a0 = (int)((uintptr_t)nt & 15);
+	const int ng = (int)(((int64_t)nl + a0 + 15) / 16), gb = (int)((int64_t)ng * warp / (THREADS / 32)),
+			ge = (int)((int64_t)ng * (warp + 1) / (THREADS / 32));
 	{
-		const int a0 = (int)((uintptr_t)nt & 15);
 		const uint4 *ntv = reinterpret_cast<const uint4 *>(nt - a0);
-		const int ng = (int)(((int64_t)nl + a0 + 15) / 16), gb = (int)((int64_t)ng * warp / (THREADS / 32)),
-				ge = (int)((int64_t)ng * (warp + 1) / (THREADS / 32));
 		/* of the position group before lane 0's: 2 codes with their marks, 12 residues */
 		uint32_t pc = 0x30000000u, p1 = ~0u, p2 = ~0u, p3 = ~0u;
 		for (int g0 = gb - 1; gb < ge && g0 < ge; g0 += 32) {
@@ -215,16 +264,12 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 					const uint32_t w = at < 4 ? b1 : at < 8 ? b2 : at < 12 ? b3 : at < 16 ? o[0] : at < 20 ? o[1] : at < 24 ? o[2] : o[3];
 					code = code * 20u + (w >> (8 * (at & 3)) & 255);
 				}
-				uint32_t sl = h5(hmul(code));
-				for (int t = 0; t < HSLOTS; ++t, sl = (sl + 1) & (HSLOTS - 1)) {
-					const int32_t key = S.hkey[sl];
-					if (key == 0) break;
-					if (key == (int32_t)code + 1) {
-						const int at = atomicAdd(&S.n_anchor, 1);
-						/* both coordinates are k-mer ends */
-						if (at < MAXA) S.akey[at] = ((p0 + i - 12) << 20) | (int64_t)S.hpos[sl];
-						break;
-					}
+				const int32_t rp = lookup5(S, code);
+				if (rp >= 0) {
+					const int at = atomicAdd(&S.n_anchor, 1);
+					++nh;
+					/* both coordinates are k-mer ends */
+					if (at < MAXA) S.akey[at] = ((p0 + i - 12) << 20) | (int64_t)rp;
 				}
 			}
 		}
@@ -234,6 +279,15 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 
 	/* 3. sort the kept anchors by (position, protein position) -- all keys differ -- and chain them */
 	const int na_all = S.n_anchor, na = na_all < MAXA ? na_all : MAXA;
+	if (na_all > MAXA) {
+		nh = __reduce_add_sync(0xffffffffu, nh);
+		if (lane == 0) S.part_n[warp] = nh;
+		__syncthreads();
+		int base = 0;
+		for (int w = 0; w < warp; ++w) base += S.part_n[w];
+		first_anchors(S, nt, nl, 16 * (int64_t)gb - a0, 16 * (int64_t)ge - a0, base, lane);
+		__syncthreads();
+	}
 	if (na <= THREADS) { /* an anchor per thread: its rank by counting */
 		int rank = 0;
 		const int64_t key = tid < na ? S.akey[tid] : 0;
