@@ -484,17 +484,21 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
  *
  * Hand-off.  Lane 31 writes each column's state as a 48-byte entry of three 16-byte words,
  * each three values and the tag k + 1, into the job's ring (two strips deep, zeroed before
- * the launch: strip k writes half k & 1).  Lane 0 of the strip below copies the entry with
- * cp.async one column ahead (L2 is the point of coherence for both) and takes it when all
- * three words carry its tag, else fetches again; a 16-byte aligned access is one transaction,
- * so a word's values are those of its tag.  Strip k + 2 reaches column c only after strip
- * k + 1 has taken the entry of column c from strip k, so no entry is overwritten before it
- * is read and the halves need no other guard.
+ * the launch: strip k writes half k & 1).  The words are written and read by relaxed .b128
+ * accesses of gpu scope, which are single-copy atomic, so a word's values are those of its
+ * tag (vector stores and cp.async, tried first, promise that for no more than their parts).
+ * Lanes 0-2 of the strip below load a word each one column ahead, look again while one carries
+ * another tag, and hand them to lane 0 through shared memory.  Strip k + 2 reaches column c only
+ * after strip k + 1 has taken the entry of column c from strip k, and what it writes there depends
+ * on that entry's values, so no entry is overwritten before it is read and the halves need no
+ * other guard.  The load sits at the end of a step: ahead of the step's own loads these waited
+ * for it too (2.9 ms a request).
  *
- * Measured (DP launch before -> after): one 500 aa x 20 kb request 5.9 -> 2.3 ms, 96 short jobs
- * 1.82 -> 0.44 ms, 509 loci of 1-50 kb 52.9 -> 18.7 ms; the batch of 8192 strands 291 -> 190 ms
+ * Measured (DP launch before -> after): one 500 aa x 20 kb request 5.9 -> 2.5 ms, 96 short jobs
+ * 1.82 -> 0.44 ms, 509 loci of 1-50 kb 52.9 -> 17.9 ms; the batch of 8192 strands 291 -> 197 ms
  * a call (its waves end without a tail of long jobs, and no block barrier holds eight warps
- * in step).
+ * in step).  With cp.async for the words: the request 2.3 ms, 64 of them 5.9 against 5.7, the 509
+ * loci's call 21.9 against 20.7, the strands' call 192 against 197.
  *
  * Progress.  Warps claim units by an atomic ticket in an order that has every strip after the
  * one above it (k_strip_order), and a claimed unit runs to its end, so the strip a warp waits
@@ -505,46 +509,53 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
  */
 #define STRIP_WAIT 20000000000LL
 
-__device__ __forceinline__ void ring_fetch(int32_t *pre, const int32_t *e)
+/* one 16-byte word of an entry, as one access */
+__device__ __forceinline__ int4 ring_load(const int32_t *e)
 {
-	cp_async16(pre, e), cp_async16(pre + 4, e + 4), cp_async16(pre + 8, e + 8);
+	uint64_t a, b;
+	asm volatile("{\n\t.reg .b128 v;\n\tld.relaxed.gpu.global.b128 v, [%2];\n\tmov.b128 {%0, %1}, v;\n\t}" : "=l"(a), "=l"(b) : "l"(e));
+	return make_int4((int)a, (int)(a >> 32), (int)b, (int)(b >> 32));
 }
 
-/* the entry at e, already fetched into pre, once it carries tag; false when the wait ran out */
-__device__ __forceinline__ bool ring_take(int32_t *pre, const int32_t *e, const int tag, int32_t *ctl, int (&in)[9])
+__device__ __forceinline__ void ring_store(int32_t *e, const int x, const int y, const int z, const int tag)
 {
-	bool ok = true;
-	cp_async_wait_all();
-	int4 v0 = *(const int4*)pre, v1 = *(const int4*)(pre + 4), v2 = *(const int4*)(pre + 8);
-	if (v0.w != tag || v1.w != tag || v2.w != tag) {
-		const long long t0 = clock64();
-		do {
-			if (*(volatile int32_t*)(ctl + 2) != 0) { ok = false; break; }
-			if (clock64() - t0 > STRIP_WAIT) { atomicExch(ctl + 2, 1); ok = false; break; }
-			ring_fetch(pre, e);
-			cp_async_wait_all();
-			v0 = *(const int4*)pre, v1 = *(const int4*)(pre + 4), v2 = *(const int4*)(pre + 8);
-		} while (v0.w != tag || v1.w != tag || v2.w != tag);
-	}
+	const uint64_t a = (uint32_t)x | (uint64_t)(uint32_t)y << 32, b = (uint32_t)z | (uint64_t)(uint32_t)tag << 32;
+	asm volatile("{\n\t.reg .b128 v;\n\tmov.b128 v, {%1, %2};\n\tst.relaxed.gpu.global.b128 [%0], v;\n\t}" :: "l"(e), "l"(a), "l"(b));
+}
+
+/* the whole warp: the words that lanes with fetch set loaded (w, from e), once all carry tag; false when the
+ * wait ran out.  The word and the abort flag are asked for together, a round trip a look */
+__device__ __forceinline__ bool ring_settle(const int32_t *e, int4 &w, const bool fetch, const int tag, int32_t *ctl)
+{
+	if (!__any_sync(FULL, fetch && w.w != tag)) return true;
+	const long long t0 = clock64();
+	int stop;
+	do {
+		stop = *(volatile int32_t*)(ctl + 2);
+		if (fetch) w = ring_load(e);
+		if (stop == 0 && clock64() - t0 > STRIP_WAIT) stop = 1, atomicExch(ctl + 2, 1);
+		stop = __any_sync(FULL, stop != 0);
+	} while (__any_sync(FULL, fetch && w.w != tag) && !stop);
+	return !__any_sync(FULL, fetch && w.w != tag);
+}
+
+/* lane 0's entry of this column */
+__device__ __forceinline__ void ring_read(const int32_t *pre, int (&in)[9])
+{
+	const int4 v0 = *(const int4*)pre, v1 = *(const int4*)(pre + 4), v2 = *(const int4*)(pre + 8);
 	in[0] = v0.x, in[1] = v0.y, in[2] = v0.z, in[3] = v1.x, in[4] = v1.y, in[5] = v1.z;
 	in[6] = v2.x, in[7] = v2.y, in[8] = v2.z;
-	return ok;
 }
 
 __device__ __forceinline__ void ring_put(int32_t *e, const int tag, const int (&o)[9])
 {
-	__stcg((int4*)e, make_int4(o[0], o[1], o[2], tag));
-	__stcg((int4*)(e + 4), make_int4(o[3], o[4], o[5], tag));
-	__stcg((int4*)(e + 8), make_int4(o[6], o[7], o[8], tag));
+	ring_store(e, o[0], o[1], o[2], tag), ring_store(e + 4, o[3], o[4], o[5], tag), ring_store(e + 8, o[6], o[7], o[8], tag);
 }
 
-/* lane 0's first entry: the -inf row above strip 0 (both buffers, tag 0), else column 0 of strip k-1 */
-__device__ __forceinline__ void strip_begin(int32_t (*pre)[PLK_RING_INTS], const int32_t *rin, const int k, const int neg,
-		const int lane)
+/* the -inf row above strip 0, in both buffers for good */
+__device__ __forceinline__ void strip_top(int32_t (*pre)[PLK_RING_INTS], const int neg, const int lane)
 {
-	if (lane == 0 && k > 0) ring_fetch(pre[0], rin);
-	if (k == 0 && lane < 2 * PLK_RING_INTS) pre[0][lane] = (lane & 3) == 3 ? 0 : neg;
-	__syncwarp();
+	if (lane < 2 * PLK_RING_INTS) pre[0][lane] = neg;
 }
 
 template <int MODE, int R>
@@ -567,7 +578,10 @@ __device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k,
 	const int GOE = P.s16[8], GE16 = P.s16[1];
 	const int i0 = 2 + k * HS + lane * R;
 
-	strip_begin(pre, rin, k, NEG, lane);
+	const bool taker = k > 0 && lane < 3;  /* lanes 0-2 fetch a word of an entry each */
+	int4 w = make_int4(0, 0, 0, 0);
+	if (taker) w = ring_load(rin + 4 * lane);
+	if (k == 0) strip_top(pre, NEG, lane);
 	int ip[R], lh[R], ic[R], hm[R], code[R], gi[R], dn[R + 2], ac[R + 2], o[9];
 	int ah1 = NEG, ah2 = NEG, ah3 = NEG;
 #pragma unroll
@@ -586,16 +600,17 @@ __device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k,
 		ac[r] = MODE == 0 ? -16 * av : av;
 	}
 	const bool rows_in = i0 < nl;
+	if (!ring_settle(rin + 4 * lane, w, taker, k, ctl)) J->status = -3;
+	if (taker) *(int4*)(pre[0] + 4 * lane) = w;
+	if (taker && 1 < al) w = ring_load(rin + PLK_RING_INTS + 4 * lane);
+	__syncwarp();
 	int cs = 0, dcol = 0;  /* dcol: s modulo al, the trace diagonal of every lane in step s */
 	for (int s = 0; s < al + 31; ++s) {
 		const int c = s - lane;
 		int in[9];
 #pragma unroll
 		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
-		if (lane == 0 && s < al) {
-			if (!ring_take(pre[s & 1], rin + (int64_t)s * PLK_RING_INTS, k, ctl, in)) J->status = -3;
-			if (k > 0 && s + 1 < al) ring_fetch(pre[(s + 1) & 1], rin + (int64_t)(s + 1) * PLK_RING_INTS);
-		}
+		if (lane == 0 && s < al) ring_read(pre[s & 1], in);
 		const bool live = (unsigned)c < (unsigned)al && rows_in;
 		const bool any_seg = __any_sync(FULL, live && cs == 0);
 		if (live) {
@@ -626,11 +641,13 @@ __device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k,
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
+		if (!ring_settle(rin + (int64_t)(s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl)) J->status = -3;
+		if (taker && s + 1 < al) *(int4*)(pre[(s + 1) & 1] + 4 * lane) = w;
+		if (taker && s + 2 < al) w = ring_load(rin + (int64_t)(s + 2) * PLK_RING_INTS + 4 * lane);
 		__syncwarp();
 		if (c >= 0 && ++cs == slen) cs = 0;
 		if (++dcol == al) dcol = 0;
 	}
-	cp_async_wait_all();
 	{ /* H(nl-1, al-1): in the last strip, the lane holding row nl-1 keeps the last column in hm */
 		const int rl = nl - 1 - i0;
 		if (rl >= 0 && rl < R) {
@@ -1025,7 +1042,10 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 	const unsigned r2h = P.pair_b * 0x10001u, r2f = (unsigned)(P.pair_b - P.fs) * 0x10001u;
 	const int i0 = 2 + k * HS + lane * R;
 
-	strip_begin(pre, rout + (int64_t)rdif * PLK_RING_INTS, k, (int)NEG, lane);
+	const bool taker = k > 0 && lane < 3;
+	int4 w = make_int4(0, 0, 0, 0);
+	if (taker) w = ring_load(rout + (int64_t)rdif * PLK_RING_INTS + 4 * lane);
+	if (k == 0) strip_top(pre, (int)NEG, lane);
 	unsigned ip[R], lh[R], ic[R], hm[R], gi[R], dn[R + 2], ac[R + 2], o[9];
 	int cp[R];
 	unsigned ah1 = NEG, ah2 = NEG, ah3 = NEG;
@@ -1050,6 +1070,11 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 		}
 	}
 	const bool rows_in = i0 < nl;
+	if (!ring_settle(rout + (int64_t)rdif * PLK_RING_INTS + 4 * lane, w, taker, k, ctl))
+		jobs[ja].status = jobs[jobs[ja].pair].status = -3;
+	if (taker) *(int4*)(pre[0] + 4 * lane) = w;
+	if (taker && 1 < al) w = ring_load(rout + (int64_t)(rdif + 1) * PLK_RING_INTS + 4 * lane);
+	__syncwarp();
 	int cs = 0, dcol = 0;  /* dcol: s modulo al, the trace diagonal of every lane in step s */
 	for (int s = 0; s < al + 31; ++s) {
 		const int c = s - lane;
@@ -1058,11 +1083,9 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 		for (int q = 0; q < 9; ++q) in[q] = __shfl_up_sync(FULL, o[q], 1);
 		if (lane == 0 && s < al) {
 			int v[9];
-			if (!ring_take(pre[s & 1], rout + (int64_t)(rdif + s) * PLK_RING_INTS, k, ctl, v))
-				jobs[ja].status = jobs[jobs[ja].pair].status = -3;
+			ring_read(pre[s & 1], v);
 #pragma unroll
 			for (int q = 0; q < 9; ++q) in[q] = (unsigned)v[q];
-			if (k > 0 && s + 1 < al) ring_fetch(pre[(s + 1) & 1], rout + (int64_t)(rdif + s + 1) * PLK_RING_INTS);
 		}
 		const bool live = (unsigned)c < (unsigned)al && rows_in;
 		const bool any_seg = __any_sync(FULL, live && cs == 0);
@@ -1093,11 +1116,14 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
+		if (!ring_settle(rout + (int64_t)(rdif + s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl))
+			jobs[ja].status = jobs[jobs[ja].pair].status = -3;
+		if (taker && s + 1 < al) *(int4*)(pre[(s + 1) & 1] + 4 * lane) = w;
+		if (taker && s + 2 < al) w = ring_load(rout + (int64_t)(rdif + s + 2) * PLK_RING_INTS + 4 * lane);
 		__syncwarp();
 		if (c >= 0 && ++cs == slen) cs = 0;
 		if (++dcol == al) dcol = 0;
 	}
-	cp_async_wait_all();
 	{ /* H(nl-1, al-1) of both jobs, unbiased */
 		const int rl = nl - 1 - i0;
 		if (rl >= 0 && rl < R) {
