@@ -151,7 +151,8 @@ typedef struct {
 	int32_t n_cigar;
 	int64_t cigar_off;
 	int32_t mode;      /* 16 or 32: the DP width the job ran at (ns_global_gs_auto's rule) */
-	int32_t status;    /* 0 = ok; <0 = error (see pl_last_error()) */
+	int32_t status;    /* 0 = ok; -2 = its CIGAR does not fit cigar_cap; -3 = a wait between its
+	                    * strips ran out: score INT32_MIN, no CIGAR, and the call fails */
 } pl_splice_result_t;
 
 typedef struct pl_engine_s pl_engine_t;
@@ -178,7 +179,9 @@ int pl_splice_batch_host(pl_engine_t *e, const ns_opt_t *opt,
  * engine's second stream after the preparation and joins it back before the
  * compaction) and the call returns once it has completed.
  * *total_cigar (optional) receives the number of CIGAR words produced; jobs
- * beyond cigar_cap get status -2.  Returns 1 on success. */
+ * beyond cigar_cap get status -2.  Returns 1 on success; 0 with the reason in
+ * pl_last_error() otherwise, when a job has status -3 among others (the results
+ * of the other jobs are then valid). */
 int pl_splice_batch_device(pl_engine_t *e, const ns_opt_t *opt,
 		const pl_splice_job_t *jobs, int32_t n_jobs,
 		const uint8_t *nt, const uint8_t *aa, const uint8_t *ss,
@@ -219,6 +222,12 @@ int pl_engine_autotune(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_
  * (after+1)-th pass from now (after < 0 disarms).  No device work is involved:
  * the failure is the error path the real failure takes.  Returns 1 when armed. */
 int pl_debug_fault(int32_t site, int32_t after);
+/* Test hook (no counterpart in the reference): the clock-cycle limit of the waits between
+ * the strips of a shared job of the global DP, for every later call of the process; 0
+ * restores the default (some ten seconds).  Where a wait runs out the call fails with the
+ * reason and without faulting the device: no strip waits any more and the launch ends, the
+ * jobs concerned get status -3, and the engine stays usable.  Returns 1. */
+int pl_debug_strip_wait(int64_t cycles);
 
 /* Number of trace waves, jobs with shared strips and DP launches of the last batch. */
 void pl_engine_last_plan(const pl_engine_t *e, int32_t *n_waves, int32_t *n_coop, int32_t *n_dp_launches);

@@ -493,6 +493,15 @@ static uint64_t pl_plan_key(const pl_engine_t *e, int32_t n, int32_t n_waves, in
 }
 
 /* Runs the whole batch on `st`.  Inputs (nt/aa/ss) and outputs (res/cig) are device pointers. */
+/* the limit of the waits between the strips of a job (pl_debug_strip_wait), 0: the default */
+static int64_t g_strip_wait = 0;
+
+PL_EXPORT int pl_debug_strip_wait(int64_t cycles)
+{
+	__atomic_store_n(&g_strip_wait, cycles > 0 ? cycles : 0, __ATOMIC_RELAXED);
+	return 1;
+}
+
 static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n,
 		const uint8_t *nt, const uint8_t *aa, const uint8_t *ss, pl_splice_result_t *res_dev,
 		uint32_t *cig_dev, int64_t cig_cap, int64_t *total_out, cudaStream_t st)
@@ -504,13 +513,15 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	const int64_t units_off = ((int64_t)n * 4 + 15) / 16 * 16;  /* the strip queues sit behind the order array */
 	plk_dp_group_t *grp = 0;
 	int32_t *wave_grp = 0, *bucket = 0;
-	int64_t *wave_bytes = 0, *wave_cells = 0, total_words = 0;
+	int64_t *wave_bytes = 0, *wave_cells = 0, total[2] = {0, 0};  /* CIGAR words; a job failed */
 	int ok = 0, capturing = 0;
 	uint64_t g_launch0 = 0, g_key = 0;
 
 	e->last_waves = e->last_coop = e->last_dp_launches = e->last_pairs = 0;
 	if (n <= 0) { if (total_out) *total_out = 0; return 1; }
 	if (!pl_params(opt, &P, 0)) return 0;
+	P.strip_wait = __atomic_load_n(&g_strip_wait, __ATOMIC_RELAXED);
+	if (P.strip_wait == 0) P.strip_wait = PLK_STRIP_WAIT;
 	if (!pl_grow_host(e, n)) return 0;
 	max_sub = pl_max_sub(opt);
 	slots = (int64_t)e->n_sm * e->ctas_per_sm[0][0] * PLK_WARPS_PER_CTA;
@@ -748,9 +759,10 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		CK(cudaGraphLaunch(e->g_exec, st));
 	}
 launched:
-	CK(cudaMemcpyAsync(&total_words, e->total.p, sizeof(int64_t), cudaMemcpyDeviceToHost, st));
+	CK(cudaMemcpyAsync(total, e->total.p, sizeof(total), cudaMemcpyDeviceToHost, st));
 	CK(cudaStreamSynchronize(st));
-	if (total_out) *total_out = total_words;
+	if (total[1]) { pl_set_error("a wait between the strips of an alignment ran out (results with status -3)"); goto fail; }
+	if (total_out) *total_out = total[0];
 	e->last_waves = n_waves, e->last_coop = wave_n_coop;
 	if (e->timing) {
 		/* event pairs: prep, every DP launch and every traceback (on the stream of their

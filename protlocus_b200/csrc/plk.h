@@ -40,7 +40,9 @@ typedef struct {
 	/* the paired DP's trace-bit gather runs as multiply-adds on the FMA pipe, its
 	 * multipliers read as kernel constants: 2^0 .. 2^15, and -(2^10 - 1), -2^10 .. -2^15 */
 	int32_t pair_pw[16], pair_nw[7];
+	int64_t strip_wait;         /* clock cycles that a strip of a shared job waits for the one above it */
 } plk_params_t;
+#define PLK_STRIP_WAIT 20000000000LL  /* some ten seconds */
 
 /* fills plk_params_t.s16 from go/ge/io/fs (every host path that builds parameters calls it) */
 static inline void plk_fill_scaled(plk_params_t *p)

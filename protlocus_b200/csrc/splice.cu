@@ -503,11 +503,10 @@ __device__ __forceinline__ void dp_job(plk_job_t *__restrict__ J, const uint8_t 
  * Progress.  Warps claim units by an atomic ticket in an order that has every strip after the
  * one above it (k_strip_order), and a claimed unit runs to its end, so the strip a warp waits
  * for is always held by a running warp: no co-residency of the grid is needed.  A wait is
- * bounded all the same (STRIP_WAIT cycles, some ten seconds): on expiry the launch's abort
- * word ctl[2] is set, every waiting strip goes on with what it has, and the jobs concerned
- * get status -3.
+ * bounded all the same (P.strip_wait cycles): on expiry the launch's abort word ctl[2] is set,
+ * no strip waits any more (a strip that would have to goes on with what it has, so every claimed
+ * unit still ends), and the jobs concerned get status -3, no traceback, and make the call fail.
  */
-#define STRIP_WAIT 20000000000LL
 
 /* one 16-byte word of an entry, as one access */
 __device__ __forceinline__ int4 ring_load(const int32_t *e)
@@ -525,7 +524,8 @@ __device__ __forceinline__ void ring_store(int32_t *e, const int x, const int y,
 
 /* the whole warp: the words that lanes with fetch set loaded (w, from e), once all carry tag; false when the
  * wait ran out.  The word and the abort flag are asked for together, a round trip a look */
-__device__ __forceinline__ bool ring_settle(const int32_t *e, int4 &w, const bool fetch, const int tag, int32_t *ctl)
+__device__ __forceinline__ bool ring_settle(const int32_t *e, int4 &w, const bool fetch, const int tag, int32_t *ctl,
+		const plk_params_t &P)
 {
 	if (!__any_sync(FULL, fetch && w.w != tag)) return true;
 	const long long t0 = clock64();
@@ -533,7 +533,7 @@ __device__ __forceinline__ bool ring_settle(const int32_t *e, int4 &w, const boo
 	do {
 		stop = *(volatile int32_t*)(ctl + 2);
 		if (fetch) w = ring_load(e);
-		if (stop == 0 && clock64() - t0 > STRIP_WAIT) stop = 1, atomicExch(ctl + 2, 1);
+		if (stop == 0 && clock64() - t0 > P.strip_wait) stop = 1, atomicExch(ctl + 2, 1);
 		stop = __any_sync(FULL, stop != 0);
 	} while (__any_sync(FULL, fetch && w.w != tag) && !stop);
 	return !__any_sync(FULL, fetch && w.w != tag);
@@ -600,7 +600,7 @@ __device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k,
 		ac[r] = MODE == 0 ? -16 * av : av;
 	}
 	const bool rows_in = i0 < nl;
-	if (!ring_settle(rin + 4 * lane, w, taker, k, ctl)) J->status = -3;
+	if (!ring_settle(rin + 4 * lane, w, taker, k, ctl, P)) J->status = -3;
 	if (taker) *(int4*)(pre[0] + 4 * lane) = w;
 	if (taker && 1 < al) w = ring_load(rin + PLK_RING_INTS + 4 * lane);
 	__syncwarp();
@@ -641,7 +641,7 @@ __device__ __forceinline__ void dp_strip(plk_job_t *__restrict__ J, const int k,
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
-		if (!ring_settle(rin + (int64_t)(s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl)) J->status = -3;
+		if (!ring_settle(rin + (int64_t)(s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl, P)) J->status = -3;
 		if (taker && s + 1 < al) *(int4*)(pre[(s + 1) & 1] + 4 * lane) = w;
 		if (taker && s + 2 < al) w = ring_load(rin + (int64_t)(s + 2) * PLK_RING_INTS + 4 * lane);
 		__syncwarp();
@@ -1070,7 +1070,7 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 		}
 	}
 	const bool rows_in = i0 < nl;
-	if (!ring_settle(rout + (int64_t)rdif * PLK_RING_INTS + 4 * lane, w, taker, k, ctl))
+	if (!ring_settle(rout + (int64_t)rdif * PLK_RING_INTS + 4 * lane, w, taker, k, ctl, P))
 		jobs[ja].status = jobs[jobs[ja].pair].status = -3;
 	if (taker) *(int4*)(pre[0] + 4 * lane) = w;
 	if (taker && 1 < al) w = ring_load(rout + (int64_t)(rdif + 1) * PLK_RING_INTS + 4 * lane);
@@ -1116,7 +1116,7 @@ __device__ __forceinline__ void dp_strip_pair(plk_job_t *__restrict__ jobs, cons
 			for (int r = 0; r < R; ++r) hm[r] = hn[r];
 			ah1 = in[0], ah2 = in[1], ah3 = in[2];
 		}
-		if (!ring_settle(rout + (int64_t)(rdif + s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl))
+		if (!ring_settle(rout + (int64_t)(rdif + s + 1) * PLK_RING_INTS + 4 * lane, w, taker && s + 1 < al, k, ctl, P))
 			jobs[ja].status = jobs[jobs[ja].pair].status = -3;
 		if (taker && s + 1 < al) *(int4*)(pre[(s + 1) & 1] + 4 * lane) = w;
 		if (taker && s + 2 < al) w = ring_load(rout + (int64_t)(rdif + s + 2) * PLK_RING_INTS + 4 * lane);
@@ -1281,6 +1281,10 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 	const int q = blockIdx.x * TB_WARPS + wib;
 	if (q >= n_order) return;
 	plk_job_t *J = jobs + order[q];
+	if (J->status != 0) { /* a strip's wait ran out: no trace to walk */
+		if (lane == 0) J->n_tmp = 0;
+		return;
+	}
 	const int nl = J->nl, al = J->al, R = J->rows;
 	const uint16_t *tr = trace + J->trace_off;
 	TbOut T;  /* lane 0's */
@@ -1374,14 +1378,16 @@ __global__ void __launch_bounds__(32 * TB_WARPS) k_traceback(plk_job_t *__restri
 	}
 }
 
-/* exclusive scan of the CIGAR lengths in job order (single CTA) */
+/* exclusive scan of the CIGAR lengths in job order (single CTA); total[1]: whether a job failed */
 __global__ void k_scan(plk_job_t *jobs, int n_jobs, int64_t *total)
 {
 	__shared__ int64_t s_part[1024];
 	const int tid = threadIdx.x, nt = blockDim.x;
 	const int per = (n_jobs + nt - 1) / nt, b = tid * per, e = min(n_jobs, b + per);
 	int64_t acc = 0;
-	for (int q = b; q < e; ++q) acc += jobs[q].n_tmp;
+	int bad = 0;
+	for (int q = b; q < e; ++q) acc += jobs[q].n_tmp, bad |= jobs[q].status != 0;
+	bad = __syncthreads_or(bad);
 	s_part[tid] = acc;
 	__syncthreads();
 	for (int off = 1; off < nt; off <<= 1) {
@@ -1392,7 +1398,7 @@ __global__ void k_scan(plk_job_t *jobs, int n_jobs, int64_t *total)
 	}
 	int64_t run = s_part[tid] - acc;
 	for (int q = b; q < e; ++q) jobs[q].out_off = run, run += jobs[q].n_tmp;
-	if (tid == nt - 1) *total = s_part[tid];
+	if (tid == nt - 1) total[0] = s_part[tid], total[1] = bad;
 }
 
 __global__ void k_compact(const plk_job_t *__restrict__ jobs, int n_jobs, const uint32_t *__restrict__ tmp,
@@ -1411,7 +1417,7 @@ __global__ void k_compact(const plk_job_t *__restrict__ jobs, int n_jobs, const 
 	}
 	if (lane == 0) {
 		pl_splice_result_t r;
-		r.score = J.score, r.n_cigar = n, r.cigar_off = J.out_off, r.mode = J.mode == 1 ? 32 : 16;
+		r.score = J.status == 0 ? J.score : INT32_MIN, r.n_cigar = n, r.cigar_off = J.out_off, r.mode = J.mode == 1 ? 32 : 16;
 		r.status = fits ? J.status : -2;
 		res[w] = r;
 	}
