@@ -595,7 +595,8 @@ typedef struct pl_pf_model_s pl_pf_model_t;
 /* in_dim: a multiple of 64 (PL_PF_FDIM for pl_pf_features_device rows); hidden 128 or 256. */
 pl_pf_model_t *pl_pf_model_create(int32_t device, int32_t in_dim, int32_t hidden, uint64_t seed);
 void pl_pf_model_destroy(pl_pf_model_t *m);
-/* parameters as fp32, layer by layer: W [out x in] row-major then bias [out] */
+/* parameters as fp32, layer by layer: W [out x in] row-major then bias [out].  get and set
+ * of one model may run in several threads: each reads or writes all of them at once. */
 int64_t pl_pf_model_size(const pl_pf_model_t *m);
 int pl_pf_model_get(const pl_pf_model_t *m, float *params, int64_t n);
 int pl_pf_model_set(pl_pf_model_t *m, const float *params, int64_t n);

@@ -8,13 +8,14 @@
  *
  * Parameters live on the device as fp32 masters with bf16 copies W [out x in] (the
  * forward operand) and W^T [in x out_pad] (the backward operand, out padded to 64).
- * One optimizer step (gather, 4 forward GEMMs, loss, 7 backward GEMMs, 4 bias
- * reductions, 8 Adam updates, step counter) is captured once as a CUDA graph and
+ * One optimizer step (gather, 4 forward GEMMs, loss, 3 backward GEMMs, then one launch
+ * each for the weight gradients, the bias reductions and Adam, step counter) is captured once as a CUDA graph and
  * replayed; the batch position comes from a device step counter, so the graph is the
  * same for every step.
  */
 #define _POSIX_C_SOURCE 200809L
 #include <math.h>
+#include <pthread.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -39,7 +40,9 @@ struct pl_pf_model_s {
 	int32_t in_dim, hidden;
 	pf_layer_t L[PF_LAYERS];
 	int32_t *err, *step;
-	float *loss_sum, *loss_log, *flat;
+	float *loss_sum, *loss_log;
+	float *flat;             /* all parameters in one array, between the host and the tensors: */
+	pthread_mutex_t mu;      /* one upload or download at a time, from any thread */
 	/* training buffers for batch size tb */
 	int32_t tb;
 	void *X, *XT, *H[3], *HT[3], *dout, *doutT, *dZ[3], *dZT[3];
@@ -88,6 +91,7 @@ PL_EXPORT void pl_pf_model_destroy(pl_pf_model_t *m)
 		cudaFree(y->W), cudaFree(y->WT), cudaFree(y->gW), cudaFree(y->gb);
 	}
 	cudaFree(m->err), cudaFree(m->step), cudaFree(m->loss_sum), cudaFree(m->loss_log), cudaFree(m->flat);
+	pthread_mutex_destroy(&m->mu);
 	free(m);
 }
 
@@ -123,14 +127,17 @@ static void pf_tensors(const pl_pf_model_t *m, plk_mlp_adam_t *a)
 static int pf_upload(pl_pf_model_t *m, const float *params)
 {
 	plk_mlp_adam_t a;
+	int ok = 0;
 	pf_tensors(m, &a);
+	pthread_mutex_lock(&m->mu);
 	CK(cudaMemcpy(m->flat, params, sizeof(float) * (size_t)pl_pf_model_size(m), cudaMemcpyHostToDevice));
 	CKK(plk_mlp_params(&a, m->flat, 1, 0));
 	CK(cudaMemsetAsync(m->step, 0, sizeof(int32_t), 0));
 	CK(cudaStreamSynchronize(0));
-	return 1;
+	ok = 1;
 fail:
-	return 0;
+	pthread_mutex_unlock(&m->mu);
+	return ok;
 }
 
 PL_EXPORT int pl_pf_model_set(pl_pf_model_t *m, const float *params, int64_t n)
@@ -144,15 +151,20 @@ PL_EXPORT int pl_pf_model_set(pl_pf_model_t *m, const float *params, int64_t n)
 PL_EXPORT int pl_pf_model_get(const pl_pf_model_t *m, float *params, int64_t n)
 {
 	plk_mlp_adam_t a;
+	pthread_mutex_t *mu;
+	int ok = 0;
 	if (!m || !params || n != pl_pf_model_size(m)) { pl_set_error("parameter count mismatch"); return 0; }
+	mu = (pthread_mutex_t*)&m->mu;
+	pf_tensors(m, &a);
+	pthread_mutex_lock(mu);
 	CK(cudaSetDevice(m->device));
 	CK(cudaDeviceSynchronize());
-	pf_tensors(m, &a);
 	CKK(plk_mlp_params(&a, m->flat, 0, 0));
 	CK(cudaMemcpy(params, m->flat, sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost));
-	return 1;
+	ok = 1;
 fail:
-	return 0;
+	pthread_mutex_unlock(mu);
+	return ok;
 }
 
 PL_EXPORT pl_pf_model_t *pl_pf_model_create(int32_t device, int32_t in_dim, int32_t hidden, uint64_t seed)
@@ -168,6 +180,7 @@ PL_EXPORT pl_pf_model_t *pl_pf_model_create(int32_t device, int32_t in_dim, int3
 	}
 	m = (pl_pf_model_t*)calloc(1, sizeof(*m));
 	if (!m) { pl_set_error("out of host memory"); return 0; }
+	pthread_mutex_init(&m->mu, 0);
 	m->device = device, m->in_dim = in_dim, m->hidden = hidden;
 	CK(cudaSetDevice(device));
 	for (l = 0; l < PF_LAYERS; ++l) {
