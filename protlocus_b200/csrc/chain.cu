@@ -4,8 +4,8 @@
  * there, its predecessor p[i] and the peak score v[i] along that chain.
  *
  * Two kernels.  k_chain_score computes comput_sc of every anchor against the 32
- * before it, a lane per pair.  k_chain_fill walks one query per thread, one such
- * thread per warp (the host orders queries longest first, so the longest start
+ * before it, a lane per pair.  k_chain_fill walks one query per thread, one or four such
+ * threads per warp (the host orders queries longest first, so the longest start
  * first).  The loop over predecessors is the reference's,
  * statement for statement: a running best (strictly greater wins, so the nearest j
  * keeps a tie), a skip counter that rises on a non-improving predecessor already
@@ -31,7 +31,7 @@ extern "C" void plk_add_launches(uint64_t n);
 
 namespace {
 
-constexpr int CHAIN_THREADS = 128, CHAIN_STRIDE = 32;
+constexpr int CHAIN_THREADS = 128;
 constexpr int BLOCK_BONUS = 2;  /* MP_BLOCK_BONUS (protlocus.h:47) */
 
 /* log2 approximation of the reference (mppriv.h:143-151), valid for x >= 2: the
@@ -88,20 +88,20 @@ __device__ __forceinline__ int chain_score(uint64_t ai, uint64_t aj, const plk_c
 	return sc;
 }
 
-/* rows[(r0 + i) * 32 + k] = the score of chaining anchor i - 1 - k before anchor i, k < 32, for the
- * queries order[first ..]: a CTA per query, a warp per anchor */
+/* rows[(row0 + i - i0) * 32 + k] = the score of chaining anchor i - 1 - k before anchor i, k < 32, for
+ * this launch's anchors: a CTA per query, a warp per anchor */
 __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_score(plk_chain_args_t A)
 {
 	const int q = A.order[blockIdx.x];
 	if (q < 0 || q >= A.n_all) return;  /* k_chain_fill reports it */
 	const int64_t base = A.off[q];
-	const int n = A.n[q], lane = threadIdx.x & 31;
+	const int n = A.n[q], lane = threadIdx.x & 31, end = min(n, A.i1);
 	if (base < 0 || n < 0 || base + n > A.n_a) return;
 	const uint64_t *__restrict__ a = A.a + base;
 	int32_t *row = A.rows + (A.row0[blockIdx.x] << 5);
-	for (int i = threadIdx.x >> 5; i < n; i += CHAIN_THREADS / 32) {
+	for (int i = A.i0 + (threadIdx.x >> 5); i < end; i += CHAIN_THREADS / 32) {
 		const int j = i - 1 - lane;
-		if (j >= 0) row[((int64_t)i << 5) + lane] = chain_score(a[i], a[j], A);
+		if (j >= 0) row[((int64_t)(i - A.i0) << 5) + lane] = chain_score(a[i], a[j], A);
 	}
 }
 
@@ -109,11 +109,14 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_score(plk_chain_args_t 
  * early exit, skip counter and marks, so the order of every comparison is the
  * reference's.  Per anchor a record {f, p, t, v}.  Every per-query index is checked against the
  * query's length; a bad one records the site and the query (err[0], err[1]) and the access is
- * skipped. */
+ * skipped.  A batch whose score rows do not fit runs in several launches, every query some
+ * anchors further in each (its walk's three values kept between them): launches of fewer
+ * queries instead, each waiting for its own longest walk, took 1,100 ms for 400 queries of
+ * 100,000 anchors where these take 110. */
 __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_fill(plk_chain_args_t A)
 {
-	if (threadIdx.x % CHAIN_STRIDE) return;
-	const int qi = (blockIdx.x * CHAIN_THREADS + threadIdx.x) / CHAIN_STRIDE;
+	if (threadIdx.x & (A.stride - 1)) return;
+	const int qi = (blockIdx.x * CHAIN_THREADS + threadIdx.x) / A.stride;
 	if (qi >= A.n_q) return;
 	const int q = A.order[qi];
 	if (q < 0 || q >= A.n_all) { atomicExch(A.err, 1); return; }
@@ -122,15 +125,20 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_fill(plk_chain_args_t A
 	if (base < 0 || n < 0 || base + n > A.n_a) { atomicExch(A.err, 2), atomicExch(A.err + 1, q); return; }
 	const uint64_t *__restrict__ a = A.a + base;
 	const int32_t *__restrict__ rows = A.rows + (A.row0[qi] << 5);
+	const int end = min(n, A.i1);
 	int32_t *f = A.f + base, *p = A.p + base, *v = A.v + base;
 	int4 *rec = (int4*)A.rec + base;
 #define CHK(x, site) ((unsigned)(x) < (unsigned)n ? true : (atomicExch(A.err, (site)), atomicExch(A.err + 1, q), false))
 	int st = 0, hi = -1, hf = 0;
+	if (A.i0 > 0) {
+		const int4 s = ((const int4*)A.state)[q];
+		st = s.x, hi = s.y, hf = s.z;
+	}
 	unsigned long long pairs = 0;
-	for (int i = 0; i < n; ++i) {
+	for (int i = A.i0; i < end; ++i) {
 		const uint64_t ai = a[i];
-		const int32_t *row = rows + ((int64_t)i << 5);
-		if (i + 2 < n) { /* the next anchors' row and the anchors, on their way from L2 */
+		const int32_t *row = rows + ((int64_t)(i - A.i0) << 5);
+		if (i + 2 < end) { /* the next anchors' row and the anchors, on their way from L2 */
 			asm volatile("prefetch.global.L1 [%0];" :: "l"(row + 64));
 			asm volatile("prefetch.global.L1 [%0];" :: "l"(a + min(i + 16, n - 1)));
 		}
@@ -190,6 +198,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain_fill(plk_chain_args_t A
 		if (hf < max_f) hf = max_f, hi = i;
 	}
 #undef CHK
+	if (end < n) ((int4*)A.state)[q] = make_int4(st, hi, hf, 0);
 	if (A.pairs) atomicAdd(A.pairs, pairs);
 }
 
@@ -202,7 +211,7 @@ extern "C" int plk_chain_fill(const plk_chain_args_t *a, void *stream)
 	k_chain_score<<<a->n_q, CHAIN_THREADS, 0, st>>>(*a);
 	cudaError_t e = cudaGetLastError();
 	if (e != cudaSuccess) return (int)e;
-	constexpr int per = CHAIN_THREADS / CHAIN_STRIDE;
+	const int per = CHAIN_THREADS / a->stride;
 	k_chain_fill<<<(a->n_q + per - 1) / per, CHAIN_THREADS, 0, st>>>(*a);
 	plk_add_launches(2);
 	return (int)cudaGetLastError();

@@ -392,19 +392,21 @@ static inline PLK_HD int plk_ps_band_ok(int32_t L, int32_t n, int32_t band, int3
 }
 
 /* anchor chaining DP (chain.c:160-208): thread g takes query order[g], anchors a[off[q] ..
- * off[q] + n[q]); f, p, v per anchor out, t per anchor scratch (mark stamps) */
+ * off[q] + n[q]), of which this launch fills i0 .. i1 - 1; f, p, v per anchor out */
 typedef struct {
 	const int64_t *off;
 	const int32_t *n, *order;
 	const uint64_t *a;
 	int32_t *f, *p, *v;
 	void *rec;                   /* per anchor 16 bytes of scratch */
-	int32_t *rows;               /* scores against the 32 anchors before, from row row0[i] for query order[i] */
+	int32_t *rows;               /* scores against the 32 anchors before, of anchors i0 on from row row0[g] on */
 	const int64_t *row0;
+	void *state;                 /* per query 16 bytes: where its walk is at i1, for the launch that goes on */
 	unsigned long long *pairs;   /* optional: predecessors scored, summed over queries */
 	int32_t *err;                /* set non-zero by a query whose indices leave their ranges (then skipped) */
 	int64_t n_a;                 /* anchors in a / f / p / v / rec */
 	int32_t n_q, n_all;          /* queries of this launch, of the batch */
+	int32_t i0, i1, stride;      /* stride: lanes a query, 32 or 8 */
 	int32_t max_dist_x, max_dist_y, bw, max_skip, max_iter, is_spliced, kmer, bbit;
 	float coef;
 } plk_chain_args_t;
