@@ -122,7 +122,6 @@ void pl_hmm_engine_free(pl_engine_t *e)
 	{
 		int s;
 		for (s = 0; s < PL_HMM_STREAMS; ++s) {
-			dbuf_free(&e->h_edge_s[s]);
 			if (e->h_st[s]) cudaStreamDestroy(e->h_st[s]), e->h_st[s] = 0;
 		}
 		for (s = 0; s <= PL_HMM_STREAMS; ++s)
@@ -168,26 +167,39 @@ static int pl_hmm_plan(pl_engine_t *e, int32_t n, const int32_t *len, int64_t **
 	return 1;
 }
 
+/* CTAs of a profile's launch over n regions; its edge buffer (columns handed from tile to tile, two
+ * rows of 16 bytes a warp, the rows in fours as the paired kernel walks them): none for one tile */
+static int32_t pl_hmm_ctas(const pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n)
+{
+	const int32_t units = p->k.cols ? (n + 1) / 2 : n, warps = plk_hmm_warps_per_cta();  /* the paired kernel: two regions a warp */
+	int64_t ctas = plk_hmm_ctas_per_sm(&p->k);
+	if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
+	ctas *= e->n_sm;
+	if (ctas * warps > units) ctas = (units + warps - 1) / warps;
+	return (int32_t)ctas;
+}
+static int64_t pl_hmm_edge_rows(int32_t max_rows) { return ((int64_t)max_rows + 3) / 4 * 4 + 4; }
+static size_t pl_hmm_edge_bytes(const pl_hmm_profile_t *p, int32_t max_rows, int32_t ctas)
+{
+	if (p->k.mpad <= PLK_HMM_TILE) return 0;
+	return (size_t)16 * 2 * (size_t)pl_hmm_edge_rows(max_rows) * (size_t)ctas * plk_hmm_warps_per_cta();
+}
+
 static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, const uint8_t *nt_dev,
 		const int32_t *off, const int32_t *len, int32_t *score_dev, cudaStream_t st)
 {
-	int64_t *row_off, rows_total, cells = 0, edge_rows;
-	int32_t *order, max_rows, ctas, units, q;
+	int64_t *row_off, rows_total, cells = 0;
+	int32_t *order, max_rows, ctas, q;
 	if (n <= 0) return 1;
 	if (!p) { pl_set_error("no profile"); return 0; }
 	if (p->device != e->device) { pl_set_error("profile on device %d, engine on device %d", p->device, e->device); return 0; }
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
-	edge_rows = ((int64_t)max_rows + 3) / 4 * 4 + 4;  /* the paired kernel walks rows in fours */
 	for (q = 0; q < n; ++q) cells += (int64_t)(len[q] >= 3 ? len[q] / 3 : 0) * p->k.m;
-	ctas = plk_hmm_ctas_per_sm(&p->k);
-	if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
-	ctas *= e->n_sm;
-	units = p->k.cols ? (n + 1) / 2 : n;  /* the paired kernel takes two regions a warp */
-	if ((int64_t)ctas * plk_hmm_warps_per_cta() > units) ctas = (units + plk_hmm_warps_per_cta() - 1) / plk_hmm_warps_per_cta();
+	if ((ctas = pl_hmm_ctas(e, p, n)) < 1) return 0;
 	if (!dbuf_ensure(&e->h_off, sizeof(int32_t) * (size_t)n) || !dbuf_ensure(&e->h_len, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rowoff, sizeof(int64_t) * (size_t)n) || !dbuf_ensure(&e->h_order, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rows, (size_t)(rows_total > 0 ? rows_total : 16)) || !dbuf_ensure(&e->h_counter, 64) ||
-			!dbuf_ensure(&e->h_edge, (size_t)16 * 2 * (size_t)edge_rows * (size_t)ctas * plk_hmm_warps_per_cta()))
+			!dbuf_ensure(&e->h_edge, pl_hmm_edge_bytes(p, max_rows, ctas)))
 		return 0;
 	CK(cudaMemcpyAsync(e->h_off.p, off, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->h_len.p, len, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
@@ -200,7 +212,7 @@ static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, cons
 	PL_TIME(e, st, 0);
 	PL_TIME(e, st, 1);
 	CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
-			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, edge_rows, ctas,
+			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, pl_hmm_edge_rows(max_rows), ctas,
 			score_dev, st));
 	PL_TIME(e, st, 1);
 	CK(cudaStreamSynchronize(st));
@@ -229,14 +241,18 @@ PL_EXPORT int pl_hmm_score_device(pl_engine_t *e, const pl_hmm_profile_t *p, int
 
 /* Many profiles against one region set: the planning, the upload of the region tables and
  * the codon translation once (again only when a profile's codon table differs from the
- * previous one's), then one DP launch per profile, round-robin on PL_HMM_STREAMS streams
- * with their own queue counters and edge buffers, so that the launches of a region set too
- * small to fill the GPU run side by side. */
+ * previous one's), then one DP launch per profile, round-robin on up to PL_HMM_STREAMS streams
+ * with their own queue counters and parts of the edge buffer, so that the launches of a region set
+ * too small to fill the GPU run side by side.  All memory is there before the first launch (growing
+ * a buffer waits for the launches under way), streams and events as many as there are profiles for. */
 PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *const *ps, int32_t n_prof, int32_t n,
 		const uint8_t *nt, const int32_t *off, const int32_t *len, int32_t *score_dev, void *stream)
 {
-	int64_t *row_off, rows_total, cells = 0, rows_sum = 0, edge_rows;
-	int32_t *order, max_rows, q, k, s, warps;
+	int64_t *row_off, rows_total, cells = 0, rows_sum = 0;
+	size_t edge[PL_HMM_STREAMS + 1] = {0};  /* bytes of each stream's part, then where it starts */
+	int32_t *order, max_rows, q, k, s, *ctas = 0;
+	const int32_t n_st = n_prof < PL_HMM_STREAMS ? n_prof : PL_HMM_STREAMS;
+	int ok = 0;
 	const uint8_t *codon = 0;
 	cudaStream_t st;
 	if (!e) { pl_set_error("no engine"); return 0; }
@@ -247,18 +263,25 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	CK(cudaSetDevice(e->device));
 	st = stream ? (cudaStream_t)stream : e->stream;
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
-	edge_rows = ((int64_t)max_rows + 3) / 4 * 4 + 4;  /* the paired kernel walks rows in fours */
 	for (q = 0; q < n; ++q) rows_sum += len[q] >= 3 ? len[q] / 3 : 0;
-	warps = plk_hmm_warps_per_cta();
-	for (s = 0; s < PL_HMM_STREAMS; ++s)
+	ctas = (int32_t*)malloc(sizeof(int32_t) * (size_t)n_prof);
+	if (!ctas) { pl_set_error("out of host memory"); goto fail; }
+	for (k = 0; k < n_prof; ++k) {
+		size_t b;
+		if ((ctas[k] = pl_hmm_ctas(e, ps[k], n)) < 1) goto fail;
+		b = pl_hmm_edge_bytes(ps[k], max_rows, ctas[k]);
+		if (b > edge[k % PL_HMM_STREAMS + 1]) edge[k % PL_HMM_STREAMS + 1] = b;
+	}
+	for (s = 0; s < n_st; ++s) edge[s + 1] += edge[s];
+	for (s = 0; s < n_st; ++s)
 		if (!e->h_st[s]) CK(cudaStreamCreateWithFlags(&e->h_st[s], cudaStreamNonBlocking));
 	for (s = 0; s <= PL_HMM_STREAMS; ++s)
-		if (!e->h_ev[s]) CK(cudaEventCreateWithFlags(&e->h_ev[s], cudaEventDisableTiming));
+		if ((s < n_st || s == PL_HMM_STREAMS) && !e->h_ev[s]) CK(cudaEventCreateWithFlags(&e->h_ev[s], cudaEventDisableTiming));
 	if (!dbuf_ensure(&e->h_off, sizeof(int32_t) * (size_t)n) || !dbuf_ensure(&e->h_len, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rowoff, sizeof(int64_t) * (size_t)n) || !dbuf_ensure(&e->h_order, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rows, (size_t)(rows_total > 0 ? rows_total : 16)) ||
-			!dbuf_ensure(&e->h_counter, 64 * PL_HMM_STREAMS))
-		return 0;
+			!dbuf_ensure(&e->h_counter, 64 * PL_HMM_STREAMS) || !dbuf_ensure(&e->h_edge, edge[n_st]))
+		goto fail;
 	CK(cudaMemcpyAsync(e->h_off.p, off, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->h_len.p, len, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->h_rowoff.p, row_off, sizeof(int64_t) * (size_t)n, cudaMemcpyHostToDevice, st));
@@ -267,15 +290,10 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	PL_TIME(e, st, 1);
 	for (k = 0; k < n_prof; ++k) {
 		const pl_hmm_profile_t *p = ps[k];
-		int32_t ctas = plk_hmm_ctas_per_sm(&p->k), units;
 		cudaStream_t sk;
-		if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
-		ctas *= e->n_sm;
-		units = p->k.cols ? (n + 1) / 2 : n;
-		if ((int64_t)ctas * warps > units) ctas = (units + warps - 1) / warps;
 		if (!codon || memcmp(codon, p->codon, 64) != 0) {  /* the rows of this codon table, then fork again */
 			if (codon) {  /* every launch reading the previous rows has finished */
-				for (s = 0; s < PL_HMM_STREAMS; ++s) {
+				for (s = 0; s < n_st; ++s) {
 					CK(cudaEventRecord(e->h_ev[s], e->h_st[s]));
 					CK(cudaStreamWaitEvent(st, e->h_ev[s], 0));
 				}
@@ -283,17 +301,16 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 			CKK(plk_hmm_codons(nt, (const int32_t*)e->h_off.p, (const int32_t*)e->h_len.p, (const int64_t*)e->h_rowoff.p,
 					n, p->codon_dev, (uint8_t*)e->h_rows.p, st));
 			CK(cudaEventRecord(e->h_ev[PL_HMM_STREAMS], st));
-			for (s = 0; s < PL_HMM_STREAMS; ++s) CK(cudaStreamWaitEvent(e->h_st[s], e->h_ev[PL_HMM_STREAMS], 0));
+			for (s = 0; s < n_st; ++s) CK(cudaStreamWaitEvent(e->h_st[s], e->h_ev[PL_HMM_STREAMS], 0));
 			codon = p->codon;
 		}
 		s = k % PL_HMM_STREAMS, sk = e->h_st[s];
-		if (!dbuf_ensure(&e->h_edge_s[s], (size_t)16 * 2 * (size_t)edge_rows * (size_t)ctas * warps)) return 0;
 		CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
-				(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p + 16 * s, e->h_edge_s[s].p,
-				edge_rows, ctas, score_dev + (int64_t)k * n, sk));
+				(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p + 16 * s,
+				(char*)e->h_edge.p + edge[s], pl_hmm_edge_rows(max_rows), ctas[k], score_dev + (int64_t)k * n, sk));
 		cells += rows_sum * p->k.m;
 	}
-	for (s = 0; s < PL_HMM_STREAMS; ++s) {  /* join */
+	for (s = 0; s < n_st; ++s) {  /* join */
 		CK(cudaEventRecord(e->h_ev[s], e->h_st[s]));
 		CK(cudaStreamWaitEvent(st, e->h_ev[s], 0));
 	}
@@ -305,9 +322,10 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 		e->acc_dp_launches += n_prof, e->acc_cells += cells;
 	}
 	e->h_last_cells = cells;
-	return 1;
+	ok = 1;
 fail:
-	return 0;
+	free(ctas);
+	return ok;
 }
 
 /* pl_hmm_score_many_device from host buffers: the region set uploaded once, the
