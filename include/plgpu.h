@@ -207,7 +207,8 @@ int pl_measure_int_peak(int32_t device, double *int32_lane_ops, double *int16x2_
 /* Tuning of the batched global DP: jobs with at most r4_rows DP rows (nl - 2) run 4
  * rows per lane, the rest 8; the strips of a job (32 lanes of rows each) are shared among
  * the GPU's warps when it holds more than coop_ratio times a third of a warp's share of its
- * wave's cells, else one warp runs them all.  set: negative / non-positive
+ * wave's cells (four times that, or never, where the wave is estimated to end sooner so: many
+ * jobs of about a warp's share), else one warp runs them all.  set: negative / non-positive
  * arguments keep the current value.  autotune: times the given batch (results
  * discarded) under a grid of both, keeps the fastest on the engine and reports it. */
 void pl_engine_set_tuning(pl_engine_t *e, int32_t r4_rows, double coop_ratio);

@@ -25,6 +25,7 @@
 #include <errno.h>
 #include <limits.h>
 #include <pthread.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 #include <stdlib.h>
@@ -502,6 +503,59 @@ PL_EXPORT int pl_debug_strip_wait(int64_t cycles)
 	return 1;
 }
 
+/* Which of a wave's jobs share their strips: those of more than *limit cells.  The share of
+ * pl_coop_ratio is right where a batch's jobs differ: the large ones must not trail.  A strip of its
+ * own costs al + 51 steps, though (31 of filling and draining, some twenty to start), against al (at
+ * least 33) in a whole job, so where all jobs are about a warp's share or less, and short proteins
+ * above all, whole jobs on the warps end sooner: 5,000 jobs of some 20 aa against 300 bases 0.45 ms
+ * shared, 0.35 whole; of 40 aa against 4 kb 4.1 and 3.3; but 2,400 of 350 aa against 4 kb 10.8 and
+ * 16.0.  So the launch's time is estimated for that share, four times it and no sharing, and the
+ * least is taken.  In steps of a full GPU (1.45 us): the strips' work over the warps, then the whole
+ * jobs' over the warps or the longest of them (a step of one that others do not cover: 1.65 us), and
+ * a quarter of a mean unit for the uneven end; at least the longest chain of strips (0.74 us a
+ * step). */
+static int pl_share_limits(const pl_engine_t *e, int32_t n, int32_t n_waves, const int64_t *wave_cells, int64_t slots, double *limit)
+{
+	typedef struct { double strips, whole, units, chain, longest; } est_t;
+	est_t *est = (est_t*)calloc((size_t)n_waves * 3, sizeof(est_t));
+	int32_t q, w;
+	int c;
+	if (!est) { pl_set_error("out of host memory"); return 0; }
+	for (w = 0; w < n_waves; ++w) limit[w] = (double)(wave_cells[w] / slots) * e->coop_ratio / 3.0;
+	for (q = 0; q < n; ++q) {
+		const plk_job_t *J = &e->hj[q];
+		const int pair = J->mode == 3;
+		const double S = (double)plk_strips(J->nl, J->rows), f = pair ? 1.7 : 1, cells = (double)(J->nl - 2) * J->al * (pair ? 2 : 1);
+		if (pair && J->pair < 0) continue;  /* a pair once */
+		for (c = 0; c < 3; ++c) {
+			est_t *x = &est[e->hwave[q] * 3 + c];
+			if (S <= PLK_MAX_STRIPS && c < 2 && cells > (c ? 4 : 1) * limit[e->hwave[q]]) {
+				const double t = 0.5 * f * (S * 40 + J->al);
+				x->strips += f * S * (J->al + 51), x->units += S;
+				if (t > x->chain) x->chain = t;
+			} else {
+				const double t = f * (S * (J->al > 33 ? J->al : 33) + 31);
+				x->whole += t, x->units += 1;
+				if (1.14 * t > x->longest) x->longest = 1.14 * t;
+			}
+		}
+	}
+	for (w = 0; w < n_waves; ++w) {
+		const double share = limit[w];
+		double best = 0;
+		for (c = 0; c < 3; ++c) {
+			const est_t *x = &est[w * 3 + c];
+			double t = x->whole / (double)slots + (x->units > 0 ? 0.25 * (x->strips + x->whole) / x->units : 0);
+			if (t < x->longest) t = x->longest;
+			t += x->strips / (double)slots;
+			if (t < x->chain) t = x->chain;
+			if (c == 0 || t < best) best = t, limit[w] = c == 0 ? share : c == 1 ? 4 * share : INFINITY;
+		}
+	}
+	free(est);
+	return 1;
+}
+
 static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jobs, int32_t n,
 		const uint8_t *nt, const uint8_t *aa, const uint8_t *ss, pl_splice_result_t *res_dev,
 		uint32_t *cig_dev, int64_t cig_cap, int64_t *total_out, cudaStream_t st)
@@ -512,6 +566,7 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 	int64_t ring_ints = 0, sring_ints = 0, ring_stride = 0, max_units = 0;
 	const int64_t units_off = ((int64_t)n * 4 + 15) / 16 * 16;  /* the strip queues sit behind the order array */
 	plk_dp_group_t *grp = 0;
+	double *share_limit = 0;
 	int32_t *wave_grp = 0, *bucket = 0;
 	int64_t *wave_bytes = 0, *wave_cells = 0, total[2] = {0, 0};  /* CIGAR words; a job failed */
 	int ok = 0, capturing = 0;
@@ -595,13 +650,16 @@ static int pl_run(pl_engine_t *e, const ns_opt_t *opt, const pl_splice_job_t *jo
 		}
 	}
 	/* 3. shared or solo, trace offsets inside each wave's arena */
+	share_limit = (double*)malloc(sizeof(double) * (size_t)n_waves);
+	if (!share_limit) { pl_set_error("out of host memory"); goto fail; }
+	if (!pl_share_limits(e, n, n_waves, wave_cells, slots, share_limit)) goto fail;
 	memset(wave_bytes, 0, sizeof(int64_t) * (size_t)n_waves);
 	for (q = 0; q < n; ++q) {
 		const int32_t j = sorted[q];
 		plk_job_t *J = &e->hj[j];
 		const int64_t cells = (int64_t)(J->nl - 2) * J->al * (J->mode == 3 ? 2 : 1), strips = plk_strips(J->nl, J->rows);
 		J->shared = strips <= PLK_MAX_STRIPS &&
-				(double)cells > (double)(wave_cells[e->hwave[j]] / slots) * e->coop_ratio / 3.0;
+				(double)cells > share_limit[e->hwave[j]];
 		J->trace_off = wave_bytes[e->hwave[j]] / 2;
 		wave_bytes[e->hwave[j]] += (plk_trace_words(J->nl, J->al, J->rows) * 2 + 15) / 16 * 16;
 	}
@@ -798,7 +856,7 @@ fail:
 		cudaGetLastError();
 		e->g_prev_key = 0;
 	}
-	free(wave_bytes), free(wave_cells), free(grp), free(wave_grp), free(bucket);
+	free(wave_bytes), free(wave_cells), free(share_limit), free(grp), free(wave_grp), free(bucket);
 	return ok;
 }
 
