@@ -8,7 +8,7 @@
  *                patterns lo, lo+stride, ... < hi and counts the results that differ
  *                in any bit (NaN results compare equal to NaN);
  *   lm_host:     fills out[] with the host libm's values at n bit patterns, for the
- *                comparison with the device build.
+ *                comparison with the device build (fn 6: rc_logsum's term log1pf(expf(-x))).
  * Built with -ffp-contract=off so the header's host build keeps its written roundings.
  */
 #include <stdint.h>
@@ -20,7 +20,7 @@
 
 /* fn 0 / 1: gl_expf / gl_log1pf; fn 2 / 3: their branch-free forms for rc_logsum's ranges,
  * gl_expf_rng (|x| < 88) and gl_log1pf_unit (0 <= x <= 1), checked on those ranges */
-static float lm_host_fn(int fn, float x) { return (fn & 1) == 0 ? expf(x) : log1pf(x); }
+static float lm_host_fn(int fn, float x) { return fn == 6 ? log1pf(expf(-x)) : (fn & 1) == 0 ? expf(x) : log1pf(x); }
 static float lm_port_fn(int fn, float x)
 {
 	return fn == 0 ? gl_expf(x) : fn == 1 ? gl_log1pf(x) : fn == 2 ? gl_expf_rng(x) : gl_log1pf_unit(x);
