@@ -65,7 +65,8 @@ k_hmm_dp(const plk_hmm_prof_t P, const uint8_t *__restrict__ rows, const int64_t
 		__syncthreads();
 	}
 	const int16_t *emit = SMEM_EMIT ? s_emit : (const int16_t*)P.emit_t;
-	int4 *my_edge = edge + (int64_t)(blockIdx.x * HMM_WARPS + wib) * 2 * edge_stride;
+	if (wib >= P.warps) return;
+	int4 *my_edge = edge + (int64_t)(blockIdx.x * P.warps + wib) * 2 * edge_stride;
 	for (;;) {
 		int idx = 0;
 		if (lane == 0) idx = atomicAdd(counter, 1);
@@ -163,7 +164,8 @@ k_hmm_pair(const plk_hmm_prof_t P, const uint8_t *__restrict__ rows, const int64
 		__syncthreads();
 	}
 	const uint32_t *emit = SMEM_EMIT ? s_emit2 : (const uint32_t*)P.emit_t;
-	int4 *my_edge = edge + (int64_t)(blockIdx.x * HMM_WARPS + wib) * 2 * edge_stride;
+	if (wib >= P.warps) return;
+	int4 *my_edge = edge + (int64_t)(blockIdx.x * P.warps + wib) * 2 * edge_stride;
 	for (;;) {
 		int idx = 0;
 		if (lane == 0) idx = atomicAdd(counter, 1);
@@ -291,7 +293,7 @@ extern "C" int plk_hmm_codons(const uint8_t *nt, const int32_t *off, const int32
 
 extern "C" int plk_hmm_dp(const plk_hmm_prof_t *p, const uint8_t *rows, const int64_t *row_off, const int32_t *len,
 		const int32_t *order, int32_t n, int32_t *counter, void *edge, int64_t edge_stride_rows, int32_t n_ctas,
-		int32_t *score, void *stream)
+		int32_t warps, int32_t *score, void *stream)
 {
 	if (n <= 0) return 0;
 	cudaStream_t st = (cudaStream_t)stream;
@@ -300,7 +302,9 @@ extern "C" int plk_hmm_dp(const plk_hmm_prof_t *p, const uint8_t *rows, const in
 	hmm_kernel_t f = hmm_kernel(p);
 	e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, PLK_HMM_SMEM_PAIR);
 	if (e != cudaSuccess) return (int)e;
-	f<<<n_ctas, 32 * HMM_WARPS, hmm_smem(p), st>>>(*p, rows, row_off, len, order, n, counter, (int4*)edge, edge_stride_rows, score);
+	plk_hmm_prof_t P = *p;
+	P.warps = warps;
+	f<<<n_ctas, 32 * HMM_WARPS, hmm_smem(p), st>>>(P, rows, row_off, len, order, n, counter, (int4*)edge, edge_stride_rows, score);
 	plk_add_launches(1);
 	return (int)cudaGetLastError();
 }

@@ -21,8 +21,10 @@
 
 struct pl_hmm_profile_s {
 	int device;
-	plk_hmm_prof_t k;      /* device tables */
-	uint8_t *codon_dev;    /* codon index -> HMMER column, 20 = no emission */
+	plk_hmm_prof_t k;      /* the profile for the paired kernel where it fits that, else for the 32-bit one */
+	plk_hmm_prof_t k32;    /* a paired profile for the 32-bit kernel, where that can be the faster one */
+	void *dev;             /* their tables, one block */
+	uint8_t *codon_dev;    /* codon index -> HMMER column, 20 = no emission (in dev) */
 	uint8_t codon[64];     /* the same, on the host */
 };
 
@@ -45,62 +47,78 @@ static int pl_hmm_cols(int32_t m, const int16_t *emit, const int16_t *trans, int
 	return cols < 2 ? 2 : cols;
 }
 
+/* the 32-bit kernel's tables: column j holds profile position j (the DP's column j+1) */
+static void pl_hmm_tables32(int32_t m, int32_t mpad, const int16_t *emit, const int16_t *trans, int16_t *e, int32_t *t)
+{
+	int32_t j, k;
+	for (j = 0; j < m; ++j)
+		for (k = 0; k < 20; ++k) e[(size_t)k * mpad + j] = emit[(size_t)j * 20 + k];
+	for (k = 0; k < 7; ++k)
+		for (j = 0; j < mpad; ++j) t[(size_t)k * mpad + j] = j < m ? trans[(size_t)j * 7 + k] : -(1 << 28);
+}
+
+/* With one region a warp on a scheduler of its own, the 32-bit kernel takes 0.11 us a row and tile and
+ * the paired one 0.08 to 0.16, by its columns a lane: 2,000 rows of 250 columns 0.23 and 0.32 ms, of
+ * 400 0.46 and 0.53, of 300 (five columns a lane) 0.46 and 0.44.  So profiles of more than five columns
+ * a lane have both kernels' tables, and scans of at most a region a scheduler take the 32-bit one. */
+#define PL_HMM_BOTH 6
+
 PL_EXPORT pl_hmm_profile_t *pl_hmm_profile_create(int32_t device, int32_t m, const int16_t *emit,
 		const int16_t *trans, const uint8_t *codon_alpha)
 {
 	pl_hmm_profile_t *p;
-	int16_t *e = 0;
-	uint32_t *e32 = 0;
-	int32_t *t = 0;
+	char *host = 0;
 	int32_t mpad, j, k, cols, t_floor = 0, e_floor = 0;
+	size_t row, o_t, o_codon, o_e32, o_t32, size;
 	if (m <= 0 || !emit || !trans || !codon_alpha) { pl_set_error("pl_hmm_profile_create: empty profile"); return 0; }
 	for (k = 0; k < 64; ++k)
 		if (codon_alpha[k] > 20) { pl_set_error("codon_alpha[%d] = %d (HMMER columns 0-19, 20 = none)", k, codon_alpha[k]); return 0; }
 	mpad = (m + PLK_HMM_TILE - 1) / PLK_HMM_TILE * PLK_HMM_TILE;
-	p = (pl_hmm_profile_t*)calloc(1, sizeof(*p));
-	e = (int16_t*)calloc((size_t)21 * mpad, sizeof(uint32_t));  /* either kernel's table */
-	t = (int32_t*)malloc(sizeof(int32_t) * 7 * (size_t)mpad);
-	if (!p || !e || !t) { pl_set_error("out of host memory"); goto fail; }
 	cols = pl_hmm_cols(m, emit, trans, &t_floor, &e_floor);
-	if (cols == 0) {
-		for (j = 0; j < m; ++j) /* column j holds profile position j (the DP's column j+1) */
-			for (k = 0; k < 20; ++k) e[(size_t)k * mpad + j] = emit[(size_t)j * 20 + k];
-		for (k = 0; k < 7; ++k)
-			for (j = 0; j < mpad; ++j) t[(size_t)k * mpad + j] = j < m ? trans[(size_t)j * 7 + k] : -(1 << 28);
-	} else {
-		e32 = (uint32_t*)e;
+	/* emissions | transitions | codons, then the 32-bit kernel's of a paired profile */
+	row = (size_t)mpad;
+	o_t = (cols ? sizeof(uint32_t) : sizeof(int16_t)) * 21 * row, o_codon = o_t + sizeof(int32_t) * 7 * row;
+	o_e32 = o_codon + 64, o_t32 = o_e32 + sizeof(int16_t) * 21 * row;
+	size = cols >= PL_HMM_BOTH ? o_t32 + sizeof(int32_t) * 7 * row : o_e32;
+	p = (pl_hmm_profile_t*)calloc(1, sizeof(*p));
+	host = (char*)calloc(size, 1);
+	if (!p || !host) { pl_set_error("out of host memory"); goto fail; }
+	if (cols == 0) pl_hmm_tables32(m, mpad, emit, trans, (int16_t*)host, (int32_t*)(host + o_t));
+	else {
+		uint32_t *e = (uint32_t*)host;
+		int32_t *t = (int32_t*)(host + o_t);
 		const uint32_t none = ((uint32_t)t_floor & 0xffffu) * 0x10001u;
 		for (j = 0; j < 7 * mpad; ++j) t[j] = (int32_t)none;
 		for (j = 0; j < m; ++j) { /* the slot of column j in the paired kernel's tables */
 			const size_t x = (size_t)(j / (32 * cols)) * PLK_HMM_TILE + (size_t)(j % (32 * cols) / cols) * 8 + j % cols;
 			for (k = 0; k < 20; ++k) {
 				const int32_t v = emit[(size_t)j * 20 + k];
-				e32[(size_t)k * mpad + x] = (uint32_t)(v < e_floor ? e_floor : v) & 0xffffu;
+				e[(size_t)k * mpad + x] = (uint32_t)(v < e_floor ? e_floor : v) & 0xffffu;
 			}
 			for (k = 0; k < 7; ++k) {
 				const int32_t v = trans[(size_t)j * 7 + k];
 				t[(size_t)k * mpad + x] = (int32_t)(((uint32_t)(v < t_floor ? t_floor : v) & 0xffffu) * 0x10001u);
 			}
 		}
+		if (cols >= PL_HMM_BOTH)
+			pl_hmm_tables32(m, mpad, emit, trans, (int16_t*)(host + o_e32), (int32_t*)(host + o_t32));
 	}
-	p->k.cols = cols, p->k.hi = 65536;
-	p->device = device, p->k.m = m, p->k.mpad = mpad;
+	memcpy(host + o_codon, codon_alpha, 64);
 	memcpy(p->codon, codon_alpha, 64);
+	p->device = device, p->k.m = p->k32.m = m, p->k.mpad = p->k32.mpad = mpad, p->k.cols = cols;
+	p->k.hi = p->k32.hi = 65536;
 	CK(cudaSetDevice(device));
-	CK(cudaMalloc((void**)&p->k.emit_t, (cols ? sizeof(uint32_t) : sizeof(int16_t)) * 21 * (size_t)mpad));
-	CK(cudaMalloc((void**)&p->k.trans_t, sizeof(int32_t) * 7 * (size_t)mpad));
-	CK(cudaMalloc((void**)&p->codon_dev, 64));
-	CK(cudaMemcpy((void*)p->k.emit_t, e, (cols ? sizeof(uint32_t) : sizeof(int16_t)) * 21 * (size_t)mpad, cudaMemcpyHostToDevice));
-	CK(cudaMemcpy((void*)p->k.trans_t, t, sizeof(int32_t) * 7 * (size_t)mpad, cudaMemcpyHostToDevice));
-	CK(cudaMemcpy(p->codon_dev, codon_alpha, 64, cudaMemcpyHostToDevice));
-	free(e), free(t);
+	CK(cudaMalloc(&p->dev, size));
+	CK(cudaMemcpy(p->dev, host, size, cudaMemcpyHostToDevice));
+	p->k.emit_t = p->dev, p->k.trans_t = (const int32_t*)((char*)p->dev + o_t), p->codon_dev = (uint8_t*)p->dev + o_codon;
+	if (cols >= PL_HMM_BOTH)
+		p->k32.emit_t = (char*)p->dev + o_e32, p->k32.trans_t = (const int32_t*)((char*)p->dev + o_t32);
+	free(host);
 	return p;
 fail:
-	free(e), free(t);
+	free(host);
 	if (p) {
-		if (p->k.emit_t) cudaFree((void*)p->k.emit_t);
-		if (p->k.trans_t) cudaFree((void*)p->k.trans_t);
-		if (p->codon_dev) cudaFree(p->codon_dev);
+		if (p->dev) cudaFree(p->dev);
 		free(p);
 	}
 	return 0;
@@ -110,7 +128,7 @@ PL_EXPORT void pl_hmm_profile_destroy(pl_hmm_profile_t *p)
 {
 	if (!p) return;
 	cudaSetDevice(p->device);
-	cudaFree((void*)p->k.emit_t), cudaFree((void*)p->k.trans_t), cudaFree(p->codon_dev);
+	cudaFree(p->dev);
 	free(p);
 }
 
@@ -167,39 +185,50 @@ static int pl_hmm_plan(pl_engine_t *e, int32_t n, const int32_t *len, int64_t **
 	return 1;
 }
 
-/* CTAs of a profile's launch over n regions; its edge buffer (columns handed from tile to tile, two
- * rows of 16 bytes a warp, the rows in fours as the paired kernel walks them): none for one tile */
-static int32_t pl_hmm_ctas(const pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n)
+/* A profile's launch over n regions, one of n_st side by side: its kernel, and as few warps a CTA as
+ * leave one CTA to an SM of its part of the GPU, so that the regions of a small scan spread over the
+ * SMs and their schedulers (with eight warps to a CTA whatever their number, 186 regions of 12 kb
+ * against 4 profiles of up to 800 columns took 2.1 ms, on 48 SMs; a second CTA on an SM puts two
+ * warps on a scheduler where others have none). */
+typedef struct { const plk_hmm_prof_t *k; int32_t ctas, warps; } pl_hmm_grid_t;
+static int pl_hmm_grid(const pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, int32_t n_st, pl_hmm_grid_t *g)
 {
-	const int32_t units = p->k.cols ? (n + 1) / 2 : n, warps = plk_hmm_warps_per_cta();  /* the paired kernel: two regions a warp */
-	int64_t ctas = plk_hmm_ctas_per_sm(&p->k);
-	if (ctas < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
-	ctas *= e->n_sm;
-	if (ctas * warps > units) ctas = (units + warps - 1) / warps;
-	return (int32_t)ctas;
+	const int32_t most = plk_hmm_warps_per_cta(), part = e->n_sm > n_st ? e->n_sm / n_st : 1;
+	int32_t units, all;
+	g->k = p->k.cols >= PL_HMM_BOTH && n <= 4 * part ? &p->k32 : &p->k;
+	units = g->k->cols ? (n + 1) / 2 : n;  /* the paired kernel: two regions a warp */
+	all = plk_hmm_ctas_per_sm(g->k);
+	if (all < 1) { pl_set_error("HMM DP kernel does not fit on an SM"); return 0; }
+	all *= e->n_sm;
+	g->warps = units > part * most ? most : (units + part - 1) / part;
+	g->ctas = units > (int64_t)all * g->warps ? all : (units + g->warps - 1) / g->warps;
+	return 1;
 }
+/* its edge buffer (columns handed from tile to tile, two rows of 16 bytes a warp, the rows in fours as
+ * the paired kernel walks them): none for one tile */
 static int64_t pl_hmm_edge_rows(int32_t max_rows) { return ((int64_t)max_rows + 3) / 4 * 4 + 4; }
-static size_t pl_hmm_edge_bytes(const pl_hmm_profile_t *p, int32_t max_rows, int32_t ctas)
+static size_t pl_hmm_edge_bytes(int32_t max_rows, const pl_hmm_grid_t *g)
 {
-	if (p->k.mpad <= PLK_HMM_TILE) return 0;
-	return (size_t)16 * 2 * (size_t)pl_hmm_edge_rows(max_rows) * (size_t)ctas * plk_hmm_warps_per_cta();
+	if (g->k->mpad <= PLK_HMM_TILE) return 0;
+	return (size_t)16 * 2 * (size_t)pl_hmm_edge_rows(max_rows) * (size_t)g->ctas * g->warps;
 }
 
 static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, const uint8_t *nt_dev,
 		const int32_t *off, const int32_t *len, int32_t *score_dev, cudaStream_t st)
 {
 	int64_t *row_off, rows_total, cells = 0;
-	int32_t *order, max_rows, ctas, q;
+	int32_t *order, max_rows, q;
+	pl_hmm_grid_t g;
 	if (n <= 0) return 1;
 	if (!p) { pl_set_error("no profile"); return 0; }
 	if (p->device != e->device) { pl_set_error("profile on device %d, engine on device %d", p->device, e->device); return 0; }
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
 	for (q = 0; q < n; ++q) cells += (int64_t)(len[q] >= 3 ? len[q] / 3 : 0) * p->k.m;
-	if ((ctas = pl_hmm_ctas(e, p, n)) < 1) return 0;
+	if (!pl_hmm_grid(e, p, n, 1, &g)) return 0;
 	if (!dbuf_ensure(&e->h_off, sizeof(int32_t) * (size_t)n) || !dbuf_ensure(&e->h_len, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rowoff, sizeof(int64_t) * (size_t)n) || !dbuf_ensure(&e->h_order, sizeof(int32_t) * (size_t)n) ||
 			!dbuf_ensure(&e->h_rows, (size_t)(rows_total > 0 ? rows_total : 16)) || !dbuf_ensure(&e->h_counter, 64) ||
-			!dbuf_ensure(&e->h_edge, pl_hmm_edge_bytes(p, max_rows, ctas)))
+			!dbuf_ensure(&e->h_edge, pl_hmm_edge_bytes(max_rows, &g)))
 		return 0;
 	CK(cudaMemcpyAsync(e->h_off.p, off, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
 	CK(cudaMemcpyAsync(e->h_len.p, len, sizeof(int32_t) * (size_t)n, cudaMemcpyHostToDevice, st));
@@ -211,8 +240,8 @@ static int pl_hmm_run(pl_engine_t *e, const pl_hmm_profile_t *p, int32_t n, cons
 			p->codon_dev, (uint8_t*)e->h_rows.p, st));
 	PL_TIME(e, st, 0);
 	PL_TIME(e, st, 1);
-	CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
-			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, pl_hmm_edge_rows(max_rows), ctas,
+	CKK(plk_hmm_dp(g.k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
+			(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p, e->h_edge.p, pl_hmm_edge_rows(max_rows), g.ctas, g.warps,
 			score_dev, st));
 	PL_TIME(e, st, 1);
 	CK(cudaStreamSynchronize(st));
@@ -250,7 +279,8 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 {
 	int64_t *row_off, rows_total, cells = 0, rows_sum = 0;
 	size_t edge[PL_HMM_STREAMS + 1] = {0};  /* bytes of each stream's part, then where it starts */
-	int32_t *order, max_rows, q, k, s, *ctas = 0;
+	int32_t *order, max_rows, q, k, s;
+	pl_hmm_grid_t *g = 0;
 	const int32_t n_st = n_prof < PL_HMM_STREAMS ? n_prof : PL_HMM_STREAMS;
 	int ok = 0;
 	const uint8_t *codon = 0;
@@ -264,12 +294,12 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	st = stream ? (cudaStream_t)stream : e->stream;
 	if (!pl_hmm_plan(e, n, len, &row_off, &order, &rows_total, &max_rows)) return 0;
 	for (q = 0; q < n; ++q) rows_sum += len[q] >= 3 ? len[q] / 3 : 0;
-	ctas = (int32_t*)malloc(sizeof(int32_t) * (size_t)n_prof);
-	if (!ctas) { pl_set_error("out of host memory"); goto fail; }
+	g = (pl_hmm_grid_t*)malloc(sizeof(*g) * (size_t)n_prof);
+	if (!g) { pl_set_error("out of host memory"); goto fail; }
 	for (k = 0; k < n_prof; ++k) {
 		size_t b;
-		if ((ctas[k] = pl_hmm_ctas(e, ps[k], n)) < 1) goto fail;
-		b = pl_hmm_edge_bytes(ps[k], max_rows, ctas[k]);
+		if (!pl_hmm_grid(e, ps[k], n, n_st, &g[k])) goto fail;
+		b = pl_hmm_edge_bytes(max_rows, &g[k]);
 		if (b > edge[k % PL_HMM_STREAMS + 1]) edge[k % PL_HMM_STREAMS + 1] = b;
 	}
 	for (s = 0; s < n_st; ++s) edge[s + 1] += edge[s];
@@ -305,9 +335,10 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 			codon = p->codon;
 		}
 		s = k % PL_HMM_STREAMS, sk = e->h_st[s];
-		CKK(plk_hmm_dp(&p->k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
+		CKK(plk_hmm_dp(g[k].k, (const uint8_t*)e->h_rows.p, (const int64_t*)e->h_rowoff.p, (const int32_t*)e->h_len.p,
 				(const int32_t*)e->h_order.p, n, (int32_t*)e->h_counter.p + 16 * s,
-				(char*)e->h_edge.p + edge[s], pl_hmm_edge_rows(max_rows), ctas[k], score_dev + (int64_t)k * n, sk));
+				(char*)e->h_edge.p + edge[s], pl_hmm_edge_rows(max_rows), g[k].ctas, g[k].warps,
+				score_dev + (int64_t)k * n, sk));
 		cells += rows_sum * p->k.m;
 	}
 	for (s = 0; s < n_st; ++s) {  /* join */
@@ -324,7 +355,7 @@ PL_EXPORT int pl_hmm_score_many_device(pl_engine_t *e, const pl_hmm_profile_t *c
 	e->h_last_cells = cells;
 	ok = 1;
 fail:
-	free(ctas);
+	free(g);
 	return ok;
 }
 

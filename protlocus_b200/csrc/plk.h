@@ -100,6 +100,7 @@ typedef struct {
 	                            j-1 at tile * 256 + lane * 8 + c and each transition in both halves;
 	                            0: the 32-bit kernel, 8 columns a lane */
 	uint32_t hi;             /* 65536, read as a kernel constant: a shift would issue on the ALU pipe */
+	int32_t warps;           /* of a CTA that take regions (a launch's; the others only stage the emissions) */
 } plk_hmm_prof_t;
 #define PLK_HMM_TILE 256
 #define PLK_HMM_SMEM_MAX (96 * 1024)   /* emissions staged in shared memory up to mpad = 2048, */
@@ -166,12 +167,12 @@ int plk_ext_warps_per_cta(void);
 /* results[q] (pl_ext_result_t) from the job table */
 int plk_ext_results(const plk_ext_job_t *jobs, int32_t n_jobs, void *results, void *stream);
 void plk_add_launches(uint64_t n);
-/* integer HMM DP: codon rows of every region, then one warp per region (order) */
+/* integer HMM DP: codon rows of every region, then one warp per region or pair (order), `warps` to a CTA */
 int plk_hmm_codons(const uint8_t *nt, const int32_t *off, const int32_t *len, const int64_t *row_off, int32_t n,
 		const uint8_t *codon_alpha, uint8_t *rows, void *stream);
 int plk_hmm_dp(const plk_hmm_prof_t *p, const uint8_t *rows, const int64_t *row_off, const int32_t *len,
 		const int32_t *order, int32_t n, int32_t *counter, void *edge, int64_t edge_stride_rows, int32_t n_ctas,
-		int32_t *score, void *stream);
+		int32_t warps, int32_t *score, void *stream);
 int plk_hmm_ctas_per_sm(const plk_hmm_prof_t *p);
 int plk_hmm_warps_per_cta(void);
 int plk_hmm_smem_bytes(int32_t mpad, int32_t cols);  /* 0: read from global memory */
