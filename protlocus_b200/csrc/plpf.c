@@ -36,7 +36,7 @@ typedef struct {
 } pf_layer_t;
 
 struct pl_pf_model_s {
-	int device;
+	int device, n_sm;
 	int32_t in_dim, hidden;
 	pf_layer_t L[PF_LAYERS];
 	int32_t *err, *step;
@@ -183,6 +183,7 @@ PL_EXPORT pl_pf_model_t *pl_pf_model_create(int32_t device, int32_t in_dim, int3
 	pthread_mutex_init(&m->mu, 0);
 	m->device = device, m->in_dim = in_dim, m->hidden = hidden;
 	CK(cudaSetDevice(device));
+	CK(cudaDeviceGetAttribute(&m->n_sm, cudaDevAttrMultiProcessorCount, device));
 	for (l = 0; l < PF_LAYERS; ++l) {
 		pf_layer_t *y = &m->L[l];
 		y->in = l == 0 ? in_dim : hidden;
@@ -247,7 +248,7 @@ static int pf_gemm(pl_pf_model_t *m, const void *A, int64_t lda, const void *B, 
 /* n_tile of an M x N output (N = hidden, 128 or 256): all columns in one tile where the row tiles
  * make two waves of the SMs, else 64, which gives four times the CTAs for A read four times from
  * L2 (4096 rows: 32 CTAs or 128) */
-static int32_t pf_tile(int32_t M, int32_t N) { return M / 128 >= 296 ? N : 64; }
+static int32_t pf_tile(const pl_pf_model_t *m, int32_t M, int32_t N) { return M / 128 >= 2 * m->n_sm ? N : 64; }
 
 /* forward of rows [0, M) of X (bf16 [M x in]) into H[0..2] (and their transposes when HT) and out f32 [M x 16] */
 static int pf_forward(pl_pf_model_t *m, const void *X, int32_t M, void *const *H, void *const *HT, float *out, cudaStream_t st)
@@ -257,7 +258,7 @@ static int pf_forward(pl_pf_model_t *m, const void *X, int32_t M, void *const *H
 	for (l = 0; l < 3; ++l) {
 		const void *in = l == 0 ? X : H[l - 1];
 		const int64_t ld_in = l == 0 ? m->in_dim : h;
-		int e = pf_gemm(m, in, ld_in, m->L[l].W, m->L[l].in, M, h, m->L[l].in, pf_tile(M, h), m->L[l].pb, 1, 0, 0,
+		int e = pf_gemm(m, in, ld_in, m->L[l].W, m->L[l].in, M, h, m->L[l].in, pf_tile(m, M, h), m->L[l].pb, 1, 0, 0,
 				H[l], h, HT ? HT[l] : 0, M, 0, 0, st);
 		if (e) return e;
 	}
@@ -330,10 +331,10 @@ static int pf_step(pl_pf_model_t *m, const void *feats, const float *tgt, const 
 	T_(pf_forward(m, m->X, B, m->H, m->HT, m->out, st));
 	T_(plk_mlp_loss(m->out, PF_OUT, m->T, B, pos_w, box_w, m->dout, PF_OUT_PAD, m->doutT, m->loss_sum, st));
 	/* dZ2 = (dout . W3) masked by H2, dZ_{l-1} = (dZ_l . W_l) masked by H_{l-1} */
-	T_(pf_gemm(m, m->dout, PF_OUT_PAD, m->L[3].WT, PF_OUT_PAD, B, h, PF_OUT_PAD, pf_tile(B, h), 0, 0, m->H[2], h,
+	T_(pf_gemm(m, m->dout, PF_OUT_PAD, m->L[3].WT, PF_OUT_PAD, B, h, PF_OUT_PAD, pf_tile(m, B, h), 0, 0, m->H[2], h,
 			m->dZ[2], h, m->dZT[2], B, 0, 0, st));
 	for (l = 2; l > 0; --l)
-		T_(pf_gemm(m, m->dZ[l], h, m->L[l].WT, m->L[l].out_pad, B, h, h, pf_tile(B, h), 0, 0, m->H[l - 1], h,
+		T_(pf_gemm(m, m->dZ[l], h, m->L[l].WT, m->L[l].out_pad, B, h, h, pf_tile(m, B, h), 0, 0, m->H[l - 1], h,
 				m->dZ[l - 1], h, m->dZT[l - 1], B, 0, 0, st));
 	/* gW_l = dZ_l^T . (input of layer l), the output layer's dout^T . H2 (rows >= 16 of dout^T are
 	 * zero), one launch; then all bias gradients */
