@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(THREADS) k_pf_features(plk_pf_feat_args_t A)
 	/* 3. sort the kept anchors by (position, protein position) -- all keys differ -- and chain them */
 	const int na_all = S.n_anchor, na = na_all < MAXA ? na_all : MAXA;
 	if (na_all > MAXA) {
-		nh = __reduce_add_sync(0xffffffffu, nh);
+		for (int o = 16; o >= 1; o >>= 1) nh += __shfl_xor_sync(0xffffffffu, nh, o);
 		if (lane == 0) S.part_n[warp] = nh;
 		__syncthreads();
 		int base = 0;
