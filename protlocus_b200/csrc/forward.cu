@@ -773,7 +773,7 @@ __global__ void __launch_bounds__(32 * RC_UW, 1) k_rc_lanes(RcArgs A)
 	else if (w == RC_W_E) rc_fwd_e(S, P, R, on, Y, A.err);
 	else if (w == RC_W_B) { if (G.full) rc_bwd_chain(S, P, R, n2, Y, A.err); }
 	else if (w == RC_W_F) { if (G.full) rc_bwd_feed(S, P, R, dsq, n2, Y, A.err); }
-	else { /* of the other eight, the first RC_MI to the Forward */
+	else { /* of the other six, the first RC_MI to the Forward, the next to the Backward */
 		const int x = w < RC_WARPS ? w - (w > RC_W_D) - (w > RC_W_B) - (w > RC_W_E) - (w > RC_W_F) : 2 * RC_MI;
 		if (x < RC_MI) rc_fwd_mi(S, P, R, dsq, x, Y, A.err);
 		else if (G.full && x < 2 * RC_MI) rc_bwd_mi(S, P, R, dsq, n2, x - RC_MI, Y, A.err);

@@ -24,8 +24,9 @@
  * K instead would sum in another order, which Adam's division amplifies), and all bias
  * gradients and all Adam updates are one launch each: 13 launches instead of 26, 16 steps of
  * 4096 rows with the parameters set before and read after 16.4 -> 3.9 ms.  A K step now takes
- * 0.9 us whatever the tile (a 256 x 576 gradient over 4096 rows 58 us): the proxy fence and
- * the CTA's barrier of every stage.
+ * 0.9 us whatever the tile (a 256 x 576 gradient over 4096 rows, 64 steps, 58 us): the proxy fence
+ * and the CTA's barrier of every stage.  The weight gradients' 152 CTAs of eight stages fit one to an
+ * SM, so on 148 SMs four of them make a second pass.
  *
  * Every mbarrier wait is bounded: on expiry the kernel sets *err, waits once more
  * (bounded) for its own tensor-core work, frees its tensor memory and returns.

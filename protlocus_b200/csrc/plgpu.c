@@ -1002,8 +1002,8 @@ static int32_t ns_q_n;
 /* When a batch is complete.  A request is worth waiting for only while some caller that could
  * send it is not waiting itself.  So the collection ends before its 2 ms once a caller waits for a
  * queued request and the queue holds as many requests as were ever outstanding at once around the
- * last batches: a lone caller, who sends one request and waits, is served at once (2.0 of the
- * 4.7 ms of a 500-residue protein against 20 kb were this wait), T callers get one batch
+ * last batches: a lone caller, who sends one request and waits, is served at once (a 500-residue
+ * protein against 20 kb takes 2.9 ms, and took these 2 more), T callers get one batch
  * of T as soon as the last of them is back, and requests sent ahead of any wait are collected as
  * before. */
 #define NS_PEAKS 8

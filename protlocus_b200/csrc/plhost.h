@@ -36,7 +36,7 @@ struct pl_engine_s {
 	int64_t g_nlaunch, g_replays;           /* kernel launches in the graph; replays so far */
 	int32_t g_dp_launches, g_coop;
 	int32_t r4_rows;                        /* jobs with at most this many DP rows take 4 rows per lane */
-	double coop_ratio;                      /* cooperative-job threshold (pl_coop_ratio by default) */
+	double coop_ratio;                      /* shared-job threshold (pl_coop_ratio by default) */
 	cudaStream_t stream;
 	/* second stream of the global DP: when a batch needs several waves, odd waves run
 	 * on it with their own trace arena, so a wave's DP fills the tail of the one before */

@@ -26,8 +26,9 @@
  *                Trace words (state in bits 0-3, extension and lazy-F flags) are written
  *                with one 16-byte store per lane per step into a diagonal-major
  *                layout, so every warp store is a contiguous 512-byte run.
- *   k_traceback  one thread per job walks the trace (nasw-sse.c:44-93) and
- *                writes the run-length merged CIGAR in reverse.
+ *   k_traceback  one warp per job: lane 0 walks the trace (nasw-sse.c:44-93) over tiles
+ *                the warp stages, the warp scans intron runs, and the run-length
+ *                merged CIGAR is written in reverse.
  *   k_scan / k_compact  exclusive scan of CIGAR lengths and the reversed copy
  *                into the dense output with ns_fix_tiny_UV (nasw-sse.c:34-42).
  */
