@@ -49,8 +49,8 @@ from protlocus_b200.abi import NS_F_CIGAR, ExtJob, ExtResult, Options, SpliceJob
 from protlocus_b200.ranks import Ranks, job_rate  # noqa: E402
 
 METRIC = "spliced-DP GCUPS (bit-exact) at 1 B200"
-DP_DRAM_BYTES_PER_CELL = 2.08  # ncu: k_splice_dp dram__bytes_read+write per cell (trace words are 2.0 B/cell)
-PAIR_DRAM_BYTES_PER_CELL = 2.20  # ncu: k_splice_pair<8>, uniform 4736x2000x250 (0.41 GB read + 6.54 GB written)
+DP_DRAM_BYTES_PER_CELL = 2.24  # ncu: k_splice_dp dram__bytes_read+write per cell, 700 loci (trace words are 2.0 B/cell)
+PAIR_DRAM_BYTES_PER_CELL = 2.22  # ncu: k_splice_pair<8>, 5,000 strands of 1-2.5 kb (0.57 GB read + 9.74 GB written)
 OPS_PER_CELL = 65  # int16 lane-ops per cell with traceback bits, counted from nasw-sse.c:465-553
 WORKLOAD = ("batched global spliced DP: 4096 protein/window pairs x 2 strands = 8192 DPs with CIGAR; "
             "protein log-normal median 350 aa (50-2500), window uniform 1-50 kb, Poisson(4) introns, "
@@ -570,10 +570,10 @@ def main():
                          "peak": peak, "unit": "lane-ops/s", "frac": achieved / peak if peak else None,
                          "traffic": (int((PAIR_DRAM_BYTES_PER_CELL if n_pairs else DP_DRAM_BYTES_PER_CELL)
                                          * tm["cells"] / tm["dp_launches"]) if tm["dp_launches"] else None),
-                         "traffic_source": ("ncu dram bytes read+write of one k_splice_pair launch on the uniform "
-                                            "4736x2000x250 case (2.20 B/cell)" if n_pairs else
-                                            "ncu dram bytes read+write of one k_splice_dp launch on the uniform "
-                                            "2400x2000x350 case (2.08 B/cell)") + ", scaled by this run's cells per launch",
+                         "traffic_source": ("ncu dram bytes read+write of one k_splice_pair launch over 5,000 strands "
+                                            "of 1-2.5 kb (2.22 B/cell)" if n_pairs else
+                                            "ncu dram bytes read+write of one k_splice_dp launch over 700 loci of "
+                                            "1-4 kb (2.24 B/cell)") + ", scaled by this run's cells per launch",
                          "ops_per_cell": OPS_PER_CELL, "dp_kernel_gcups": round(dp_gcups, 3),
                          "peak_source": "measured live: pl_measure_int_peak (int32 %.3g, int16x2 %.3g lane-ops/s)"
                                         % (int32_peak, i16x2_peak),
@@ -1310,7 +1310,7 @@ def main_forward(args):
                     "api": "pl_rc_score_host (C ABI, host buffers), wall clock"},
             "gpu_launches": int(launches),
             "roofline": {"bound": "latency", "kernel": "k_rc_lanes", "achieved": None, "peak": None, "frac": None,
-                         "note": "one peptide per lane of seven warps; the longest peptide's chains (three dependent logsums per "
+                         "note": "one peptide per lane of eight warps; the longest peptide's chains (three dependent logsums per "
                                  "Backward cell, each a restated glibc expf + log1pf) bound the step"},
             "cpu_baseline": {"value": round(c / secs / 1e9, 4), "unit": "GCUPS", "cores": threads, "kind": "reference",
                              "sample": f"{k} peptides, recheck.c rc_score via kt_for"}}
